@@ -117,8 +117,9 @@ int mpd_advance(mpd_solver *s, double dt);
  * (Diagnostics::ComputeDt after every step), the reference's relative-L2
  * convergence check every check_frequency steps, and an L-inf residual
  * criterion.  Runs until t >= T, convergence, or max_steps. */
-/* How mpd_run drives the steps.  GRAPH: an interior and a boundary kernel per
- * step, replayed from captured CUDA graphs.  PERSISTENT: one cooperative
+/* How mpd_run drives the steps.  GRAPH: one kernel per step (an interior and a
+ * boundary kernel where mpd_set_ring_overlap says so), replayed from captured
+ * CUDA graphs.  PERSISTENT: one cooperative
  * launch runs many steps with grid barriers between the interior and the
  * boundary phase (fast precision, no SolutionChange checks).  AUTO takes
  * GRAPH.  Both give the same results, bit for bit. */
@@ -236,16 +237,15 @@ int mpd_set_expression_ic(mpd_solver *s, const char *const exprs[8], int n_vars,
 
 /* Where a fast step's boundary ring runs (new; no reference counterpart: the
  * reference applies the faces after the central update, src/solver.cpp:
- * 22-37, and both forms keep that order of values).  on = 1: beside the
- * interior kernel, in bc_overlap_kernel, which recomputes the
- * central cells the faces read from the step's input state, so the ring's
- * dependent chains overlap the interior and only the end-of-step controller
- * waits for it; the interior kernel then computes rows 2..L-1.  on = 0 (the
- * default): after the interior kernel, reading the central cells it stored.  The two give
+ * 22-37, and every form keeps that order of values).  on = 0 (the default):
+ * in the interior's own kernel where the boundary configuration allows
+ * (lf_step_kernel: no interpreted expressions, every face cell covered, AxisLF
+ * segments disjoint), else in a kernel after it, reading the central cells it
+ * stored.  on = 1: in bc_overlap_kernel beside the interior kernel.  All give
  * the same bits.  Takes effect from the next step; exact precision, the first
- * step and grids with L_max < 4 always use the second form.
- * mpd_ring_overlap_active reports whether fast steps of the handle use the
- * first. */
+ * step and (on = 1) grids with L_max < 4 always run it after the interior.
+ * mpd_ring_overlap_active reports whether fast steps of the handle use
+ * bc_overlap_kernel. */
 int mpd_set_ring_overlap(mpd_solver *s, int on);
 int mpd_ring_overlap_active(mpd_solver *s, int *active);
 
@@ -264,7 +264,8 @@ int mpd_profile_kernels(mpd_solver *s, int steps, double dt, double out_ms[2]);
 /* Measurement support (new; no reference counterpart): the mean device time
  * in ms of one launch of a step kernel, from `launches` back-to-back launches
  * between two events on the handle's stream, with nothing else between them.
- * MPD_KERNEL_INTERIOR: the interior kernel of the handle's precision at time
+ * MPD_KERNEL_INTERIOR: the interior kernel of the handle's precision (a fast
+ * step's one kernel, ring included, where it has one) at time
  * step dt; every launch recomputes the next step's interior cells from the
  * current state (the step counter does not advance; the state stays valid).
  * MPD_KERNEL_RESIDUAL: the L-inf residual pass over the current and previous

@@ -103,43 +103,67 @@ void ClosedForm(const mpd_config &cfg, const ExprCode &ec, int j, SegDesc &d) {
         d.ca[j] = eval_code(ec.code.data(), ec.consts.data(), sym);
         return;
     }
-    // operand: a symbol (cell-independent ones become constants) or a constant
-    auto operand = [&](int32_t ins, int &sym, double &c) {
+    // The program on a symbolic stack: constants (cell-independent symbols
+    // among them) fold as they meet; what is left must be one operand or one
+    // operation on two.
+    struct Term {
+        int kind;  // 0 constant, 1 symbol, 2 operation on two operands
+        int sym, op, a, b;
+        double c, ca, cb;
+    };
+    std::vector<Term> st;
+    for (int32_t ins : ec.code) {
         const int op = ins & 0xff;
         const int arg = ins >> 8;
+        Term t{};
+        t.sym = t.a = t.b = -1;
+        if (op == OP_END) break;
         if (op == OP_CONST) {
-            sym = -1;
-            c = ec.consts[arg];
-            return true;
-        }
-        if (op != OP_VAR) return false;
-        if (CellIndependent(arg)) {
-            sym = -1;
-            c = CellIndependentValue(cfg, arg);
+            t.c = ec.consts[arg];
+        } else if (op == OP_VAR && CellIndependent(arg)) {
+            t.c = CellIndependentValue(cfg, arg);
+        } else if (op == OP_VAR) {
+            t.kind = 1;
+            t.sym = arg;
+        } else if (op == OP_NEG && !st.empty() && st.back().kind == 0) {
+            t = st.back();
+            st.pop_back();
+            t.c = -t.c;
+        } else if ((op == OP_ADD || op == OP_SUB || op == OP_MUL || op == OP_DIV) &&
+                   st.size() >= 2) {
+            const Term y = st.back(), x = st[st.size() - 2];
+            st.pop_back();
+            st.pop_back();
+            if (x.kind == 2 || y.kind == 2) return;
+            if (x.kind == 0 && y.kind == 0) {
+                t.c = bc_binop(op, x.c, y.c);
+            } else {
+                t.kind = 2;
+                t.op = op;
+                t.a = x.sym;
+                t.ca = x.c;
+                t.b = y.sym;
+                t.cb = y.c;
+            }
         } else {
-            sym = arg;
-        }
-        return true;
-    };
-    const std::vector<int32_t> &c = ec.code;
-    if (c.size() == 2 && (c[1] & 0xff) == OP_END && operand(c[0], d.fa[j], d.ca[j])) {
-        // x * 1.0 is x exactly
-        d.form[j] = EF_BIN;
-        d.fop[j] = OP_MUL;
-        d.fb[j] = -1;
-        d.cb[j] = 1.0;
-        return;
-    }
-    if (c.size() == 4 && (c[3] & 0xff) == OP_END) {
-        const int op = c[2] & 0xff;
-        if ((op == OP_ADD || op == OP_SUB || op == OP_MUL || op == OP_DIV) &&
-            operand(c[0], d.fa[j], d.ca[j]) && operand(c[1], d.fb[j], d.cb[j])) {
-            d.form[j] = EF_BIN;
-            d.fop[j] = op;
             return;
         }
+        st.push_back(t);
     }
-    d.fa[j] = d.fb[j] = -1;
+    if (st.size() != 1 || st[0].kind == 0) return;
+    const Term &t = st[0];
+    d.form[j] = EF_BIN;
+    if (t.kind == 1) {  // x * 1.0 is x exactly
+        d.fop[j] = OP_MUL;
+        d.fa[j] = t.sym;
+        d.cb[j] = 1.0;
+    } else {
+        d.fop[j] = t.op;
+        d.fa[j] = t.a;
+        d.ca[j] = t.ca;
+        d.fb[j] = t.b;
+        d.cb[j] = t.cb;
+    }
 }
 
 }  // namespace
@@ -251,6 +275,96 @@ int CompileBc(const mpd_config &cfg, CompiledBc &out, std::string &err) {
     if (out.code.empty()) out.code.push_back(OP_END);
     if (out.consts.empty()) out.consts.push_back(0.0);
     return MPD_OK;
+}
+
+namespace {
+
+// Ring-table operand of a boundary expression symbol (BcSym), -1 for none:
+// cell-independent symbols were folded into constants by ClosedForm.
+int RingSymOf(int sym) {
+    static const int nb_field[8] = {Q_RHO, Q_VZ, Q_VR, Q_VPHI, Q_E, Q_HZ, Q_HR, Q_HPHI};
+    if (sym >= BS_CUR0 && sym < BS_CUR0 + 8) return RS_CUR0 + (sym - BS_CUR0);
+    if (sym >= BS_NB0 && sym < BS_NB0 + 8) return RS_NB0 + nb_field[sym - BS_NB0];
+    switch (sym) {
+        case BS_DR: return RS_DR;
+        case BS_R: return RS_R;
+        case BS_RZ: return RS_RZ;
+        case BS_Z: return RS_Z;
+        case BS_RNB: return RS_RNB;
+        case BS_RZNB: return RS_RZNB;
+        default: return RS_CONST;
+    }
+}
+
+bool ConstantField(const SegDesc &d, int j) {
+    return d.type[j] == COND_DIRICHLET || (d.type[j] == COND_EXPR && d.form[j] == EF_CONST);
+}
+
+}  // namespace
+
+bool CompileRing(const CompiledBc &bc, int L, int M, CompiledRing &out) {
+    out = CompiledRing();
+    if (bc.seg.size() > static_cast<size_t>(kRingSegments)) return false;
+    for (const SegDesc &d : bc.seg) {
+        RingSeg r{};
+        for (int j = 0; j < 8; ++j) {
+            switch (d.type[j]) {
+                case COND_NEUMANN:
+                    r.neu |= 1u << j;
+                    r.value[j] = d.value[j];
+                    break;
+                case COND_DIRICHLET: r.value[j] = d.value[j]; break;
+                case COND_AXIS_LF: r.axis |= 1u << j; break;
+                default: {
+                    if (d.form[j] == EF_CONST) {
+                        r.value[j] = d.ca[j];
+                    } else if (d.form[j] == EF_BIN) {
+                        RingBin &b = r.bin[r.nbin++];
+                        b.j = j;
+                        b.op = d.fop[j];
+                        b.ca = d.ca[j];
+                        b.cb = d.cb[j];
+                        b.fa = d.fa[j] < 0 ? RS_CONST : RingSymOf(d.fa[j]);
+                        b.fb = d.fb[j] < 0 ? RS_CONST : RingSymOf(d.fb[j]);
+                        if ((d.fa[j] >= 0 && b.fa < 0) || (d.fb[j] >= 0 && b.fb < 0)) return false;
+                    } else {
+                        return false;
+                    }
+                }
+            }
+        }
+        if (r.axis) out.has_axis = 1;
+        out.seg.push_back(r);
+    }
+    // the segment that decides each face cell: the last one that covers it
+    out.len = line_len(L, M);
+    out.cov.assign(4 * static_cast<size_t>(out.len), 0);
+    // L_LO, L_HI, M_LO, M_HI; (1, M+1) is M_HI's, (L, M+1) is L_HI's
+    const int lo[4] = {1, 1, 2, 1}, hi[4] = {M, M + 1, L - 1, L - 1};
+    for (int f = 0; f < 4; ++f)
+        for (int k = lo[f]; k <= hi[f]; ++k) {
+            int found = -1, n = 0;
+            for (int t = 0; t < bc.nseg[f]; ++t) {
+                const SegDesc &d = bc.seg[bc.first[f] + t];
+                if (k < d.lo || k > d.hi) continue;
+                found = bc.first[f] + t;
+                ++n;
+            }
+            if (found < 0) return false;
+            // AxisLF keeps what an earlier segment left: one segment per cell
+            if (f == FACE_M_LO && out.has_axis && n > 1) return false;
+            out.cov[static_cast<size_t>(f) * out.len + k] = static_cast<unsigned char>(found);
+        }
+    if (!out.has_axis) return true;
+    const unsigned char *m_lo = out.cov.data() + static_cast<size_t>(FACE_M_LO) * out.len;
+    for (int l = 2; l <= L - 1; ++l) {
+        const SegDesc &d = bc.seg[m_lo[l]];
+        if (l > 2 && m_lo[l] < m_lo[l - 1]) return false;
+        if (!d.has_axis) continue;
+        for (int j : {Q_VZ, Q_HZ})
+            if (d.type[j] != COND_AXIS_LF && !ConstantField(d, j)) return false;
+    }
+    return true;
 }
 
 }  // namespace mpd

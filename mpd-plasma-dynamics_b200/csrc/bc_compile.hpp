@@ -25,6 +25,19 @@ struct CompiledBc {
 // Boundary expression symbol names in BcSym order.
 const std::vector<std::string> &BcSymbolNames();
 
+// The ring table of a compiled configuration: seg and cov (4 x len) of
+// RingTable.  False when only bc_kernel can run the ring: an expression the
+// closed forms don't cover, a face cell no segment covers, more than
+// kRingSegments segments, or AxisLF segments whose half-stencil reads more
+// than a row's own neighbours (overlapping or unordered M_LO segments, a v_z or
+// H_z that is neither AxisLF nor a constant).
+struct CompiledRing {
+    std::vector<RingSeg> seg;
+    std::vector<unsigned char> cov;
+    int len = 0, has_axis = 0;
+};
+bool CompileRing(const CompiledBc &bc, int L, int M, CompiledRing &out);
+
 // Returns an MPD_* status; on failure `err` holds a message in the
 // reference's wording where the reference has one.
 int CompileBc(const mpd_config &cfg, CompiledBc &out, std::string &err);

@@ -34,7 +34,36 @@ struct EmuSolver {
     long long step = 0;
     int len = 0;
     std::vector<double> cphys, wall[2];
+    bool has_ring = false;  // the configuration has a ring table
+    mpd::CompiledRing ring;
 };
+
+// 8 primitive values in host memory (the device's are shared-memory slots).
+struct HostSlots {
+    double *v;
+    double get(int j) const { return v[j]; }
+    void set(int j, double x) const { v[j] = x; }
+};
+
+// The fast step's ring as lf_step_kernel computes it: every cell from the input
+// state alone.
+void RingFromTable(const EmuSolver *s, const double *u0, double *u, double dt) {
+    mpd::RingTable t{};
+    t.seg = s->ring.seg.data();
+    t.cov = s->ring.cov.data();
+    t.len = s->ring.len;
+    t.nseg = static_cast<int>(s->ring.seg.size());
+    t.has_axis = s->ring.has_axis;
+    for (int i = 0; i < mpd::ring_count(s->g); ++i) {
+        mpd::RingLane c;
+        c.place(s->g, t, i);
+        if (!c.act) continue;
+        c.load(s->g, u0);
+        double nb[8], cur[8], uf[8], r;
+        mpd::ring_cell_new<true>(s->g, t, t.seg, c, u0, dt, HostSlots{nb}, HostSlots{cur}, uf, r);
+        for (int k = 0; k < 8; ++k) u[k * s->g.ps + s->g.ix(c.l, c.m)] = uf[k];
+    }
+}
 
 }  // namespace
 
@@ -121,6 +150,7 @@ int mpd_emu_create(const mpd_config *cfg, const mpd_geometry *geom, const double
     s->bc.ncode = static_cast<int>(s->cbc.code.size());
     s->bc.nconst = static_cast<int>(s->cbc.consts.size());
     s->precision = cfg->precision;
+    s->has_ring = mpd::CompileRing(s->cbc, L, M, s->ring);
     *out = s;
     return MPD_OK;
 }
@@ -130,7 +160,8 @@ void mpd_emu_destroy(void *h) { delete static_cast<EmuSolver *>(h); }
 // order: 0 = compute every ring cell, then write them; 1 = write each as it is
 // computed, in ring order; 2 = the same in reverse order.  All three must give
 // the same state, which is what makes the one-thread-per-cell device kernel
-// free of read/write hazards.
+// free of read/write hazards.  3 (fast steps after the first, configurations
+// with a ring table): the ring from the table.
 int mpd_emu_advance(void *h, double dt, int order) {
     auto *s = static_cast<EmuSolver *>(h);
     const mpd::Geo &g = s->g;
@@ -196,6 +227,11 @@ int mpd_emu_advance(void *h, double dt, int order) {
     v.fast = s->precision == MPD_PRECISION_FAST ? 1 : 0;
     v.dt = dt;
     v.bc = s->bc;
+    if (order == 3 && s->has_ring && !first && s->precision == MPD_PRECISION_FAST) {
+        RingFromTable(s, u0, u, dt);
+        s->step++;
+        return MPD_OK;
+    }
     const int nring = mpd::ring_count(g);
     std::vector<double> ring(8 * static_cast<size_t>(nring));
     for (int t = 0; t < nring; ++t) {
@@ -247,6 +283,8 @@ int mpd_emu_download(void *h, int which, double *out) {
         }
     return MPD_OK;
 }
+
+int mpd_emu_has_ring(void *h) { return static_cast<EmuSolver *>(h)->has_ring ? 1 : 0; }
 
 double mpd_emu_wave_speed(void *h) {
     auto *s = static_cast<EmuSolver *>(h);

@@ -68,6 +68,36 @@ struct HostMirror {
     int ws_valid, wait_fail;
 };
 
+// The controller between two lf_step_kernel launches (lf_step.cuh): the state
+// after `step` steps, with the end of the last one (the next dt and the stop
+// flags from its wave speed, in StepHot) still to be worked out when
+// `stepped`.  A 128-byte line of its own: every block of a launch reads it
+// with one request of one warp.
+struct alignas(128) StepCtl {
+    double t, dt, dt_used, last_ws;
+    long long step;
+    int stepped, done, nonfinite, ws_valid;
+    int pad[18];
+};
+
+// What the step kernels share: controller slots by launch parity; each step's
+// wave-speed maximum and non-finite flag by step count mod 3 (one being read,
+// one being accumulated, one being cleared) with the wait-failure flag, one
+// line; the run parameters (written by the host only), one line.
+struct StepHot {
+    StepCtl ctl[2];
+    struct alignas(128) Acc {
+        unsigned long long ws[3];
+        unsigned int nf[4];
+        int wait_fail;
+    } acc;
+    struct alignas(128) Run {
+        double T, cfl, growth, dt_min, dt_max;
+        long long max_steps;
+        int run_mode, adaptive;
+    } run;
+};
+
 // Device-resident controller and reduction accumulators of one solve.  The
 // boundary kernel's last block finalises each step here, so a captured CUDA
 // graph can run many steps without the host (dt, t, step, stop flags stay on
@@ -90,6 +120,7 @@ struct DevState {
     long long resid_step;
     unsigned long long t0_ns, done_ns;  // persistent loops: first step taken, run done
     HostMirror *mirror;                 // mapped host memory, or null
+    StepHot hot;                        // lf_step.cuh
 };
 
 constexpr int kFlagWs = 1;
@@ -286,6 +317,18 @@ __device__ __forceinline__ void step_controller(const Geo &g, DevState *st, long
     }
     st->ws_acc = 0ull;
     st->nf_acc = 0u;
+    // where lf_step_kernel would take over
+    StepCtl c{};
+    c.t = t;
+    c.dt = c.dt_used = dt;
+    if (run_mode) c.dt = st->dt;
+    c.last_ws = ws;
+    c.step = nstep;
+    c.stepped = 0;
+    c.done = run_mode ? st->done : 0;
+    c.nonfinite = nonfinite;
+    c.ws_valid = (flags & kFlagWs) ? 1 : 0;
+    st->hot.ctl[0] = c;
     // per-call mode only: a run's loop is never watched from the host (the
     // host state, mirror included, is refreshed when the run ends), and a
     // system-scope fence costs each step ~1.7 us on its critical path
@@ -598,11 +641,9 @@ __global__ void __launch_bounds__(256) residual_kernel(Geo g, const double *buf0
     st->last_resid = R;
     st->resid_valid = 1;
     st->resid_step = step;
-    if (run_mode && resid_tol > 0.0 && R <= resid_tol) {
-        st->converged = 1;
-        st->done = 1;
-    }
-    if (run_mode && nonfinite) st->done = 1;
+    const bool met = run_mode && resid_tol > 0.0 && R <= resid_tol;
+    if (met) st->converged = 1;
+    if (met || (run_mode && nonfinite)) st->done = st->hot.ctl[0].done = 1;
     st->res_arrive = 0u;  // the next arrivals come from a later launch
 }
 
@@ -803,7 +844,7 @@ __global__ void change_finish_kernel(const double *partials, int nblocks, DevSta
         st->check_due = 0;
         if (change < st->conv_thr) {
             st->converged = 1;
-            st->done = 1;
+            st->done = st->hot.ctl[0].done = 1;
         }
     }
 }
@@ -947,6 +988,22 @@ __global__ void init_wall_kernel(Geo g, const double *ic, double *wall0, int len
         const bool in = l >= 1 && l <= g.L;
         store_line_phys(wall0, len, 0, l, in ? load_phys(ic, g.ps, g.ix(l, 1)) : phys_zero());
         store_line_phys(wall0, len, 1, l, in ? load_phys(ic, g.ps, g.ix(l, g.M + 1)) : phys_zero());
+    }
+}
+
+// The wall lines a boundary kernel reads, from the current state (steps >= 1,
+// fast precision): what it would have left after the last step.
+__global__ void wall_lines_kernel(Geo g, const double *u0, double *wall, int len) {
+    for (int l = 1 + blockIdx.x * blockDim.x + threadIdx.x; l <= g.L; l += gridDim.x * blockDim.x) {
+        BcView v;
+        v.g = g;
+        v.fast = 1;
+        for (int side = 0; side < 2; ++side) {
+            const int m = side ? g.M + 1 : 1;
+            double u[8];
+            load_cons(u0, g.ps, g.ix(l, m), u);
+            store_line_phys(wall, len, side, l, recon_bc(v, u, g.r(l, m)));
+        }
     }
 }
 

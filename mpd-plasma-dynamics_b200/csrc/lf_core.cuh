@@ -509,6 +509,38 @@ struct BcTable {
     int nseg_total, ncode, nconst;
 };
 
+// The boundary ring in a form whose cells cost a few hundred instructions
+// each (ring_kernel, lf_step.cuh): a segment's fields without the interpreter,
+// and per face the segment that decides each cell.  CompileRing
+// (bc_compile.cpp) says which configurations have one.
+constexpr int kRingSegments = 16;  // segments of all faces a ring table holds
+
+// Operands of a binary field: slots of the neighbour's and of the cell's own
+// primitives (PrimIdx), then geometry.
+enum RingSym {
+    RS_CONST = -1, RS_NB0 = 0, RS_CUR0 = 8, RS_DR = 16, RS_R, RS_RZ, RS_Z, RS_RNB, RS_RZNB
+};
+
+struct RingBin {
+    double ca, cb;    // constant operands
+    int j, op, fa, fb;  // field, OP_ADD .. OP_DIV, RingSym of each operand
+};
+
+struct RingSeg {
+    double value[8];    // Neumann offset, Dirichlet value or folded constant
+    unsigned int neu;   // bit j: field j is the neighbour's plus value[j]
+    unsigned int axis;  // bit j: field j is AxisLF
+    int nbin, pad;
+    RingBin bin[8];     // binary fields in evaluation order
+};
+
+struct RingTable {
+    const RingSeg *seg;
+    const unsigned char *cov;  // [4][len]: segment of free index k of each face
+    int len, nseg;
+    int has_axis;
+};
+
 // Values of the cells the boundary faces read, laid out as "lines" along one
 // grid row or column (field stride len).
 //   central lines (the interior kernel's new conserved values, 8 fields, of
@@ -582,58 +614,88 @@ MPD_HD bool wants_central(int L, int M, int l, int m) {
     return l == 2 || l == L - 1 || m == 2 || m == M;
 }
 
-// Point (n, p) of the step's input state as the fast interior's warp sees it:
-// conserved values, primitives and radius (ghost rows: U = 0, r = 1, every
-// primitive 0).
-MPD_HD void fast_point(const Geo &g, const double *u0, int n, int p, double gm1, double U[8],
-                       FastPrim &q, double &r) {
-    const bool gh = n <= 0 || n >= g.L + 1 || p > g.M + 1;
-    load_cons(u0, g.ps, g.ix(n, p), U);
-    r = gh ? 1.0 : g.r(n, p);
-    q = fast_prim(U, r, gm1, gh);
+// load_cons through L2: another SM's writes of the same launch are seen.
+MPD_HD void load_cons_l2(const double *base, size_t ps, size_t i, double u[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+#ifdef __CUDA_ARCH__
+        u[k] = __ldcg(base + (size_t)k * ps + i);
+#else
+        u[k] = base[(size_t)k * ps + i];
+#endif
+    }
 }
 
-// The fast interior's new conserved values of cell (l, m), 1 <= l <= L,
-// 2 <= m <= M, computed on their own from the step's input state u0: the
-// operations of lf_tma_kernel's warp in the same order (A from point row
-// l-1; B from the east and west points' shares, which the warp moves by
-// shuffles, and the point's own sources; closed with point row l+1), so the
-// result is bit-identical to the value that kernel stores for the cell.
-MPD_HD void fast_cell_alone(const Geo &g, const double *u0, double dt, int l, int m,
-                            double out[8]) {
+// The five points the fast interior's warp folds into cell (l, m), 1 <= l <= L,
+// 2 <= m <= M: south (l-1), east (m+1), west (m-1), the cell, north (l+1).
+struct FastStencil {
+    double U[5][8];  // conserved values of the step's input state
+    double r[5];     // radii (1 at a ghost point)
+    bool ghost[5];   // U = 0, every primitive 0
+    double hdr;
+
+    MPD_HD void place(const Geo &g, int l, int m) {
+        const int n[5] = {l - 1, l, l, l, l + 1}, p[5] = {m, m + 1, m - 1, m, m};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            ghost[k] = n[k] <= 0 || n[k] >= g.L + 1 || p[k] > g.M + 1;
+            r[k] = ghost[k] ? 1.0 : g.r(n[k], p[k]);
+        }
+        hdr = g.hdr[l];
+    }
+    MPD_HD void load(const Geo &g, const double *u0, int l, int m) {
+        const int n[5] = {l - 1, l, l, l, l + 1}, p[5] = {m, m + 1, m - 1, m, m};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) load_cons_l2(u0, g.ps, g.ix(n[k], p[k]), U[k]);
+    }
+};
+
+// The fast interior's new conserved values of a cell, computed on their own
+// from its stencil: the operations of lf_tma_kernel's warp in the same order
+// (A from the south point; B from the east and west points' shares, which the
+// warp moves by shuffles, and the point's own sources; closed with the north
+// point), so the result is bit-identical to the value that kernel stores for
+// the cell.
+MPD_HD void fast_cell_of(const Geo &g, const FastStencil &x, double dt, double out[8]) {
     const double gm1 = g.gamma - 1.0;
     const double kz = dt * (0.5 / g.dz);
-    double U[8], Gz[8], A[9], B[9], S[10];
-    FastPrim q;
-    double r;
-    fast_point(g, u0, l - 1, m, gm1, U, q, r);
-    fast_gz(U, q, r, Gz);
-    fast_a(U, Gz, kz, A);
-    const double kr = dt * g.hdr[l];
+    double Gz[8], A[9], B[9], S[10];
+    FastPrim q = fast_prim(x.U[0], x.r[0], gm1, x.ghost[0]);
+    fast_gz(x.U[0], q, x.r[0], Gz);
+    fast_a(x.U[0], Gz, kz, A);
+    const double kr = dt * x.hdr;
     {
-        double Ue[8], Uw[8], Gre[8], Grw[8], re, rw;
-        FastPrim qe, qw;
-        fast_point(g, u0, l, m + 1, gm1, Ue, qe, re);
-        fast_gr(Ue, qe, re, Gre);
-        fast_point(g, u0, l, m - 1, gm1, Uw, qw, rw);
-        fast_gr(Uw, qw, rw, Grw);
+        double Gre[8], Grw[8];
+        const FastPrim qe = fast_prim(x.U[1], x.r[1], gm1, x.ghost[1]);
+        fast_gr(x.U[1], qe, x.r[1], Gre);
+        const FastPrim qw = fast_prim(x.U[2], x.r[2], gm1, x.ghost[2]);
+        fast_gr(x.U[2], qw, x.r[2], Grw);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const double ce = (k == 7) ? 0.25 * Ue[7] : fma(kr, Gre[k], 0.25 * Ue[k]);
-            const double cw = (k == 7) ? 0.25 * Uw[7] : fma(-kr, Grw[k], 0.25 * Uw[k]);
+            const double ce = (k == 7) ? 0.25 * x.U[1][7] : fma(kr, Gre[k], 0.25 * x.U[1][k]);
+            const double cw = (k == 7) ? 0.25 * x.U[2][7] : fma(-kr, Grw[k], 0.25 * x.U[2][k]);
             B[k] = ce + cw;
         }
         const double d7 = Gre[7] - Grw[7];
-        fast_point(g, u0, l, m, gm1, U, q, r);
+        q = fast_prim(x.U[3], x.r[3], gm1, x.ghost[3]);
         B[2] = fma(dt, fma(q.rho * q.vphi, q.vphi, q.P) - q.Hphi * q.Hphi, B[2]);
         B[3] = fma(dt, fma(-q.rho * q.vr, q.vphi, q.Hphi * q.Hr), B[3]);
         B[4] = fma(-q.p * kr, d7, B[4]);
         B[8] = q.p;
     }
     fast_sum(A, B, S);
-    fast_point(g, u0, l + 1, m, gm1, U, q, r);
-    fast_gz(U, q, r, Gz);
-    fast_finish(S, U, Gz, kz, out);
+    q = fast_prim(x.U[4], x.r[4], gm1, x.ghost[4]);
+    fast_gz(x.U[4], q, x.r[4], Gz);
+    fast_finish(S, x.U[4], Gz, kz, out);
+}
+
+// fast_cell_of cell (l, m) of input state u0.
+MPD_HD void fast_cell_alone(const Geo &g, const double *u0, double dt, int l, int m,
+                            double out[8]) {
+    FastStencil x;
+    x.place(g, l, m);
+    x.load(g, u0, l, m);
+    fast_cell_of(g, x, dt, out);
 }
 
 // Everything one boundary step reads.
@@ -833,6 +895,69 @@ MPD_HD void eval_segment(const BcView &v, const SegDesc &d, int l, int m, int ln
         }
         out.v[j] = val;
     }
+}
+
+// The geometry a cell's binary fields may read: cell (l, m), neighbour (ln, mn).
+struct RingGeo {
+    double dr, r, rz, z, rnb, rznb;
+};
+
+MPD_HD RingGeo ring_geo(const Geo &g, int l, int m, int ln, int mn) {
+    RingGeo x;
+    x.dr = g.dr[l];
+    x.r = g.r(l, m);
+    x.rz = g.rz(l, m);
+    x.z = (double)(l - 1) * g.dz;
+    x.rnb = g.r(ln, mn);
+    x.rznb = g.rz(ln, mn);
+    return x;
+}
+
+// One operand of a binary field.  Slots: 8 primitive values with get(j) and
+// set(j, v) (the neighbour's, the cell's own).
+template <class Slots>
+MPD_HD double ring_operand(const RingGeo &x, int sym, double c, const Slots &nb,
+                           const Slots &cur) {
+    if (sym < 0) return c;
+    if (sym < RS_CUR0) return nb.get(sym);
+    if (sym < RS_DR) return cur.get(sym - RS_CUR0);
+    double v = x.rznb;
+    v = sym == RS_DR ? x.dr : v;
+    v = sym == RS_R ? x.r : v;
+    v = sym == RS_RZ ? x.rz : v;
+    v = sym == RS_Z ? x.z : v;
+    return sym == RS_RNB ? x.rnb : v;
+}
+
+// eval_segment for a ring-table segment: the 8 new primitives of a cell from
+// its neighbour's (nb), the same operations on the same operands.  AxisLF
+// fields take keep[j].  cur: the cell's own slots, scratch for fields that
+// read fields evaluated before them.
+template <class Slots>
+MPD_HD void ring_eval(const RingSeg &d, const RingGeo &x, const Slots &nb, const Slots &cur,
+                      const double keep[8], double q[8]) {
+    const unsigned int neu = d.neu, axis = d.axis;
+    const int nbin = d.nbin < 8 ? d.nbin : 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = nb.get(j);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const double v = d.value[j];
+        q[j] = (neu >> j & 1u) ? q[j] + v : v;
+        if (axis >> j & 1u) q[j] = keep[j];
+    }
+    if (nbin == 0) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cur.set(j, q[j]);
+#pragma unroll 1
+    for (int b = 0; b < nbin; ++b) {
+        const RingBin &e = d.bin[b];
+        const double a = ring_operand(x, e.fa, e.ca, nb, cur);
+        const double c = ring_operand(x, e.fb, e.cb, nb, cur);
+        cur.set(e.j & 7, bc_binop(e.op, a, c));
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = cur.get(j);
 }
 
 // Physical primitives of (1, m) after the L_LO face; covered = false if no
@@ -1126,6 +1251,180 @@ MPD_HD void bc_ring_final(const BcView &v, int l, int m, double u[8]) {
         return;
     }
     for (int k = 0; k < 8; ++k) u[k] = 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// The ring from a ring table, each cell on its own from the step's input
+// state: the interior value its face reads is recomputed (fast_cell_of), so
+// nothing waits for the interior.  Values are bc_ring_final's, bit for bit.
+// ---------------------------------------------------------------------------
+
+// What a ring cell needs besides the state, and the stencil of the interior
+// cell its face reads.
+struct RingLane {
+    int l, m, ln, mn;  // the cell; the neighbour of its first evaluation
+    int is, is2;       // segments of the first and second evaluation
+    bool act, two, old, m_lo;
+    RingGeo x, x2;
+    FastStencil f;
+
+    MPD_HD void place(const Geo &g, const RingTable &t, int i) {
+        act = i < ring_count(g) && ring_cell(g, i, l, m);
+        if (!act) return;
+        // first evaluation: face, index k, cell (l1, m1), neighbour (ln, mn)
+        const int L = g.L, M = g.M;
+        two = (l == 1 && m == M + 1) || (l == L && (m == 1 || m == M + 1));
+        old = l == 1 && m == 1;
+        int face, k, l1 = l, m1 = m;
+        if (l == 1) {
+            m1 = two ? M : m;
+            face = FACE_L_LO, k = m1, ln = 2, mn = m1;
+        } else if (l == L && !two) {
+            face = FACE_L_HI, k = m, ln = L - 1, mn = m;
+        } else {
+            l1 = two ? L - 1 : l;
+            face = m == 1 ? FACE_M_LO : FACE_M_HI, k = l1, ln = l1, mn = m == 1 ? 2 : M;
+        }
+        m_lo = face == FACE_M_LO;
+        is = t.cov[face * t.len + k] & (kRingSegments - 1);
+        is2 = 0;
+        x = ring_geo(g, l1, m1, ln, mn);
+        if (two) {
+            const int f2 = l == 1 ? FACE_M_HI : FACE_L_HI;
+            is2 = t.cov[f2 * t.len + (l == 1 ? 1 : m)] & (kRingSegments - 1);
+            x2 = ring_geo(g, l, m, l1, m1);
+        }
+        f.place(g, ln, old ? 2 : mn);
+    }
+    // (1, 1) reads the old (2, 1): the west point of (2, 2)'s stencil
+    MPD_HD void load(const Geo &g, const double *u0) {
+        if (act) f.load(g, u0, ln, old ? 2 : mn);
+    }
+};
+
+template <class Slots>
+MPD_HD void ring_put(const Slots &a, const FastPrim &q) {
+    const double v[8] = {q.rho, q.vz, q.vr, q.vphi, q.Hz, q.Hr, q.Hphi, q.e};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a.set(j, v[j]);
+}
+
+// Old primitives of cell (l, m) of the input state at radius r (recon_bc's
+// operations).
+MPD_HD FastPrim ring_old(const Geo &g, const double *u0, int l, int m, double r, double U[8]) {
+    load_cons_l2(u0, g.ps, g.ix(l, m), U);
+    return fast_prim(U, r, g.gamma - 1.0);
+}
+
+MPD_HD AxisPoint ring_axis_point(const FastPrim &q, double r) {
+    AxisPoint a;
+    a.u0 = 0.0;
+    a.r = r;
+    a.vz = q.vz;
+    a.vr = q.vr;
+    a.Hz = q.Hz;
+    a.Hr = q.Hr;
+    a.P = q.P;
+    a.p = q.p;
+    return a;
+}
+
+// The new conserved values uf of ring cell c (c.act, its stencil loaded) and
+// its radius, for the step that takes u0 on by dt.  A cell is one segment
+// evaluation on its neighbour's new state; three corners take two ((1, M+1)
+// reads L_LO's (1, M), (L, 1) and (L, M+1) the walls' row L-1), and (1, 1)
+// reads the old (2, 1).  nb, cur: scratch.
+template <bool AXIS, class Slots>
+MPD_HD void ring_cell_new(const Geo &g, const RingTable &t, const RingSeg *seg,
+                          const RingLane &c, const double *u0, double dt, const Slots &nb,
+                          const Slots &cur, double uf[8], double &r) {
+    const int l = c.l;
+    const RingSeg &d = seg[c.is];
+    const unsigned int axis = (AXIS && c.m_lo) ? d.axis : 0u;
+    {
+        double U[8];
+        if (c.old) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) U[k] = c.f.U[2][k];
+        } else {
+            fast_cell_of(g, c.f, dt, U);
+        }
+        ring_put(nb, fast_prim(U, c.x.rnb, g.gamma - 1.0));
+    }
+    double keep[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    FastPrim oc;
+    if (AXIS && axis) {
+        // the wall cell's old value: the west point of its neighbour's stencil
+        oc = fast_prim(c.f.U[2], c.x.r, g.gamma - 1.0);
+        keep[Q_RHO] = oc.rho;
+        keep[Q_VZ] = oc.vz;
+        keep[Q_E] = oc.e;
+        keep[Q_HZ] = oc.Hz;
+    }
+    Prim q;
+    ring_eval(d, c.x, nb, cur, keep, q.v);
+    r = c.x.r;
+    if (c.two) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) nb.set(j, q.v[j]);
+        ring_eval(seg[c.is2], c.x2, nb, cur, keep, q.v);
+        r = c.x2.r;
+    }
+    phys_to_prim_u(q, r, uf);
+    if (!AXIS || !axis || c.two) return;
+    // m_lo_final_u's overwrites
+    const double rn = g.r(l + 1, 1), rs = g.r(l - 1, 1);
+    double un[8], us[8];
+    const FastPrim on = ring_old(g, u0, l + 1, 1, rn, un);
+    const FastPrim os = ring_old(g, u0, l - 1, 1, rs, us);
+    AxisPoint C = ring_axis_point(oc, r), N = ring_axis_point(on, rn),
+              S = ring_axis_point(os, rs), E;
+    C.vz = q.v[Q_VZ];
+    C.vr = q.v[Q_VR];
+    C.Hz = q.v[Q_HZ];
+    C.Hr = q.v[Q_HR];
+    E.r = c.x.rnb;
+    E.vz = nb.get(Q_VZ);
+    E.vr = nb.get(Q_VR);
+    E.Hz = nb.get(Q_HZ);
+    E.Hr = nb.get(Q_HR);
+    E.P = E.p = E.u0 = 0.0;
+    // (l-1, 1) as the segment loop leaves it: L_LO's corner, what the same
+    // segment leaves (AxisLF keeps the old value), or an earlier segment's
+    const int f3 = l == 2 ? FACE_L_LO : FACE_M_LO;
+    const int is3 = t.cov[f3 * t.len + (l == 2 ? 1 : l - 1)] & (kRingSegments - 1);
+    if (l > 2 && is3 == c.is) {
+        S.vz = (axis >> Q_VZ & 1u) ? os.vz : d.value[Q_VZ];
+        S.Hz = (axis >> Q_HZ & 1u) ? os.Hz : d.value[Q_HZ];
+    } else {
+        const int ls = l == 2 ? 2 : l - 1, ms = l == 2 ? 1 : 2;
+        const RingGeo xs = ring_geo(g, l - 1, 1, ls, ms);
+        double U[8];
+        if (l == 2)
+            load_cons_l2(u0, g.ps, g.ix(ls, ms), U);
+        else
+            fast_cell_alone(g, u0, dt, ls, ms, U);
+        ring_put(nb, fast_prim(U, xs.rnb, g.gamma - 1.0));
+        const double ks[8] = {os.rho, os.vz, 0.0, 0.0, os.Hz, 0.0, 0.0, os.e};
+        Prim qs;
+        ring_eval(seg[is3], xs, nb, cur, ks, qs.v);
+        S.vz = qs.v[Q_VZ];
+        S.Hz = qs.v[Q_HZ];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int kc = a == 0 ? 0 : (a == 1 ? 1 : (a == 2 ? 4 : 6));
+        const int kp = a == 0 ? Q_RHO : (a == 1 ? Q_VZ : (a == 2 ? Q_E : Q_HZ));
+        C.u0 = c.f.U[2][kc];
+        N.u0 = un[kc];
+        S.u0 = us[kc];
+        E.u0 = c.f.U[3][kc];
+        const double v = a == 0   ? axis_u1(C, N, S, E, dt, g.dz, c.x.dr)
+                         : a == 1 ? axis_u2(C, N, S, E, dt, g.dz, c.x.dr)
+                         : a == 2 ? axis_u5(C, N, S, E, dt, g.dz, c.x.dr)
+                                  : axis_u7(C, N, S, E, dt, g.dz, c.x.dr);
+        if (axis >> kp & 1u) uf[kc] = v;
+    }
 }
 
 }  // namespace mpd

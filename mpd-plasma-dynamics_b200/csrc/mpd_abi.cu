@@ -17,6 +17,7 @@
 #include "lf_fast.cuh"
 #include "lf_pair.cuh"
 #include "lf_persist.cuh"
+#include "lf_step.cuh"
 #include "lf_tma.cuh"
 
 namespace mpd {
@@ -113,6 +114,11 @@ struct mpd_solver {
     bool overlap_ok = false;                 // bc_overlap_kernel fits beside the interior
     int overlap_blocks = 0;                  // its grid: at most one block per SM
     bool ring_beside = false;                // the interior just launched left the ring to it
+    bool ring_ok = false;                    // the configuration has a ring table
+    bool whole_step = false;                 // the kernel just launched was a whole step
+    mpd::RingTable ring{};                   // the ring inside the interior's rows
+    mpd::StepPlan step_plan;                 // lf_step_kernel's one wave
+    unsigned char *d_ring = nullptr;         // the table's segments and cover
     mpd::TmaPlan pplan;                      // persistent launch (cooperative wave)
     bool persist_ok = false;                 // the persistent engine can run here
     mpd::GridSync *gsync = nullptr;          // its barrier and reduction words
@@ -133,7 +139,7 @@ struct mpd_solver {
     int with_prev = 0;
     long long host_step = 0;
     cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0, graph_check = 0, graph_resid = 0;
+    int graph_steps = 0, graph_check = 0, graph_resid = 0, graph_every = 0, graph_at = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, snap_ev = nullptr, stage_ev = nullptr;
     bool snap_pending = false;
     size_t dev_bytes = 0;
@@ -187,6 +193,7 @@ void FreeAll(mpd_solver *s) {
     cudaFree(s->d_seg);
     cudaFree(s->d_code);
     cudaFree(s->d_consts);
+    cudaFree(s->d_ring);
     if (s->h_st) cudaFreeHost(s->h_st);
     if (s->h_ring) cudaFreeHost(s->h_ring);
     for (cudaEvent_t e : s->ev_end)
@@ -269,6 +276,8 @@ int InitFromIc(mpd_solver *s) {
     init.max_steps = LLONG_MAX;
     init.want_ws = 1;
     init.resid_every = 1;
+    init.hot.run.T = init.T;
+    init.hot.run.max_steps = init.max_steps;
     *s->h_st = init;
     MPD_CK(cudaMemcpyAsync(s->st, s->h_st, sizeof(mpd::DevState), cudaMemcpyHostToDevice,
                            s->stream));
@@ -291,6 +300,19 @@ int InitFromIc(mpd_solver *s) {
 #define MPD_INTERIOR_PAIR 0
 #endif
 
+// Whether fast steps of the handle are one lf_step_kernel each.
+bool WholeStep(const mpd_solver *s) {
+    return s->ring_ok && !s->ring_overlap && !MPD_INTERIOR_PAIR;
+}
+
+// parity: that of the step count the launch starts from, -1 where unknown.
+int LaunchStep(mpd_solver *s, bool use_state_dt, double dt, bool want_ws, int slot, int parity) {
+    MPD_CK(mpd::launch_lf_step(s->g, s->step_plan, s->tmap[0], s->tmap[1], s->buf[0], s->buf[1],
+                               s->st, dt, use_state_dt ? 1 : 0, want_ws, s->ring, slot,
+                               parity, s->stream));
+    return MPD_OK;
+}
+
 // alone: launches of the interior kernel with no boundary kernel after them
 // (per-kernel timing): the ring-beside form's rows and stores, with the
 // next launch let in only once a block's rows are done.
@@ -299,6 +321,11 @@ int LaunchInterior(mpd_solver *s, bool first, bool use_state_dt, double dt, bool
     const mpd::Geo &g = s->g;
     const int usd = use_state_dt ? 1 : 0;
     s->ring_beside = false;
+    s->whole_step = false;
+    if (!first && !variant && WholeStep(s)) {
+        s->whole_step = true;
+        return LaunchStep(s, use_state_dt, dt, want_ws, 0, (int)(s->host_step & 1));
+    }
     if (first || s->precision == MPD_PRECISION_EXACT) {
         dim3 block(32, 8);
         dim3 grid((g.M - 1 + 31) / 32, (g.L + 7) / 8);
@@ -323,7 +350,14 @@ int LaunchInterior(mpd_solver *s, bool first, bool use_state_dt, double dt, bool
     return MPD_OK;
 }
 
-int LaunchBoundary(mpd_solver *s, bool use_state_dt, double dt) {
+// What ends the step LaunchInterior began: the controller of a whole step, or
+// the boundary kernel and its controller.
+int LaunchBoundary(mpd_solver *s, bool use_state_dt, double dt, bool want_ws) {
+    if (s->whole_step) {
+        s->whole_step = false;
+        MPD_CK(mpd::launch_finish_steps(s->g, s->st, want_ws, 1, s->stream));
+        return MPD_OK;
+    }
     const int nring = mpd::ring_count(s->g);
     const size_t smem = MPD_BC_SMEM_SEG ? s->bc.nseg_total * sizeof(mpd::SegDesc) : 0;
     if (s->ring_beside) {
@@ -342,13 +376,9 @@ int LaunchBoundary(mpd_solver *s, bool use_state_dt, double dt) {
     return MPD_OK;
 }
 
-int EnqueueStep(mpd_solver *s, bool first, bool use_state_dt, double dt, bool with_check,
-                bool want_ws, bool with_residual) {
-    const mpd::Geo &g = s->g;
-    int rc = LaunchInterior(s, first, use_state_dt, dt, want_ws);
-    if (rc != MPD_OK) return rc;
-    rc = LaunchBoundary(s, use_state_dt, dt);
-    if (rc != MPD_OK) return rc;
+// The relative-change check (where the controller found it due) and the
+// residual pass of the step that just ended.
+int EnqueueChecks(mpd_solver *s, bool with_check, bool with_residual) {
     if (with_check) {
         mpd::change_kernel<<<kRedBlocks, 256, 0, s->stream>>>(Bufs(s), s->prev, s->partials, 1, 1);
         mpd::change_finish_kernel<<<1, 256, 2 * kRedBlocks * sizeof(double), s->stream>>>(
@@ -356,10 +386,20 @@ int EnqueueStep(mpd_solver *s, bool first, bool use_state_dt, double dt, bool wi
         MPD_CK(cudaGetLastError());
     }
     if (with_residual) {
-        mpd::residual_kernel<<<s->resid_blocks, 256, 0, s->stream>>>(g, s->buf[0], s->buf[1], s->st, 0);
+        mpd::residual_kernel<<<s->resid_blocks, 256, 0, s->stream>>>(s->g, s->buf[0], s->buf[1],
+                                                                     s->st, 0);
         MPD_CK(cudaGetLastError());
     }
     return MPD_OK;
+}
+
+int EnqueueStep(mpd_solver *s, bool first, bool use_state_dt, double dt, bool with_check,
+                bool want_ws, bool with_residual) {
+    int rc = LaunchInterior(s, first, use_state_dt, dt, want_ws);
+    if (rc != MPD_OK) return rc;
+    rc = LaunchBoundary(s, use_state_dt, dt, want_ws);
+    if (rc != MPD_OK) return rc;
+    return EnqueueChecks(s, with_check, with_residual);
 }
 
 int SyncState(mpd_solver *s) {
@@ -373,6 +413,26 @@ int SyncState(mpd_solver *s) {
 }
 
 int PushState(mpd_solver *s) {
+    // lf_step_kernel starts from slot 0
+    mpd::DevState &h = *s->h_st;
+    mpd::StepCtl c{};
+    c.t = h.t;
+    c.dt = h.dt;
+    c.dt_used = h.dt_used;
+    c.last_ws = h.last_ws;
+    c.step = h.step;
+    c.done = h.done;
+    c.nonfinite = h.nonfinite;
+    c.ws_valid = h.ws_valid;
+    h.hot.ctl[0] = c;
+    h.hot.run.T = h.T;
+    h.hot.run.cfl = h.cfl;
+    h.hot.run.growth = h.growth;
+    h.hot.run.dt_min = h.dt_min;
+    h.hot.run.dt_max = h.dt_max;
+    h.hot.run.max_steps = h.max_steps;
+    h.hot.run.run_mode = h.run_mode;
+    h.hot.run.adaptive = h.adaptive;
     MPD_CK(cudaMemcpyAsync(s->st, s->h_st, sizeof(mpd::DevState), cudaMemcpyHostToDevice,
                            s->stream));
     MPD_CK(cudaStreamSynchronize(s->stream));
@@ -386,10 +446,18 @@ int CheckHandle(mpd_solver *s) {
     return MPD_OK;
 }
 
-int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resid_every) {
-    const int key = (with_check ? 1 : 0) | (want_ws ? 2 : 0) | (s->ring_overlap ? 4 : 0);
+// parity: that of the step count every launch of the graph starts from, -1
+// where it may vary (a hint: a launch that finds another count is only slower).
+// check_every / check_at: the relative-change check follows the steps i (from
+// 1) with i % check_every == check_at; check_at < 0: every step (the
+// controller's own due flag decides).
+int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resid_every,
+               int check_every, int check_at, int parity) {
+    const int key = (with_check ? 1 : 0) | (want_ws ? 2 : 0) | (s->ring_overlap ? 4 : 0) |
+                    (WholeStep(s) ? 8 * (parity + 2) : 0);
     if (s->graph && s->graph_steps == steps && s->graph_check == key &&
-        s->graph_resid == resid_every)
+        s->graph_resid == resid_every &&
+        (!with_check || (s->graph_every == check_every && s->graph_at == check_at)))
         return MPD_OK;
     if (s->graph) {
         cudaGraphExecDestroy(s->graph);
@@ -398,9 +466,22 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
     cudaGraph_t graph = nullptr;
     MPD_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int rc = MPD_OK;
+    int slot = 0;
     for (int i = 0; i < steps && rc == MPD_OK; ++i) {
         const bool res = resid_every > 0 && (i + 1) % resid_every == 0;
-        rc = EnqueueStep(s, false, true, 0.0, with_check, want_ws, res);
+        const bool check = with_check && (check_at < 0 || (i + 1) % check_every == check_at);
+        if (!WholeStep(s)) {
+            rc = EnqueueStep(s, false, true, 0.0, check, want_ws, res);
+            continue;
+        }
+        rc = LaunchStep(s, true, 0.0, want_ws, slot, parity < 0 ? -1 : (parity + i) & 1);
+        slot ^= 1;
+        if (rc == MPD_OK && (res || check || i == steps - 1)) {
+            const cudaError_t ef = mpd::launch_finish_steps(s->g, s->st, want_ws, slot, s->stream);
+            if (ef != cudaSuccess) rc = Fail(MPD_ERR_CUDA, cudaGetErrorString(ef));
+            slot = 0;
+            if (rc == MPD_OK) rc = EnqueueChecks(s, check, res);
+        }
     }
     const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
     if (rc != MPD_OK) {
@@ -414,6 +495,8 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
     s->graph_steps = steps;
     s->graph_check = key;
     s->graph_resid = resid_every;
+    s->graph_every = check_every;
+    s->graph_at = check_at;
     return MPD_OK;
 }
 
@@ -580,6 +663,29 @@ int mpd_create(const mpd_config *cfg, const mpd_geometry *geom, const double *ph
             const int groups = (mpd::ring_count(g) + 31) / 32;
             s->overlap_blocks = groups < sms ? groups : sms;
             s->overlap_ok = g.L >= 4 && s->overlap_blocks > 0;
+        }
+        // the boundary ring inside the interior's rows, where the faces allow it
+        mpd::CompiledRing cr;
+        if (mpd::CompileRing(cbc, s->L, s->M, cr)) {
+            const size_t nseg = cr.seg.size() * sizeof(mpd::RingSeg);
+            STEP(DevAlloc(s, &s->d_ring, nseg + cr.cov.size()));
+            if (cudaMemcpy(s->d_ring, cr.seg.data(), nseg, cudaMemcpyHostToDevice) !=
+                    cudaSuccess ||
+                cudaMemcpy(s->d_ring + nseg, cr.cov.data(), cr.cov.size(),
+                           cudaMemcpyHostToDevice) != cudaSuccess) {
+                FreeAll(s);
+                return Fail(MPD_ERR_CUDA, "boundary table upload failed");
+            }
+            s->ring.seg = reinterpret_cast<const mpd::RingSeg *>(s->d_ring);
+            s->ring.cov = s->d_ring + nseg;
+            s->ring.len = cr.len;
+            s->ring.nseg = static_cast<int>(cr.seg.size());
+            s->ring.has_axis = cr.has_axis;
+            if (mpd::plan_lf_step(g, s->device, s->ring, s->step_plan) != cudaSuccess) {
+                FreeAll(s);
+                return Fail(MPD_ERR_CUDA, "occupancy query for the step kernel failed");
+            }
+            s->ring_ok = true;
         }
         // the persistent engine needs cooperative launch and a strip per warp
         s->persist_ok = mpd::plan_lf_persist(g, s->device, s->pplan) == cudaSuccess;
@@ -931,9 +1037,20 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
         per_graph = (per_graph / p->check_frequency) * p->check_frequency;
     if (p->residual_every > 0 && per_graph % p->residual_every != 0)
         per_graph = (per_graph / p->residual_every + 1) * p->residual_every;
-    rc = BuildGraph(s, per_graph, with_check, want_ws, p->residual_every);
-    if (rc != MPD_OK) return rc;
     long long taken_before = (!h.done && s->host_step == 0) ? 1 : 0;  // the exact first step
+    // Every graph launch starts a multiple of per_graph steps after the run's
+    // first (the monitored loop stops in between and does not): where that is
+    // a multiple of the check interval, the check's nodes follow only the
+    // steps it is due after.
+    int check_at = -1;
+    if (with_check && !monitored && per_graph % p->check_frequency == 0)
+        check_at = static_cast<int>((p->check_frequency - (step0 + taken_before) %
+                                     p->check_frequency) % p->check_frequency);
+    const int parity =
+        monitored || per_graph % 2 != 0 ? -1 : static_cast<int>((step0 + taken_before) & 1);
+    rc = BuildGraph(s, per_graph, with_check, want_ws, p->residual_every, p->check_frequency,
+                    check_at, parity);
+    if (rc != MPD_OK) return rc;
     const long long end = step0 + p->max_steps;
     for (;;) {
         // steps this segment may take: to the controller's current stop
@@ -1280,7 +1397,16 @@ int mpd_set_expression_ic(mpd_solver *s, const char *const exprs[8], int n_vars,
 int mpd_set_ring_overlap(mpd_solver *s, int on) {
     int rc = CheckHandle(s);
     if (rc != MPD_OK) return rc;
-    MPD_CK(cudaStreamSynchronize(s->stream));
+    rc = SyncState(s);
+    if (rc != MPD_OK) return rc;
+    if (on && WholeStep(s) && s->h_st->step > 0) {
+        // whole steps leave no wall lines; the boundary kernels start from them
+        const int par = static_cast<int>(s->h_st->step & 1);
+        mpd::wall_lines_kernel<<<(s->L + 127) / 128, 128, 0, s->stream>>>(s->g, s->buf[par],
+                                                                          s->wall[par], s->len);
+        MPD_CK(cudaGetLastError());
+        MPD_CK(cudaStreamSynchronize(s->stream));
+    }
     s->ring_overlap = on ? 1 : 0;
     return MPD_OK;
 }
@@ -1311,7 +1437,7 @@ int mpd_profile_kernels(mpd_solver *s, int steps, double dt, double out_ms[2]) {
         rc = LaunchInterior(s, first, false, dt, true);
         if (rc != MPD_OK) break;
         MPD_CK(cudaEventRecord(ev[3 * i + 1], s->stream));
-        rc = LaunchBoundary(s, false, dt);
+        rc = LaunchBoundary(s, false, dt, true);
         if (rc != MPD_OK) break;
         MPD_CK(cudaEventRecord(ev[3 * i + 2], s->stream));
         s->host_step++;
@@ -1368,6 +1494,7 @@ int mpd_profile_kernel(mpd_solver *s, int which, int launches, double dt, double
     if (which != MPD_KERNEL_RESIDUAL) {
         MPD_CK(cudaMemsetAsync(&s->st->ws_acc, 0, sizeof(unsigned long long), s->stream));
         MPD_CK(cudaMemsetAsync(&s->st->nf_acc, 0, sizeof(unsigned int), s->stream));
+        MPD_CK(cudaMemsetAsync(&s->st->hot.acc, 0, sizeof(s->st->hot.acc), s->stream));
         MPD_CK(cudaStreamSynchronize(s->stream));
     }
     return SyncState(s);

@@ -155,7 +155,7 @@ class GpuSolver:
         The L-inf residual (a separate pass over both state buffers) is
         evaluated every ``residual_every`` steps: by default every 50 steps
         when ``residual_tol`` is set, otherwise only for the final state.
-        ``engine``: "graph" (two kernels per step from captured CUDA graphs),
+        ``engine``: "graph" (one or two kernels per step from captured CUDA graphs),
         "persistent" (one cooperative launch for many steps; fast precision
         without convergence_threshold) or "auto" (graph); both give the same bits.
         ``monitor``: a callable given a ``MonitorReport`` after every
@@ -291,8 +291,8 @@ class GpuSolver:
     @property
     def ring_overlap(self) -> bool:
         """Whether fast steps run the boundary ring beside the interior kernel
-        (bc_overlap_kernel) instead of after it (bc_kernel, the default); both
-        give the same bits.  Setting it takes effect from the next step."""
+        (bc_overlap_kernel) instead of in it or after it (lf_step_kernel or
+        bc_kernel, the default); all give the same bits.  Setting it takes effect from the next step."""
         a = C.c_int()
         self._call("mpd_ring_overlap_active", C.byref(a))
         return bool(a.value)

@@ -1,0 +1,52 @@
+"""The ring evaluated from the ring table and the step's input state alone
+(lf_step_kernel's ring warps), on the CPU, against the general boundary path
+(bc_ring_final) over every kind of layout the table accepts; and what it
+refuses."""
+import numpy as np
+import pytest
+
+from oracle import bind
+from tests import cases, ring_layouts
+from tests.emu import Emu
+
+
+def _has_ring(emu):
+    return bool(emu.lib.mpd_emu_has_ring(emu.h))
+
+
+@pytest.mark.parametrize("L,M", [(4, 3), (5, 4), (12, 9), (40, 31)])
+@pytest.mark.parametrize("make", ring_layouts.ACCEPTED, ids=lambda f: f.__name__)
+def test_table_ring_is_the_general_ring_bitwise(make, L, M):
+    cfg = make(L, M)
+    case = cases.make_case(cfg)
+    a, b = Emu(case, "fast"), Emu(case, "fast")
+    assert _has_ring(a)
+    for _ in range(4):
+        a.advance(1e-6)
+        b.advance(1e-6, order=3)
+        np.testing.assert_array_equal(b.conserved(), a.conserved())
+
+
+@pytest.mark.parametrize("make", ring_layouts.REFUSED, ids=lambda f: f.__name__)
+def test_refused_layouts_keep_the_general_path(make):
+    emu = Emu(cases.make_case(make(12, 9)), "fast")
+    assert not _has_ring(emu)
+
+
+def test_constant_parts_of_an_expression_fold_to_the_interpreters_bits():
+    """amp * 0.2 / r: the constant product meets first, as in the sweep."""
+    for expr in ("1.3 * 0.2 / r", "(beta + 0.1) * r", "-2 * r", "r / (3 * 0.7)"):
+        cfg = ring_layouts.channel(12, 9)
+        cfg.bc_l_lo.segments[0].H_phi = cases.pkg.FieldCond("expression", 0.0, expr)
+        case = cases.make_case(cfg)
+        a, b = Emu(case, "fast"), Emu(case, "fast")
+        assert _has_ring(a)
+        oracle = bind.Port(case.oracle_dict())
+        exact = Emu(case, "exact")
+        for _ in range(3):
+            a.advance(1e-5)
+            b.advance(1e-5, order=3)
+            exact.advance(1e-5)
+            oracle.advance(1e-5)
+            np.testing.assert_array_equal(b.conserved(), a.conserved())
+            np.testing.assert_array_equal(exact.conserved(), oracle.conserved())
