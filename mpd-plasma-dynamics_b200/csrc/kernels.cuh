@@ -351,39 +351,93 @@ __device__ __forceinline__ void step_controller(const Geo &g, DevState *st, long
 // UpdatePhysicalFromU of the neighbours), one thread per cell
 // l in [1, L], m in [2, M].  FIRST: the stencil reads the initial physical
 // planes instead of reconstructing them (step 0 of src/main.cpp:147-148).
+//
+// Bound: FP64 divides (the reference's true divides, 26 in a cell's update and
+// 7 in a point's reconstruction).  A block of kExX x kExY cells reconstructs
+// each of its (kExX + 2) x (kExY + 2) points once into shared memory and every
+// cell reads its five from there; with each cell reconstructing all five for
+// itself it was 35 divides instead of 9 on top of the 26, and 40 loads a cell
+// instead of 11: 337 -> 186 us a launch at 1600 x 640, 103.6 -> 63.7 at
+// 800 x 400 (B200).  Two blocks an SM (128 registers): one (185 registers) 275,
+// three (80, with spills) 175 but 15.0 against 12.5 at 100 x 40 and the
+// thruster's 800 x 400 step 77.6 against 72.2.
+constexpr int kExX = 32, kExY = 8;
+constexpr int kExPX = kExX + 2, kExPY = kExY + 2;
+// a point's values in shared memory: u_1..u_8, then
+enum ExVal { EX_VZ = 8, EX_VR, EX_VPHI, EX_HZ, EX_HR, EX_P, EX_R, EX_COUNT };
+
 template <bool FIRST>
-__global__ void __launch_bounds__(256) lf_exact_kernel(Geo g, double *buf0, double *buf1,
-                                                       const double *__restrict__ ic, DevState *st,
-                                                       double dt_arg, int use_state_dt,
-                                                       double *cphys, int len) {
+__global__ void __launch_bounds__(kExX * kExY, 2)
+    lf_exact_kernel(Geo g, double *buf0, double *buf1, const double *__restrict__ ic,
+                    DevState *st, double dt_arg, int use_state_dt, double *cphys, int len) {
+    __shared__ double sv[EX_COUNT][kExPY][kExPX];
     if (st->done) return;
     const long long step = st->step;
     const double *__restrict__ u0 = (step & 1) ? buf1 : buf0;
     double *__restrict__ u = (step & 1) ? buf0 : buf1;
     const double dt = use_state_dt ? st->dt : dt_arg;
     const int flags = step_flags(st);
-    const int m = 2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int l = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+    const int m0 = 2 + (int)blockIdx.x * kExX, l0 = 1 + (int)blockIdx.y * kExY;
+    const int tid = (int)(threadIdx.y * blockDim.x + threadIdx.x);
+    for (int k = tid; k < kExPX * kExPY; k += kExX * kExY) {
+        const int y = k / kExPX, x = k - y * kExPX;
+        const int l = l0 - 1 + y, m = m0 - 1 + x;
+        if (l > g.L + 1 || m > g.M + 1) continue;  // no cell of the block reads it
+        const size_t i = g.ix(l, m);
+        double U[8];
+        load_cons(u0, g.ps, i, U);
+        const double r = g.r(l, m);
+        Phys q;
+        if (l == 0 || l == g.L + 1) q = phys_zero();
+        else if (FIRST) q = load_phys(ic, g.ps, i);
+        else q = recon_exact(U, r, g.gamma);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) sv[c][y][x] = U[c];
+        sv[EX_VZ][y][x] = q.vz;
+        sv[EX_VR][y][x] = q.vr;
+        sv[EX_VPHI][y][x] = q.vphi;
+        sv[EX_HZ][y][x] = q.Hz;
+        sv[EX_HR][y][x] = q.Hr;
+        sv[EX_P][y][x] = q.P;
+        sv[EX_R][y][x] = r;
+    }
+    __syncthreads();
+    const int m = m0 + (int)threadIdx.x;
+    const int l = l0 + (int)threadIdx.y;
     CellStats cs;
     cs.init();
     if (m <= g.M && l <= g.L) {
         double U[5][8];
         Phys Q[5];
         double R[5];
-        const int ls[5] = {l, l + 1, l - 1, l, l};
-        const int ms[5] = {m, m, m, m + 1, m - 1};
+        const int xs = (int)threadIdx.x + 1, ys = (int)threadIdx.y + 1;
+        const int py[5] = {ys, ys + 1, ys - 1, ys, ys};
+        const int px[5] = {xs, xs, xs, xs + 1, xs - 1};
 #pragma unroll
         for (int p = 0; p < 5; ++p) {
-            const size_t i = g.ix(ls[p], ms[p]);
-            R[p] = g.r(ls[p], ms[p]);
-            load_cons(u0, g.ps, i, U[p]);
-            if (ls[p] == 0 || ls[p] == g.L + 1) Q[p] = phys_zero();
-            else if (FIRST) Q[p] = load_phys(ic, g.ps, i);
-            else Q[p] = recon_exact(U[p], R[p], g.gamma);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) U[p][c] = sv[c][py[p]][px[p]];
+            Q[p].vz = sv[EX_VZ][py[p]][px[p]];
+            Q[p].vr = sv[EX_VR][py[p]][px[p]];
+            Q[p].vphi = sv[EX_VPHI][py[p]][px[p]];
+            Q[p].Hz = sv[EX_HZ][py[p]][px[p]];
+            Q[p].Hr = sv[EX_HR][py[p]][px[p]];
+            Q[p].P = sv[EX_P][py[p]][px[p]];
+            Q[p].Hphi = U[p][5];  // u_6 is H_phi
+            R[p] = sv[EX_R][py[p]][px[p]];
+        }
+        // the centre's rho and p (sources): the reconstruction's operations
+        const size_t ic0 = g.ix(l, m);
+        if (FIRST) {
+            Q[0].rho = ic[P_RHO * g.ps + ic0];
+            Q[0].p = ic[P_PG * g.ps + ic0];
+        } else {
+            Q[0].rho = U[0][0] / R[0];
+            const double e = U[0][4] / U[0][0];
+            Q[0].p = (g.gamma - 1.0) * Q[0].rho * e;
         }
         double out[8];
         lf_cell_exact(U, Q, R, dt, g.dz, g.dr[l], out);
-        const size_t ic0 = g.ix(l, m);
 #pragma unroll
         for (int k = 0; k < 8; ++k) u[(size_t)k * g.ps + ic0] = out[k];
         // cells no boundary face can overwrite feed the wave speed; cells the

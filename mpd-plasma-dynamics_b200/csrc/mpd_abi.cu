@@ -327,8 +327,8 @@ int LaunchInterior(mpd_solver *s, bool first, bool use_state_dt, double dt, bool
         return LaunchStep(s, use_state_dt, dt, want_ws, 0, (int)(s->host_step & 1));
     }
     if (first || s->precision == MPD_PRECISION_EXACT) {
-        dim3 block(32, 8);
-        dim3 grid((g.M - 1 + 31) / 32, (g.L + 7) / 8);
+        dim3 block(mpd::kExX, mpd::kExY);
+        dim3 grid((g.M - 1 + mpd::kExX - 1) / mpd::kExX, (g.L + mpd::kExY - 1) / mpd::kExY);
         if (first)
             mpd::lf_exact_kernel<true><<<grid, block, 0, s->stream>>>(
                 g, s->buf[0], s->buf[1], s->ic, s->st, dt, usd, s->cphys, s->len);
