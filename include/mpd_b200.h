@@ -362,6 +362,39 @@ typedef struct mpd_gemm_desc {
 int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream);
 int mpd_nn_wait_status(void *stream);
 
+/* A (rows x K) FP32 operand at src[row * s_row + k * s_k], rounded to BF16 as
+ * the GEMM rounds it and laid out as the tensor core reads it, for operands
+ * that stay the same over many calls: blocks of block_k (a multiple of 8)
+ * columns of K, in each ceil(rows / 128) tiles of 128 rows, zero past the
+ * edges: ceil(K / block_k) * ceil(rows / 128) * 128 * block_k * 2 bytes. */
+int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int rows, int K,
+                       int block_k, void *image, void *stream);
+
+/* One layer of the network in one kernel, with the roundings of the GEMMs and
+ * element-wise kernels it stands for; rows are B samples of P points:
+ *   s = h W + basis U[b]     h: rows x 64, W(n, k) at w[n * w_sn + k * w_sk],
+ *                            basis: image of P x 256 with block_k 256,
+ *                            U: B x 256 x 64, u_work: B * 32 KB of scratch
+ *   MPD_NN_FORWARD  out0 = s + bias; out1 = GELU(out0) (out1 may be NULL)
+ *   MPD_NN_ACT_BWD  out0 = s * GELU'(z_in)
+ *   MPD_NN_PLAIN    out0 = s
+ * With basis == NULL: s = h W with n_out = 128 columns, MPD_NN_FORWARD only
+ * (B = 1, P = all rows).  h, out0, out1, z_in, basis and u_work start on
+ * 16-byte boundaries. */
+enum { MPD_NN_FORWARD = 0, MPD_NN_ACT_BWD = 1, MPD_NN_PLAIN = 2 };
+typedef struct mpd_layer_desc {
+    int P, B, n_out, epilogue;
+    const float *h, *w;
+    long long w_sn, w_sk;
+    const void *basis;
+    const float *U;
+    void *u_work;
+    const float *bias, *z_in;
+    float *out0, *out1;
+} mpd_layer_desc;
+
+int mpd_nn_layer(const mpd_layer_desc *d, void *stream);
+
 /* Element-wise and reduction kernels of the network (FP32, deterministic sums):
  * z += bias (per column), out = GELU(z) (act != 0) or z;  g_z = g_out GELU'(z);
  * out[c] = sum over rows of x[r][c] (work: 128 * cols floats of scratch);

@@ -103,6 +103,14 @@ class GemmDesc(C.Structure):
                 ("work", C.c_void_p), ("work_floats", C.c_longlong)]
 
 
+class LayerDesc(C.Structure):
+    _fields_ = [("P", C.c_int), ("B", C.c_int), ("n_out", C.c_int), ("epilogue", C.c_int),
+                ("h", C.c_void_p), ("w", C.c_void_p), ("w_sn", C.c_longlong),
+                ("w_sk", C.c_longlong), ("basis", C.c_void_p), ("U", C.c_void_p),
+                ("u_work", C.c_void_p), ("bias", C.c_void_p), ("z_in", C.c_void_p),
+                ("out0", C.c_void_p), ("out1", C.c_void_p)]
+
+
 class MpdError(RuntimeError):
     def __init__(self, code: int, msg: str):
         super().__init__(f"{STATUS_NAMES.get(code, code)}: {msg}")
@@ -151,6 +159,9 @@ SIGNATURES = [
                                 C.POINTER(C.c_int), DP, C.POINTER(RunStats), DP, DP]),
     ("mpd_nn_gemm", C.c_int, [C.POINTER(GemmDesc), _VP]),
     ("mpd_nn_wait_status", C.c_int, [_VP]),
+    ("mpd_nn_basis_image", C.c_int, [_VP, C.c_longlong, C.c_longlong, C.c_int, C.c_int, C.c_int,
+                                     _VP, _VP]),
+    ("mpd_nn_layer", C.c_int, [C.POINTER(LayerDesc), _VP]),
     ("mpd_nn_bias_act", C.c_int, [_VP, _VP, _VP, C.c_longlong, C.c_int, C.c_int, _VP]),
     ("mpd_nn_act_bwd", C.c_int, [_VP, _VP, _VP, C.c_longlong, _VP]),
     ("mpd_nn_colsum", C.c_int, [_VP, C.c_longlong, C.c_int, _VP, _VP, _VP]),

@@ -44,6 +44,7 @@ void SetLastError(const std::string &msg);
 
 namespace {
 
+using mpd::mbar_expect_tx;
 using mpd::mbar_init;
 using mpd::mbar_init_fence;
 using mpd::mbar_wait_bounded;
@@ -437,7 +438,98 @@ __global__ void nn_gemm_reduce_kernel(const mpd_gemm_desc d, int ksplit) {
 
 }  // namespace
 
+#include "nn_layer.cuh"
+
+namespace {
+
+int NnLaunched(const char *what) {
+    const cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) return MPD_OK;
+    mpd::SetLastError(std::string(what) + ": " + cudaGetErrorString(e));
+    return MPD_ERR_CUDA;
+}
+
+template <int K2, int NB, int EPI>
+int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
+    constexpr int smem = layer_smem<K2, NB>();
+    static bool attr_set = false;  // per process; the attribute is per function
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            nn_layer_kernel<K2, NB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) {
+            mpd::SetLastError(std::string("mpd_nn_layer: ") + cudaGetErrorString(e));
+            return MPD_ERR_CUDA;
+        }
+        attr_set = true;
+    }
+    const long long items = (long long)a.tiles * a.B;
+    nn_layer_kernel<K2, NB, EPI>
+        <<<(int)(items < 148 ? items : 148), kLyThreads, smem, st>>>(a);
+    return NnLaunched("mpd_nn_layer");
+}
+
+bool Aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
+
+}  // namespace
+
 extern "C" {
+
+int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int rows, int K,
+                       int block_k, void *image, void *stream) {
+    if (!src || !image || rows < 1 || K < 1 || block_k < 8 || block_k % 8 || !Aligned16(image)) {
+        mpd::SetLastError("mpd_nn_basis_image: bad arguments");
+        return MPD_ERR_INVALID;
+    }
+    const int mt = (rows + 127) / 128, nkb = (K + block_k - 1) / block_k;
+    basis_image_kernel<<<148 * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        src, s_row, s_k, rows, K, mt, block_k, nkb, static_cast<uint4 *>(image));
+    return NnLaunched("mpd_nn_basis_image");
+}
+
+int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
+    if (!d || !d->h || !d->w || !d->out0 || d->P < 1 || d->B < 0) {
+        mpd::SetLastError("mpd_nn_layer: NULL operand or bad sizes");
+        return MPD_ERR_INVALID;
+    }
+    const bool spectral = d->basis != nullptr;
+    const bool shape_ok = spectral ? d->n_out == 64 && d->U && d->u_work : d->n_out == 128;
+    const bool epi_ok = d->epilogue == MPD_NN_FORWARD ? d->bias != nullptr
+                        : !spectral                   ? false
+                        : d->epilogue == MPD_NN_ACT_BWD ? d->z_in != nullptr
+                                                        : d->epilogue == MPD_NN_PLAIN;
+    if (!shape_ok || !epi_ok || !Aligned16(d->h) || !Aligned16(d->out0) || !Aligned16(d->out1) ||
+        !Aligned16(d->z_in) || !Aligned16(d->basis) || !Aligned16(d->u_work)) {
+        mpd::SetLastError("mpd_nn_layer: unsupported widths, epilogue or alignment");
+        return MPD_ERR_INVALID;
+    }
+    if (d->B == 0) return MPD_OK;
+    if (d->B > 65535) {
+        mpd::SetLastError("mpd_nn_layer: batch too large for one launch");
+        return MPD_ERR_INVALID;
+    }
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    LayerArgs a;
+    a.h = d->h;
+    a.w = d->w;
+    a.w_sn = d->w_sn;
+    a.w_sk = d->w_sk;
+    a.g_img = static_cast<const unsigned char *>(d->basis);
+    a.u_img = static_cast<const unsigned char *>(d->u_work);
+    a.bias = d->bias;
+    a.z_in = d->z_in;
+    a.out0 = d->out0;
+    a.out1 = d->out1;
+    a.P = d->P;
+    a.B = d->B;
+    a.tiles = (d->P + kLyRows - 1) / kLyRows;
+    if (!spectral) return LaunchLayer<0, 2, kEpiForward>(a, st);
+    const long long units = (long long)d->B * (kLyQ / 8) * kLyW;
+    u_image_kernel<<<(int)((units + 255) / 256 < 148 * 8 ? (units + 255) / 256 : 148 * 8), 256, 0,
+                     st>>>(d->U, d->B, static_cast<uint4 *>(d->u_work));
+    if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyQ, 1, kEpiForward>(a, st);
+    if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyQ, 1, kEpiActBwd>(a, st);
+    return LaunchLayer<kLyQ, 1, kEpiPlain>(a, st);
+}
 
 int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream) {
     if (!d || !d->A || !d->B || !d->C) {

@@ -1,0 +1,438 @@
+// The surrogate's layer product as one persistent kernel (included by
+// nn_gemm.cu, whose tcgen05 helpers it uses):
+//
+//   s = h W  +  G U[b]                 rows = B samples x P grid points, width 64
+//   forward:   z = s + bias;  out = GELU(z) (or out = z: one array)
+//   backward:  s (W and G the transposed operands), or s * GELU'(z)
+//
+// As separate launches the layer moved each row 7 times (h in; z out; z in and
+// out; z in and out, h' out) and read and rounded G once per sample: 1013 us at
+// 16 x 64400 rows against a floor of 121 (h in, z and h' out).  Both products
+// keep their own FP32 accumulator in TMEM and the epilogue adds them, so a
+// value is rounded exactly as by the separate launches.
+//   * one CTA per SM takes an even share of the (128-row tile, sample) items,
+//     samples fastest, so the tile of G (64 KB of BF16) stays in shared memory
+//     over its samples;
+//   * G and U come as images of the tensor core's K-major core-matrix layout
+//     (basis_image_kernel, once per network; u_image_kernel, each call), so
+//     they are bulk copies without any work by the threads; h arrives as FP32
+//     (a tile is 32 KB of contiguous memory) and four warps round it;
+//   * warps 0-7 run the epilogue of item i while the tensor core works on item
+//     i + 1 and the copies of item i + 2 are in flight (TMEM, h and U are
+//     double-buffered).  tcgen05.ld in the 16x256b form gives four lanes a
+//     whole 32-byte sector of a row, so the stores need no transposition.
+// 216 KB of shared memory, 256 TMEM columns, 14 warps.  Measured (B200, both
+// products, bias and GELU): 998 -> 145 us at 16 x 64400 rows (5.5 TB/s of the
+// 792 MB it must move: bound by memory), 75 -> 20 us at 16 x 4100 rows (3 to 4
+// items a CTA: the pipeline's fill and the tile of G are a third of it).
+#pragma once
+
+namespace {
+
+constexpr int kLyW = 64;             // network width: columns of h, K of the first product
+constexpr int kLyQ = 256;            // K of the second product (basis functions)
+constexpr int kLyRows = 128;
+constexpr int kLyEpiWarps = 8, kLyCvtWarps = 4;
+constexpr int kLyThreads = (kLyEpiWarps + kLyCvtWarps + 2) * 32;
+constexpr int kLyGBytes = kLyRows * kLyQ * 2;     // 64 KB
+constexpr int kLyUBytes = kLyQ * kLyW * 2;        // 32 KB
+constexpr int kLyHBytes = kLyRows * kLyW * 4;     // 32 KB
+constexpr int kLyHbBytes = kLyRows * kLyW * 2;    // 16 KB
+constexpr int kLyWBytes = kLyW * kLyW * 2;        // 8 KB per 64 output columns
+constexpr uint32_t kLyTmem = 256;
+
+enum LayerEpilogue { kEpiForward = 0, kEpiActBwd = 1, kEpiPlain = 2 };
+
+struct LayerArgs {
+    const float *h;              // rows x 64
+    const float *w;              // (n, k) at w[n * w_sn + k * w_sk]
+    long long w_sn, w_sk;
+    const unsigned char *g_img;  // tiles of kLyGBytes (K2 != 0)
+    const unsigned char *u_img;  // B x kLyUBytes     (K2 != 0)
+    const float *bias;           // forward
+    const float *z_in;           // kEpiActBwd: GELU' is taken at these
+    float *out0, *out1;          // out1: GELU(out0), or NULL
+    int P, B, tiles;             // rows of one sample, samples, 128-row tiles of one sample
+};
+
+// How items are dealt: CTA c of n takes [total c / n, total (c + 1) / n).
+__device__ __forceinline__ long long layer_first(long long total, int c, int n) {
+    return total * c / n;
+}
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
+                                          uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(dst), "l"(src), "r"(bytes), "r"(bar)
+        : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// 16 TMEM lanes x 32 columns: register 4 j + 2 i + e of lane l holds row
+// l / 4 + 8 i, column 8 j + 2 (l % 4) + e.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float v[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+        "%11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+          "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// The values of earlier tcgen05.ld may be used after this.
+__device__ __forceinline__ void tmem_ld_wait(float v[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                   "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]),
+                   "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                 :
+                 : "memory");
+}
+
+// The tanh-form GELU and its derivative (the same operations as nn_ops.cu's).
+__device__ __forceinline__ float layer_gelu(float x) {
+    const float c = 0.7978845608028654f;
+    const float u = c * (x + 0.044715f * x * x * x);
+    const float t = tanhf(u);
+    return 0.5f * x * (1.0f + t);
+}
+__device__ __forceinline__ float layer_dgelu(float x) {
+    const float c = 0.7978845608028654f;
+    const float u = c * (x + 0.044715f * x * x * x);
+    const float t = tanhf(u);
+    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
+}
+
+template <int K2, int NB>
+constexpr int layer_smem() {
+    return (K2 ? kLyGBytes + 2 * kLyUBytes : 0) + 2 * kLyHBytes + kLyHbBytes + NB * kLyWBytes;
+}
+
+template <int K2, int NB, int EPI>
+__global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs a) {
+    static_assert(K2 == 0 || NB == 1, "one accumulator pair of 64 columns each");
+    extern __shared__ __align__(1024) unsigned char gemm_smem[];
+    __shared__ __align__(8) uint64_t h_full[2], h_free[2], u_full[2], acc_full[2], acc_free[2],
+        g_full, hb_full, hb_free;
+    __shared__ uint32_t tmem_slot;
+    unsigned char *sG = gemm_smem;
+    unsigned char *sU = sG + (K2 ? kLyGBytes : 0);
+    unsigned char *sH = sU + (K2 ? 2 * kLyUBytes : 0);
+    unsigned char *sHb = sH + 2 * kLyHBytes;
+    unsigned char *sW = sHb + kLyHbBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = (long long)a.tiles * a.B;
+    const long long first = layer_first(total, blockIdx.x, gridDim.x);
+    const int items = (int)(layer_first(total, blockIdx.x + 1, gridDim.x) - first);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "r"(kLyTmem)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_addr(&h_full[i]), 1);
+            mbar_init(smem_addr(&h_free[i]), kLyCvtWarps);
+            mbar_init(smem_addr(&u_full[i]), 1);
+            mbar_init(smem_addr(&acc_full[i]), 1);
+            mbar_init(smem_addr(&acc_free[i]), kLyEpiWarps);
+        }
+        mbar_init(smem_addr(&g_full), 1);
+        mbar_init(smem_addr(&hb_full), kLyCvtWarps);
+        mbar_init(smem_addr(&hb_free), 1);
+        mbar_init_fence();
+    }
+    // W rounded once: (n, k) of 64-column block n / 64
+    for (int u = threadIdx.x; u < NB * kLyW * (kLyW / 8); u += kLyThreads) {
+        const int n = u % (NB * kLyW), c = u / (NB * kLyW), nl = n % kLyW;
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = __ldg(a.w + n * a.w_sn + (8 * c + e) * a.w_sk);
+        *reinterpret_cast<uint4 *>(sW + (n / kLyW) * kLyWBytes + (c * (kLyW / 8) + (nl >> 3)) * 128 +
+                                   (nl & 7) * 16) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                       pack_bf16(f[6], f[7]));
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    bool ok = true;
+
+    if (warp < kLyEpiWarps) {
+        // ---- epilogue: rows 32 (warp & 3) .. + 31, columns 32 (warp >> 2) .. + 31 of 64
+        const int quad = warp & 3, col0 = (warp >> 2) * 32;
+        float2 bias[NB][4];
+        if (EPI == kEpiForward) {
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float *bp = a.bias + nb * 64 + col0 + 8 * j + 2 * (lane & 3);
+                    bias[nb][j] = make_float2(bp[0], bp[1]);
+                }
+        }
+        for (int i = 0; i < items; ++i) {
+            const long long it = first + i;
+            const int tile = (int)(it / a.B), b = (int)(it % a.B), buf = i & 1;
+            const int nrows = min(kLyRows, a.P - tile * kLyRows);
+            const int r0 = quad * 32 + (lane >> 2);           // + 8 t, t = 0..3
+            const long long at =
+                ((long long)b * a.P + (long long)tile * kLyRows + r0) * (NB * 64) + col0 +
+                2 * (lane & 3);
+            float2 zin[4][4];
+            if (EPI == kEpiActBwd) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        zin[t][j] = r0 + 8 * t < nrows
+                                        ? __ldg(reinterpret_cast<const float2 *>(
+                                              a.z_in + at + t * 8 * (NB * 64) + 8 * j))
+                                        : make_float2(0.0f, 0.0f);
+            }
+            ok = mbar_wait_bounded(smem_addr(&acc_full[buf]), (i >> 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb) {
+                float s[2][16];
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const uint32_t ta = tmem + ((uint32_t)(quad * 32 + hf * 16) << 16) +
+                                        (uint32_t)(buf * 128 + nb * 64 + col0);
+                    tmem_ld_16x32(ta, s[hf]);
+                    if (K2) {
+                        float g[16];
+                        tmem_ld_16x32(ta + 64, g);
+                        tmem_ld_wait(s[hf]);
+                        tmem_ld_wait(g);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) s[hf][k] = g[k] + s[hf][k];
+                    } else {
+                        tmem_ld_wait(s[hf]);
+                    }
+                }
+                if (nb == NB - 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_addr(&acc_free[buf]));
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    if (r0 + 8 * t >= nrows) continue;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float2 v = make_float2(s[t >> 1][4 * j + 2 * (t & 1)],
+                                               s[t >> 1][4 * j + 2 * (t & 1) + 1]);
+                        const long long e = at + t * 8 * (NB * 64) + nb * 64 + 8 * j;
+                        if (EPI == kEpiForward) {
+                            v.x += bias[nb][j].x;
+                            v.y += bias[nb][j].y;
+                        } else if (EPI == kEpiActBwd) {
+                            v.x *= layer_dgelu(zin[t][j].x);
+                            v.y *= layer_dgelu(zin[t][j].y);
+                        }
+                        *reinterpret_cast<float2 *>(a.out0 + e) = v;
+                        if (EPI == kEpiForward && a.out1)
+                            *reinterpret_cast<float2 *>(a.out1 + e) =
+                                make_float2(layer_gelu(v.x), layer_gelu(v.y));
+                    }
+                }
+            }
+        }
+    } else if (warp < kLyEpiWarps + kLyCvtWarps) {
+        // ---- round h: 8 rows x 8 chunks of 8 columns per step of a warp; the
+        // chunk and the half read first rotate with the row, so the 16-byte
+        // reads (256-byte rows) and writes both fall on all banks
+        const int cw = warp - kLyEpiWarps, rl = lane & 7, cg = lane >> 3;
+        for (int i = 0; i < items; ++i) {
+            const int buf = i & 1;
+            ok = mbar_wait_bounded(smem_addr(&h_full[buf]), (i >> 1) & 1);
+            if (ok && i >= 1) ok = mbar_wait_bounded(smem_addr(&hb_free), (i - 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const unsigned char *src = sH + buf * kLyHBytes;
+#pragma unroll
+            for (int st = 0; st < 8; ++st) {
+                const int row = cw * 32 + (st >> 1) * 8 + rl;
+                const int c = ((st & 1) * 4 + cg + rl) & 7;
+                const int swap = (rl >> 2) & 1;
+                const float4 x = *reinterpret_cast<const float4 *>(src + row * 256 + c * 32 +
+                                                                   swap * 16);
+                const float4 y = *reinterpret_cast<const float4 *>(src + row * 256 + c * 32 +
+                                                                   (swap ^ 1) * 16);
+                const float4 lo = swap ? y : x, hi = swap ? x : y;
+                *reinterpret_cast<uint4 *>(sHb + (c * (kLyRows / 8) + (row >> 3)) * 128 +
+                                           (row & 7) * 16) =
+                    make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w),
+                               pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(smem_addr(&h_free[buf]));
+                mbar_arrive(smem_addr(&hb_full));
+            }
+        }
+    } else if (warp == kLyEpiWarps + kLyCvtWarps) {
+        // ---- copies
+        if (lane == 0) {
+            int nh = 0, nu = 0, ng = 0, tile_now = -1;   // copies issued of h, U, G
+            for (int i = 0; i < items; ++i) {
+                const long long it = first + i;
+                const int tile = (int)(it / a.B), b = (int)(it % a.B), buf = i & 1;
+                const uint32_t hbytes =
+                    (uint32_t)min(kLyRows, a.P - tile * kLyRows) * (kLyW * 4);
+                if (i >= 2) ok = mbar_wait_bounded(smem_addr(&h_free[buf]), ((i - 2) >> 1) & 1);
+                if (!ok) break;
+                mbar_expect_tx(smem_addr(&h_full[buf]), hbytes);
+                bulk_load(smem_addr(sH + buf * kLyHBytes),
+                          a.h + ((long long)b * a.P + (long long)tile * kLyRows) * kLyW, hbytes,
+                          smem_addr(&h_full[buf]));
+                ++nh;
+                if (!K2) continue;
+                if (i >= 2) ok = mbar_wait_bounded(smem_addr(&acc_full[buf]), ((i - 2) >> 1) & 1);
+                if (!ok) break;
+                mbar_expect_tx(smem_addr(&u_full[buf]), kLyUBytes);
+                bulk_load(smem_addr(sU + buf * kLyUBytes), a.u_img + (size_t)b * kLyUBytes,
+                          kLyUBytes, smem_addr(&u_full[buf]));
+                ++nu;
+                if (tile == tile_now) continue;
+                // the products of the item before read the old tile of G
+                if (i >= 1)
+                    ok = mbar_wait_bounded(smem_addr(&acc_full[(i - 1) & 1]), ((i - 1) >> 1) & 1);
+                if (!ok) break;
+                mbar_expect_tx(smem_addr(&g_full), kLyGBytes);
+                bulk_load(smem_addr(sG), a.g_img + (size_t)tile * kLyGBytes, kLyGBytes,
+                          smem_addr(&g_full));
+                tile_now = tile;
+                ++ng;
+            }
+            // no copy may still land after the CTA exits
+            for (int k = max(0, nh - 2); k < nh; ++k)
+                ok = mbar_wait_bounded(smem_addr(&h_full[k & 1]), (k >> 1) & 1) && ok;
+            for (int k = max(0, nu - 2); k < nu; ++k)
+                ok = mbar_wait_bounded(smem_addr(&u_full[k & 1]), (k >> 1) & 1) && ok;
+            if (ng) ok = mbar_wait_bounded(smem_addr(&g_full), (ng - 1) & 1) && ok;
+        }
+    } else {
+        // ---- products
+        if (lane == 0) {
+            int tile_now = -1, gloads = 0, done = 0;
+            for (int i = 0; i < items; ++i) {
+                const int tile = (int)((first + i) / a.B), buf = i & 1;
+                if (i >= 2)
+                    ok = mbar_wait_bounded(smem_addr(&acc_free[buf]), ((i - 2) >> 1) & 1);
+                ok = ok && mbar_wait_bounded(smem_addr(&hb_full), i & 1);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d1 = tmem + (uint32_t)(buf * 128);
+#pragma unroll
+                for (int s = 0; s < kLyW / 16; ++s) {
+                    const uint64_t ad = smem_desc(smem_addr(sHb) + s * 2 * (kLyRows / 8) * 128,
+                                                  (kLyRows / 8) * 128, 128);
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb) {
+                        const uint64_t bd =
+                            smem_desc(smem_addr(sW) + nb * kLyWBytes + s * 2 * (kLyW / 8) * 128,
+                                      (kLyW / 8) * 128, 128);
+                        mma_bf16(d1 + nb * 64, ad, bd, s > 0 ? 1u : 0u);
+                    }
+                }
+                mma_commit(smem_addr(&hb_free));
+                if (K2) {
+                    ok = mbar_wait_bounded(smem_addr(&u_full[buf]), (i >> 1) & 1);
+                    if (ok && tile != tile_now) {
+                        ok = mbar_wait_bounded(smem_addr(&g_full), gloads & 1);
+                        ++gloads;
+                        tile_now = tile;
+                    }
+                    if (!ok) {   // cover what was issued
+                        mma_commit(smem_addr(&acc_full[buf]));
+                        ++done;
+                        break;
+                    }
+                    const uint32_t ua = smem_addr(sU + buf * kLyUBytes);
+#pragma unroll
+                    for (int s = 0; s < K2 / 16; ++s) {
+                        const uint64_t ad = smem_desc(smem_addr(sG) + s * 2 * (kLyRows / 8) * 128,
+                                                      (kLyRows / 8) * 128, 128);
+                        const uint64_t bd =
+                            smem_desc(ua + s * 2 * (kLyW / 8) * 128, (kLyW / 8) * 128, 128);
+                        mma_bf16(d1 + 64, ad, bd, s > 0 ? 1u : 0u);
+                    }
+                }
+                mma_commit(smem_addr(&acc_full[buf]));
+                ++done;
+            }
+            // TMEM and shared memory are given back only after every product
+            if (done)
+                ok = mbar_wait_bounded(smem_addr(&acc_full[(done - 1) & 1]),
+                                       ((done - 1) >> 1) & 1) && ok;
+        }
+    }
+    if (!ok) atomicExch(&g_gemm_wait_fail, 1);
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(kLyTmem)
+                     : "memory");
+    }
+}
+
+// A (rows x K) operand in FP32 as BF16 images of the K-major core-matrix
+// layout, tile by tile: `mt` 128-row tiles next to each other for each block of
+// kc columns of K.  Unit (block kb, row tile t, chunk c of 8 k, row r) is 16
+// bytes; rows past `rows` and k past K are zero.
+__global__ void basis_image_kernel(const float *src, long long s_row, long long s_k, int rows,
+                                   int K, int mt, int kc, int nkb, uint4 *img) {
+    const long long units = (long long)nkb * mt * (kc / 8) * 128;
+    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < units;
+         u += (long long)gridDim.x * blockDim.x) {
+        const int rl = (int)(u % 128);
+        const long long v = u / 128;
+        const int c = (int)(v % (kc / 8));
+        const int t = (int)(v / (kc / 8) % mt);
+        const int kb = (int)(v / (kc / 8) / mt);
+        const int row = t * 128 + rl;
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int k = kb * kc + 8 * c + e;
+            f[e] = row < rows && k < K ? src[row * s_row + k * s_k] : 0.0f;
+        }
+        img[u] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                            pack_bf16(f[6], f[7]));
+    }
+}
+
+// U[b] (256 x 64, FP32) as the B operand of G U[b]: chunk c of 8 k, column n.
+__global__ void u_image_kernel(const float *U, int B, uint4 *img) {
+    const int units = B * (kLyQ / 8) * kLyW;
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < units; u += gridDim.x * blockDim.x) {
+        const int n = u % kLyW, c = u / kLyW;   // c counts chunks over all samples
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = U[((long long)c * 8 + e) * kLyW + n];
+        img[u] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                            pack_bf16(f[6], f[7]));
+    }
+}
+
+}  // namespace

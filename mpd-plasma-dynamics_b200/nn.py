@@ -32,6 +32,32 @@ def gemm(A, B, Cout, M, N_, K, batch=1, sa=None, sb=None, sc=None, alpha=1.0, be
     return Cout
 
 
+FORWARD, ACT_BWD, PLAIN = 0, 1, 2   # epilogues of layer()
+
+
+def basis_image(A, rows, K, s_row, s_k, block_k=256):
+    """The (rows x K) float32 operand at A[row * s_row + k * s_k], rounded to
+    BF16 in the tensor core's layout (blocks of block_k columns)."""
+    import torch
+    lib = N.load()
+    n = -(-K // block_k) * -(-rows // 128) * 128 * block_k
+    img = torch.empty(n, dtype=torch.bfloat16, device=A.device)
+    N.check(lib.mpd_nn_basis_image(C.c_void_p(A.data_ptr()), s_row, s_k, rows, K, block_k,
+                                   C.c_void_p(img.data_ptr()), _stream()), lib)
+    return img
+
+
+def layer(h, w, w_sn, w_sk, out0, P, B, n_out=64, epilogue=FORWARD, basis=None, U=None,
+          u_work=None, bias=None, z_in=None, out1=None):
+    """out0 = h W + basis U[b] (+ bias), out1 = GELU(out0); or the backward forms
+    of it: mpd_nn_layer in include/mpd_b200.h."""
+    lib = N.load()
+    ptr = lambda t: None if t is None else t.data_ptr()
+    d = N.LayerDesc(P, B, n_out, epilogue, h.data_ptr(), w.data_ptr(), w_sn, w_sk, ptr(basis),
+                    ptr(U), ptr(u_work), ptr(bias), ptr(z_in), out0.data_ptr(), ptr(out1))
+    N.check(lib.mpd_nn_layer(C.byref(d), _stream()), lib)
+
+
 def wait_status():
     lib = N.load()
     N.check(lib.mpd_nn_wait_status(_stream()), lib)

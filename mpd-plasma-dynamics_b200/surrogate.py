@@ -143,10 +143,16 @@ class SpectralOperator:
         Fq, G = bases(H, W)
         self.F = torch.from_numpy(Fq.astype(np.float32)).to(dev)
         self.G = torch.from_numpy(G.astype(np.float32)).to(dev)
+        # the synthesis and its transpose as the layer kernel reads them
+        self.G_img = nn.basis_image(self.G, self.P, self.Q, self.Q, 1)
+        self.Ft_img = nn.basis_image(self.F, self.P, self.Q, 1, self.P)
+        self.u_work = torch.empty(batch * self.Q * WIDTH, device=dev, dtype=torch.bfloat16)
         rows = batch * self.P
         self.x = torch.zeros(rows, N_IN, **f32)
         self.z = [torch.zeros(rows, WIDTH, **f32) for _ in range(LAYERS + 1)]
-        self.h = [torch.zeros(rows, WIDTH, **f32) for _ in range(LAYERS + 1)]
+        # the lift and the last layer have no activation: their h is their z
+        self.h = [self.z[l] if l in (0, LAYERS) else torch.zeros(rows, WIDTH, **f32)
+                  for l in range(LAYERS + 1)]
         self.V = [torch.zeros(batch, self.Q, WIDTH, **f32) for _ in range(LAYERS)]
         self.U = torch.zeros(batch, self.Q, WIDTH, **f32)
         self.zp = torch.zeros(rows, HIDDEN, **f32)
@@ -158,7 +164,6 @@ class SpectralOperator:
         self.g_b = torch.zeros(rows, max(WIDTH, HIDDEN), **f32)
         self.g_out = torch.zeros(rows, N_OUT, **f32)
         self.gh = [torch.zeros(rows, WIDTH, **f32) for _ in range(2)]
-        self.gz = torch.zeros(rows, WIDTH, **f32)
         self.gU = torch.zeros(batch, self.Q, WIDTH, **f32)
         self.gV = torch.zeros(batch, self.Q, WIDTH, **f32)
         self.parts = torch.zeros(batch * max(WIDTH, HIDDEN) * max(WIDTH, HIDDEN), **f32)
@@ -228,19 +233,18 @@ class SpectralOperator:
         self._bias_act(self.z[0], p["b_in"], self.h[0], act=False)
         for l in range(LAYERS):
             h, z = self.h[l], self.z[l + 1]
-            self._linear(h, Cw, p[f"W{l}"], Cw, z)
             # V[b] = F h[b]  (Q x C)
             nn.gemm(self.F, h, self.V[l], Q, Cw, P, B, sa=(P, 1, 0), sb=(1, Cw, P * Cw),
                     sc=(Cw, 1, Q * Cw), work=self.work)
             # U[b, q] = V[b, q] R[q]   (batched over q)
             nn.gemm(self.V[l], p[f"R{l}"], self.U, B, Cw, Cw, Q, sa=(Q * Cw, 1, Cw),
                     sb=(1, Cw, Cw * Cw), sc=(Q * Cw, 1, Cw))
-            # z[b] += G U[b]
-            nn.gemm(self.G, self.U, z, P, Cw, Q, B, sa=(Q, 1, 0), sb=(1, Cw, Q * Cw),
-                    sc=(Cw, 1, P * Cw), beta=1.0)
-            self._bias_act(z, p[f"b{l}"], self.h[l + 1], act=l < LAYERS - 1)
-        self._linear(self.h[LAYERS], Cw, p["W_p1"], HIDDEN, self.zp)
-        self._bias_act(self.zp, p["b_p1"], self.y1, act=True)
+            # z[b] = h W + G U[b] + bias, h' = GELU(z) (z itself after the last layer)
+            nn.layer(h, p[f"W{l}"], 1, Cw, z, P, B, basis=self.G_img, U=self.U,
+                     u_work=self.u_work, bias=p[f"b{l}"],
+                     out1=self.h[l + 1] if l < LAYERS - 1 else None)
+        nn.layer(self.h[LAYERS], p["W_p1"], 1, HIDDEN, self.zp, B * P, 1, n_out=HIDDEN,
+                 bias=p["b_p1"], out1=self.y1)
         self._linear(self.y1, HIDDEN, p["W_p2"], N_OUT, self.zo)
         self._bias_act(self.zo, p["b_p2"], self.out, act=False)
         return self.out
@@ -272,14 +276,9 @@ class SpectralOperator:
         gh = self.gh[0]
         nn.gemm(gzp, p["W_p1"], gh, rows, Cw, HIDDEN, 1, sa=(HIDDEN, 1, 0), sb=(HIDDEN, 1, 0),
                 sc=(Cw, 1, 0))
+        gz = gh   # the last layer has no activation
         for l in reversed(range(LAYERS)):
-            z, h = self.z[l + 1], self.h[l]
-            if l < LAYERS - 1:
-                gz = self.gz
-                self._chk(self.lib.mpd_nn_act_bwd(C.c_void_p(gh.data_ptr()), C.c_void_p(z.data_ptr()),
-                                                  C.c_void_p(gz.data_ptr()), rows * Cw, self._s()))
-            else:
-                gz = gh
+            h = self.h[l]
             self._wgrad(h, Cw, gz, Cw, g[f"W{l}"])
             self._colsum(gz, g[f"b{l}"])
             # gU[b] = G^T gz[b]
@@ -291,13 +290,12 @@ class SpectralOperator:
             # gV[b, q] = gU[b, q] R[q]^T
             nn.gemm(self.gU, p[f"R{l}"], self.gV, B, Cw, Cw, Q, sa=(Q * Cw, 1, Cw),
                     sb=(Cw, 1, Cw * Cw), sc=(Q * Cw, 1, Cw))
-            # gh = gz W^T + F^T gV
-            gh_new = self.gh[1] if gh is self.gh[0] else self.gh[0]
-            nn.gemm(gz, p[f"W{l}"], gh_new, rows, Cw, Cw, 1, sa=(Cw, 1, 0), sb=(Cw, 1, 0),
-                    sc=(Cw, 1, 0))
-            nn.gemm(self.F, self.gV, gh_new, P, Cw, Q, B, sa=(1, P, 0), sb=(1, Cw, Q * Cw),
-                    sc=(Cw, 1, P * Cw), beta=1.0)
-            gh = gh_new
+            # gh = gz W^T + F^T gV, and through the activation of the layer below
+            gh = self.gh[1] if gz is self.gh[0] else self.gh[0]
+            nn.layer(gz, p[f"W{l}"], Cw, 1, gh, P, B, basis=self.Ft_img, U=self.gV,
+                     u_work=self.u_work, epilogue=nn.ACT_BWD if l else nn.PLAIN,
+                     z_in=self.z[l] if l else None)
+            gz = gh
         # lift (the input needs no gradient)
         self._wgrad(self.x, N_IN, gh, Cw, g["W_in"])
         self._colsum(gh, g["b_in"])

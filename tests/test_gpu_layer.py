@@ -1,0 +1,88 @@
+"""The fused layer kernel against the separate launches it stands for (products
+by the general GEMM, bias + activation and its derivative as element-wise
+kernels): the same roundings in the same order, so the same bits.  Sizes around
+its tiles of 128 rows, tiles shared by several samples and by several CTAs."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(P, B, seed):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    return dict(h=rnd(B * P, 64), W=rnd(64, 64) / 8, G=rnd(P, 256), U=rnd(B, 256, 64) / 16,
+                bias=rnd(64), z=2 * rnd(B * P, 64),
+                u_work=torch.empty(B * 256 * 64, dtype=torch.bfloat16, device="cuda"))
+
+
+def _ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _sum(nn, o, P, B, trans):
+    """h W + G U[b] by the general GEMM (trans: W transposed)."""
+    import torch
+    s = torch.empty(B * P, 64, device="cuda")
+    nn.gemm(o["h"], o["W"], s, B * P, 64, 64, 1, sa=(64, 1, 0),
+            sb=(64, 1, 0) if trans else (1, 64, 0), sc=(64, 1, 0))
+    nn.gemm(o["G"], o["U"], s, P, 64, 256, B, sa=(256, 1, 0), sb=(1, 64, 256 * 64),
+            sc=(64, 1, P * 64), beta=1.0)
+    return s
+
+
+@pytest.mark.parametrize("P,B", [(1, 1), (127, 2), (128, 1), (129, 3), (400, 60), (19000, 1)])
+def test_layer_is_the_separate_launches(pkg, P, B):
+    import torch
+    nn, lib, o = pkg.nn, pkg._native.load(), _operands(P, B, P + B)
+    img = nn.basis_image(o["G"], P, 256, 256, 1)
+    stream = nn._stream()
+    z = _sum(nn, o, P, B, False)
+    out = torch.empty_like(z)
+    assert lib.mpd_nn_bias_act(_ptr(z), _ptr(o["bias"]), _ptr(out), B * P, 64, 1, stream) == 0
+    got0, got1 = torch.full_like(z, 7.0), torch.full_like(z, 7.0)
+    args = dict(basis=img, U=o["U"], u_work=o["u_work"])
+    nn.layer(o["h"], o["W"], 1, 64, got0, P, B, bias=o["bias"], out1=got1, **args)
+    assert torch.equal(got0, z) and torch.equal(got1, out)
+    got0.fill_(7.0)
+    nn.layer(o["h"], o["W"], 1, 64, got0, P, B, bias=o["bias"], **args)
+    assert torch.equal(got0, z)
+    # backward: the transposed weight, G^T's image read from its transpose
+    img_t = nn.basis_image(o["G"].t().contiguous(), P, 256, 1, P)
+    assert torch.equal(img_t, img)
+    gh = _sum(nn, o, P, B, True)
+    gz = torch.empty_like(gh)
+    assert lib.mpd_nn_act_bwd(_ptr(gh), _ptr(o["z"]), _ptr(gz), gh.numel(), stream) == 0
+    nn.layer(o["h"], o["W"], 64, 1, got0, P, B, epilogue=nn.PLAIN, **args)
+    assert torch.equal(got0, gh)
+    nn.layer(o["h"], o["W"], 64, 1, got0, P, B, epilogue=nn.ACT_BWD, z_in=o["z"], **args)
+    assert torch.equal(got0, gz)
+    nn.wait_status()
+
+
+@pytest.mark.parametrize("rows", [1, 128, 1001, 40000])
+def test_wide_linear_is_the_separate_launches(pkg, rows):
+    import torch
+    nn, lib, o = pkg.nn, pkg._native.load(), _operands(rows, 1, rows)
+    W = torch.randn(64, 128, device="cuda") / 8
+    bias = torch.randn(128, device="cuda")
+    z, out = torch.empty(rows, 128, device="cuda"), torch.empty(rows, 128, device="cuda")
+    nn.gemm(o["h"], W, z, rows, 128, 64, 1, sa=(64, 1, 0), sb=(1, 128, 0), sc=(128, 1, 0))
+    assert lib.mpd_nn_bias_act(_ptr(z), _ptr(bias), _ptr(out), rows, 128, 1, nn._stream()) == 0
+    got0, got1 = torch.full_like(z, 7.0), torch.full_like(z, 7.0)
+    nn.layer(o["h"], W, 1, 128, got0, rows, 1, n_out=128, bias=bias, out1=got1)
+    assert torch.equal(got0, z) and torch.equal(got1, out)
+    nn.wait_status()
+
+
+def test_refused_operands(pkg):
+    import torch
+    nn, o = pkg.nn, _operands(8, 1, 0)
+    out = torch.empty(8, 64, device="cuda")
+    img = nn.basis_image(o["G"], 8, 256, 256, 1)
+    for bad in (dict(basis=img, U=o["U"]), dict(basis=img, U=o["U"], u_work=o["u_work"]),
+                dict(bias=o["bias"])):
+        with pytest.raises(pkg._native.MpdError):
+            nn.layer(o["h"], o["W"], 1, 64, out, 8, 1, **bad)
