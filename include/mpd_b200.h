@@ -370,25 +370,42 @@ int mpd_nn_wait_status(void *stream);
 int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int rows, int K,
                        int block_k, void *image, void *stream);
 
+/* The spectral half of a layer, with the roundings and the split of K of the
+ * GEMMs it stands for: V[b] = basis h[b] (256 x 64 sums over P points; basis:
+ * image of 256 x P with block_k 32), U[b, q] = V[b, q] R[q] with R[q](n, k) at
+ * R[q * 4096 + n * r_sn + k * r_sk], and U as the image mpd_nn_layer reads
+ * (B * 32 KB).  All operands but R start on 16-byte boundaries. */
+typedef struct mpd_spectral_desc {
+    int P, B;
+    const float *h;
+    const void *basis;
+    const float *R;
+    long long r_sn, r_sk;
+    float *V, *U;          /* B x 256 x 64 each */
+    void *u_image;
+    float *work;           /* optional scratch for split-K partial sums (or NULL) */
+    long long work_floats;
+} mpd_spectral_desc;
+
+int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream);
+
 /* One layer of the network in one kernel, with the roundings of the GEMMs and
  * element-wise kernels it stands for; rows are B samples of P points:
  *   s = h W + basis U[b]     h: rows x 64, W(n, k) at w[n * w_sn + k * w_sk],
  *                            basis: image of P x 256 with block_k 256,
- *                            U: B x 256 x 64, u_work: B * 32 KB of scratch
+ *                            u_image: U as mpd_nn_spectral leaves it
  *   MPD_NN_FORWARD  out0 = s + bias; out1 = GELU(out0) (out1 may be NULL)
  *   MPD_NN_ACT_BWD  out0 = s * GELU'(z_in)
  *   MPD_NN_PLAIN    out0 = s
  * With basis == NULL: s = h W with n_out = 128 columns, MPD_NN_FORWARD only
- * (B = 1, P = all rows).  h, out0, out1, z_in, basis and u_work start on
+ * (B = 1, P = all rows).  h, out0, out1, z_in, basis and u_image start on
  * 16-byte boundaries. */
 enum { MPD_NN_FORWARD = 0, MPD_NN_ACT_BWD = 1, MPD_NN_PLAIN = 2 };
 typedef struct mpd_layer_desc {
     int P, B, n_out, epilogue;
     const float *h, *w;
     long long w_sn, w_sk;
-    const void *basis;
-    const float *U;
-    void *u_work;
+    const void *basis, *u_image;
     const float *bias, *z_in;
     float *out0, *out1;
 } mpd_layer_desc;

@@ -106,9 +106,16 @@ class GemmDesc(C.Structure):
 class LayerDesc(C.Structure):
     _fields_ = [("P", C.c_int), ("B", C.c_int), ("n_out", C.c_int), ("epilogue", C.c_int),
                 ("h", C.c_void_p), ("w", C.c_void_p), ("w_sn", C.c_longlong),
-                ("w_sk", C.c_longlong), ("basis", C.c_void_p), ("U", C.c_void_p),
-                ("u_work", C.c_void_p), ("bias", C.c_void_p), ("z_in", C.c_void_p),
+                ("w_sk", C.c_longlong), ("basis", C.c_void_p), ("u_image", C.c_void_p),
+                ("bias", C.c_void_p), ("z_in", C.c_void_p),
                 ("out0", C.c_void_p), ("out1", C.c_void_p)]
+
+
+class SpectralDesc(C.Structure):
+    _fields_ = [("P", C.c_int), ("B", C.c_int), ("h", C.c_void_p), ("basis", C.c_void_p),
+                ("R", C.c_void_p), ("r_sn", C.c_longlong), ("r_sk", C.c_longlong),
+                ("V", C.c_void_p), ("U", C.c_void_p), ("u_image", C.c_void_p),
+                ("work", C.c_void_p), ("work_floats", C.c_longlong)]
 
 
 class MpdError(RuntimeError):
@@ -161,6 +168,7 @@ SIGNATURES = [
     ("mpd_nn_wait_status", C.c_int, [_VP]),
     ("mpd_nn_basis_image", C.c_int, [_VP, C.c_longlong, C.c_longlong, C.c_int, C.c_int, C.c_int,
                                      _VP, _VP]),
+    ("mpd_nn_spectral", C.c_int, [C.POINTER(SpectralDesc), _VP]),
     ("mpd_nn_layer", C.c_int, [C.POINTER(LayerDesc), _VP]),
     ("mpd_nn_bias_act", C.c_int, [_VP, _VP, _VP, C.c_longlong, C.c_int, C.c_int, _VP]),
     ("mpd_nn_act_bwd", C.c_int, [_VP, _VP, _VP, C.c_longlong, _VP]),

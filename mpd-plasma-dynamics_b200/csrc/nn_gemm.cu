@@ -439,8 +439,28 @@ __global__ void nn_gemm_reduce_kernel(const mpd_gemm_desc d, int ksplit) {
 }  // namespace
 
 #include "nn_layer.cuh"
+#include "nn_spectral.cuh"
 
 namespace {
+
+// Split K when the tiles alone leave most SMs idle and the caller gave room for
+// the partial sums (summed in split order afterwards).
+void SplitK(int M, int N, int K, int batch, long long work_floats, int *ksplit, int *kspan) {
+    const long long tiles =
+        (long long)((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN) * batch;
+    *ksplit = 1;
+    if (tiles < 296 && K >= 4 * kSplitUnit) {
+        long long want = (296 + tiles - 1) / tiles;
+        const long long by_k = K / (2 * kSplitUnit);
+        const long long by_room = work_floats / ((long long)M * N * batch);
+        want = want < by_k ? want : by_k;
+        want = want < by_room ? want : by_room;
+        want = want < 64 ? want : 64;
+        if (want > 1) *ksplit = (int)want;
+    }
+    *kspan = ((K + *ksplit - 1) / *ksplit + kSplitUnit - 1) / kSplitUnit * kSplitUnit;
+    *ksplit = (K + *kspan - 1) / *kspan;
+}
 
 int NnLaunched(const char *what) {
     const cudaError_t e = cudaGetLastError();
@@ -486,19 +506,57 @@ int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int row
     return NnLaunched("mpd_nn_basis_image");
 }
 
+int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream) {
+    if (!d || !d->h || !d->basis || !d->R || !d->V || !d->U || !d->u_image || d->P < 1 ||
+        d->B < 0) {
+        mpd::SetLastError("mpd_nn_spectral: NULL operand or bad sizes");
+        return MPD_ERR_INVALID;
+    }
+    if (!Aligned16(d->h) || !Aligned16(d->basis) || !Aligned16(d->V) || !Aligned16(d->U) ||
+        !Aligned16(d->u_image) || !Aligned16(d->work)) {
+        mpd::SetLastError("mpd_nn_spectral: operands must start on 16-byte boundaries");
+        return MPD_ERR_INVALID;
+    }
+    if (d->B == 0) return MPD_OK;
+    int ksplit, kspan;
+    SplitK(kLyQ, kLyW, d->P, d->B, d->work ? d->work_floats : 0, &ksplit, &kspan);
+    if ((long long)d->B * ksplit > 65535) {
+        mpd::SetLastError("mpd_nn_spectral: batch too large for one launch");
+        return MPD_ERR_INVALID;
+    }
+    static bool attr_set = false;  // per process; the attribute is per function
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            nn_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmem);
+        if (e != cudaSuccess) {
+            mpd::SetLastError(std::string("mpd_nn_spectral: ") + cudaGetErrorString(e));
+            return MPD_ERR_CUDA;
+        }
+        attr_set = true;
+    }
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    nn_project_kernel<<<d->B * ksplit, kPjThreads, kPjSmem, st>>>(
+        static_cast<const unsigned char *>(d->basis), d->h, d->P, d->B, kspan,
+        ksplit > 1 ? d->work : d->V);
+    nn_mix_kernel<<<dim3(kLyQ, (d->B + 127) / 128), 128, 0, st>>>(
+        d->work, ksplit, d->B, d->R, d->r_sn, d->r_sk, d->V, d->U,
+        static_cast<__nv_bfloat16 *>(d->u_image));
+    return NnLaunched("mpd_nn_spectral");
+}
+
 int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     if (!d || !d->h || !d->w || !d->out0 || d->P < 1 || d->B < 0) {
         mpd::SetLastError("mpd_nn_layer: NULL operand or bad sizes");
         return MPD_ERR_INVALID;
     }
     const bool spectral = d->basis != nullptr;
-    const bool shape_ok = spectral ? d->n_out == 64 && d->U && d->u_work : d->n_out == 128;
+    const bool shape_ok = spectral ? d->n_out == 64 && d->u_image : d->n_out == 128;
     const bool epi_ok = d->epilogue == MPD_NN_FORWARD ? d->bias != nullptr
                         : !spectral                   ? false
                         : d->epilogue == MPD_NN_ACT_BWD ? d->z_in != nullptr
                                                         : d->epilogue == MPD_NN_PLAIN;
     if (!shape_ok || !epi_ok || !Aligned16(d->h) || !Aligned16(d->out0) || !Aligned16(d->out1) ||
-        !Aligned16(d->z_in) || !Aligned16(d->basis) || !Aligned16(d->u_work)) {
+        !Aligned16(d->z_in) || !Aligned16(d->basis) || !Aligned16(d->u_image)) {
         mpd::SetLastError("mpd_nn_layer: unsupported widths, epilogue or alignment");
         return MPD_ERR_INVALID;
     }
@@ -514,7 +572,7 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     a.w_sn = d->w_sn;
     a.w_sk = d->w_sk;
     a.g_img = static_cast<const unsigned char *>(d->basis);
-    a.u_img = static_cast<const unsigned char *>(d->u_work);
+    a.u_img = static_cast<const unsigned char *>(d->u_image);
     a.bias = d->bias;
     a.z_in = d->z_in;
     a.out0 = d->out0;
@@ -523,9 +581,6 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     a.B = d->B;
     a.tiles = (d->P + kLyRows - 1) / kLyRows;
     if (!spectral) return LaunchLayer<0, 2, kEpiForward>(a, st);
-    const long long units = (long long)d->B * (kLyQ / 8) * kLyW;
-    u_image_kernel<<<(int)((units + 255) / 256 < 148 * 8 ? (units + 255) / 256 : 148 * 8), 256, 0,
-                     st>>>(d->U, d->B, static_cast<uint4 *>(d->u_work));
     if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyQ, 1, kEpiForward>(a, st);
     if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyQ, 1, kEpiActBwd>(a, st);
     return LaunchLayer<kLyQ, 1, kEpiPlain>(a, st);
@@ -545,23 +600,8 @@ int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream) {
         mpd::SetLastError("mpd_nn_gemm: batch or N too large for one launch");
         return MPD_ERR_INVALID;
     }
-    // split K when the tiles alone leave most SMs idle and the caller gave
-    // room for the partial sums (summed in split order afterwards)
-    const long long tiles = (long long)((d->M + kTileM - 1) / kTileM) *
-                            ((d->N + kTileN - 1) / kTileN) * d->batch;
-    int ksplit = 1;
-    if (d->work && tiles < 296 && d->K >= 4 * kSplitUnit) {
-        long long want = (296 + tiles - 1) / tiles;
-        const long long by_k = d->K / (2 * kSplitUnit);
-        const long long by_room = d->work_floats / ((long long)d->M * d->N * d->batch);
-        want = want < by_k ? want : by_k;
-        want = want < by_room ? want : by_room;
-        want = want < 64 ? want : 64;
-        if (want > 1) ksplit = (int)want;
-    }
-    const int kspan =
-        ((d->K + ksplit - 1) / ksplit + kSplitUnit - 1) / kSplitUnit * kSplitUnit;
-    ksplit = (d->K + kspan - 1) / kspan;
+    int ksplit, kspan;
+    SplitK(d->M, d->N, d->K, d->batch, d->work ? d->work_floats : 0, &ksplit, &kspan);
     if ((long long)d->batch * ksplit > 65535) {
         mpd::SetLastError("mpd_nn_gemm: batch too large for one launch");
         return MPD_ERR_INVALID;

@@ -14,8 +14,8 @@
 //     samples fastest, so the tile of G (64 KB of BF16) stays in shared memory
 //     over its samples;
 //   * G and U come as images of the tensor core's K-major core-matrix layout
-//     (basis_image_kernel, once per network; u_image_kernel, each call), so
-//     they are bulk copies without any work by the threads; h arrives as FP32
+//     (basis_image_kernel, once per network; the mix's epilogue), so they are
+//     bulk copies without any work by the threads; h arrives as FP32
 //     (a tile is 32 KB of contiguous memory) and four warps round it;
 //   * warps 0-7 run the epilogue of item i while the tensor core works on item
 //     i + 1 and the copies of item i + 2 are in flight (TMEM, h and U are
@@ -48,7 +48,7 @@ struct LayerArgs {
     const float *w;              // (n, k) at w[n * w_sn + k * w_sk]
     long long w_sn, w_sk;
     const unsigned char *g_img;  // tiles of kLyGBytes (K2 != 0)
-    const unsigned char *u_img;  // B x kLyUBytes     (K2 != 0)
+    const unsigned char *u_img;  // B x kLyUBytes (K2 != 0): chunk of 8 k, column n, 16 bytes
     const float *bias;           // forward
     const float *z_in;           // kEpiActBwd: GELU' is taken at these
     float *out0, *out1;          // out1: GELU(out0), or NULL
@@ -417,19 +417,6 @@ __global__ void basis_image_kernel(const float *src, long long s_row, long long 
             const int k = kb * kc + 8 * c + e;
             f[e] = row < rows && k < K ? src[row * s_row + k * s_k] : 0.0f;
         }
-        img[u] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
-                            pack_bf16(f[6], f[7]));
-    }
-}
-
-// U[b] (256 x 64, FP32) as the B operand of G U[b]: chunk c of 8 k, column n.
-__global__ void u_image_kernel(const float *U, int B, uint4 *img) {
-    const int units = B * (kLyQ / 8) * kLyW;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < units; u += gridDim.x * blockDim.x) {
-        const int n = u % kLyW, c = u / kLyW;   // c counts chunks over all samples
-        float f[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = U[((long long)c * 8 + e) * kLyW + n];
         img[u] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                             pack_bf16(f[6], f[7]));
     }

@@ -1,0 +1,311 @@
+// The way into the spectral space and the mix there, as two kernels (included
+// by nn_gemm.cu after nn_layer.cuh):
+//
+//   nn_project_kernel  V[b] = basis h[b]      256 x 64 sums over the P points
+//   nn_mix_kernel      U[b, q] = V[b, q] R[q] 64 x 64 per coefficient, and the
+//                      sums over the split of K before it
+//
+// nn_project_kernel: one CTA per (sample, split of K), both 128-row tiles of the
+// basis as two TMEM accumulators, so a row of h is fetched and rounded once (the
+// general kernel: once per tile, with the basis rounded again per sample, and
+// 320 CTAs in two waves at two per SM).  The basis is an image of the tensor
+// core's layout in blocks of 32 points (basis_image_kernel), so a stage of the
+// four-stage ring is two bulk copies (16 KB of basis, 8 KB of h); four warps
+// transpose and round h, one thread issues the products.  104 KB of shared
+// memory: two CTAs per SM.  The split of K, the order of the products in an
+// accumulator and the order of the partial sums are the general kernel's, so
+// the values are too.  Both kernels together, measured against the general one
+// (B200): 450 -> 112 us at 16 samples of 64400 points (the copies: 264 MB of h
+// from memory and 530 MB of the basis from L2), 53.5 -> 21.5 us at 16 of 4100
+// and 146 -> 60 us at 1 of 64400 (one trip through the ring per CTA and a
+// quarter of the SMs busy: bound by latency).
+#pragma once
+
+namespace {
+
+constexpr int kPjK = 32, kPjStages = 4;
+constexpr int kPjThreads = 6 * 32;
+constexpr int kPjFBytes = 2 * 128 * kPjK * 2;    // 16 KB: both tiles of a block
+constexpr int kPjHBytes = kPjK * kLyW * 4;       // 8 KB
+constexpr int kPjHbBytes = kPjK * kLyW * 2;      // 4 KB
+constexpr int kPjSmem = kPjStages * (kPjFBytes + kPjHBytes) + 2 * kPjHbBytes;
+constexpr uint32_t kPjTmem = 128;
+
+// out: ksplit == 1 ? V (B x 256 x 64) : the partial sums (ksplit x B x 256 x 64)
+__global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned char *f_img,
+                                                                const float *h, int P, int B,
+                                                                int kspan, float *out) {
+    extern __shared__ __align__(1024) unsigned char gemm_smem[];
+    __shared__ __align__(8) uint64_t full[kPjStages], done[kPjStages], hb_full[2];
+    __shared__ uint32_t tmem_slot;
+    unsigned char *sF = gemm_smem, *sH = sF + kPjStages * kPjFBytes,
+                  *sHb = sH + kPjStages * kPjHBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x % B, split = blockIdx.x / B;
+    const int k_begin = split * kspan, k_end = min(P, k_begin + kspan);
+    const int n_chunks = (k_end - k_begin + kPjK - 1) / kPjK;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "r"(kPjTmem)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kPjStages; ++i) {
+            mbar_init(smem_addr(&full[i]), 1);
+            mbar_init(smem_addr(&done[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) mbar_init(smem_addr(&hb_full[i]), 4);
+        mbar_init_fence();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    bool ok = true;
+
+    if (warp < 4) {
+        // ---- h (points x columns) to its transpose in BF16, zero past K's end
+        const int n = threadIdx.x & 63, cb = threadIdx.x >> 6;
+        for (int i = 0; i < n_chunks; ++i) {
+            const int s = i % kPjStages;
+            ok = mbar_wait_bounded(smem_addr(&full[s]), (i / kPjStages) & 1);
+            if (ok && i >= 2)   // the products of chunk i - 2 read this buffer
+                ok = mbar_wait_bounded(smem_addr(&done[(i - 2) % kPjStages]),
+                                       ((i - 2) / kPjStages) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const float *src = reinterpret_cast<const float *>(sH + s * kPjHBytes);
+            unsigned char *dst = sHb + (i & 1) * kPjHbBytes;
+            const int left = k_end - k_begin - i * kPjK;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = cb + 2 * j;
+                float f[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    f[e] = 8 * c + e < left ? src[(8 * c + e) * kLyW + n] : 0.0f;
+                *reinterpret_cast<uint4 *>(dst + (c * (kLyW / 8) + (n >> 3)) * 128 +
+                                           (n & 7) * 16) =
+                    make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]),
+                               pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_addr(&hb_full[i & 1]));
+        }
+        if (ok) ok = mbar_wait_bounded(smem_addr(&done[(n_chunks - 1) % kPjStages]),
+                                       ((n_chunks - 1) / kPjStages) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            tc_fence_after();
+            float *o = out + ((long long)blockIdx.x * kLyQ + warp * 32 + (lane >> 2)) * kLyW +
+                       2 * (lane & 3);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {   // 16 rows x 32 columns each
+                    const int hf = q & 1, col = (q >> 1) * 32;
+                    float v[16];
+                    tmem_ld_16x32(tmem + ((uint32_t)(warp * 32 + hf * 16) << 16) +
+                                      (uint32_t)(mt * 64 + col),
+                                  v);
+                    tmem_ld_wait(v);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            *reinterpret_cast<float2 *>(
+                                o + (mt * 128 + hf * 16 + t * 8) * kLyW + col + 8 * j) =
+                                make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
+                }
+        }
+    } else if (warp == 4) {
+        // ---- copies
+        if (lane == 0) {
+            int n = 0;
+            for (; n < n_chunks; ++n) {
+                const int s = n % kPjStages, k0 = k_begin + n * kPjK;
+                if (n >= kPjStages)
+                    ok = mbar_wait_bounded(smem_addr(&done[s]), (n / kPjStages - 1) & 1);
+                if (!ok) break;
+                const uint32_t hbytes = (uint32_t)min(kPjK, k_end - k0) * (kLyW * 4);
+                mbar_expect_tx(smem_addr(&full[s]), kPjFBytes + hbytes);
+                bulk_load(smem_addr(sF + s * kPjFBytes), f_img + (size_t)(k0 / kPjK) * kPjFBytes,
+                          kPjFBytes, smem_addr(&full[s]));
+                bulk_load(smem_addr(sH + s * kPjHBytes), h + ((long long)b * P + k0) * kLyW,
+                          hbytes, smem_addr(&full[s]));
+            }
+            // no copy may still land after the CTA exits
+            for (int k = max(0, n - kPjStages); k < n; ++k)
+                ok = mbar_wait_bounded(smem_addr(&full[k % kPjStages]), (k / kPjStages) & 1) && ok;
+        }
+    } else {
+        // ---- products
+        if (lane == 0) {
+            int n = 0;
+            for (; n < n_chunks; ++n) {
+                const int s = n % kPjStages;
+                ok = mbar_wait_bounded(smem_addr(&full[s]), (n / kPjStages) & 1) &&
+                     mbar_wait_bounded(smem_addr(&hb_full[n & 1]), (n >> 1) & 1);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                    for (int k = 0; k < kPjK / 16; ++k) {
+                        const uint64_t ad = smem_desc(
+                            smem_addr(sF + s * kPjFBytes) + mt * (kPjFBytes / 2) + k * 2 * 2048,
+                            2048, 128);
+                        const uint64_t bd = smem_desc(
+                            smem_addr(sHb + (n & 1) * kPjHbBytes) + k * 2 * 1024, 1024, 128);
+                        mma_bf16(tmem + mt * 64, ad, bd, (n > 0 || k > 0) ? 1u : 0u);
+                    }
+                mma_commit(smem_addr(&done[s]));
+            }
+            // TMEM and shared memory are given back only after every product
+            if (n)
+                ok = mbar_wait_bounded(smem_addr(&done[(n - 1) % kPjStages]),
+                                       ((n - 1) / kPjStages) & 1) && ok;
+        }
+    }
+    if (!ok) atomicExch(&g_gemm_wait_fail, 1);
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(kPjTmem)
+                     : "memory");
+    }
+}
+
+// One CTA per coefficient q and 128 samples: the partial sums of V[b, q] in
+// split order, V, and the product with R[q] (64 x 64).  The operands are tiny
+// (16 KB of R, ksplit x 256 B a sample), so what it costs is one trip to memory
+// for both, taken together, the product and the stores.  U also leaves as the
+// image the layer kernel copies (element (q, n) of sample b: 16-byte unit q / 8).
+__global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int ksplit, int B,
+                                                     const float *R, long long r_sn,
+                                                     long long r_sk, float *V, float *U,
+                                                     __nv_bfloat16 *u_img) {
+    __shared__ __align__(1024) unsigned char sA[128 * kLyW * 2];
+    __shared__ __align__(1024) unsigned char sB[kLyW * kLyW * 2];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q = blockIdx.x, b0 = blockIdx.y * 128, rows = min(128, B - b0);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        mbar_init(smem_addr(&bar), 1);
+        mbar_init_fence();
+    }
+    const float *Rq = R + (long long)q * (kLyW * kLyW);
+    float r[4][8];
+    const bool n_inner = r_sn == 1;   // which way a warp reads whole lines of R
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int u = threadIdx.x + 128 * j;
+        const int n = n_inner ? u % kLyW : u / 8, c = n_inner ? u / kLyW : u % 8;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[j][e] = __ldg(Rq + n * r_sn + (8 * c + e) * r_sk);
+    }
+    const long long plane = (long long)B * kLyQ * kLyW;
+    for (int u = threadIdx.x; u < rows * 8; u += 128) {
+        const int row = u >> 3, c = u & 7;
+        const long long at = ((long long)(b0 + row) * kLyQ + q) * kLyW + 8 * c;
+        float f[8];
+        if (ksplit > 1) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = 0.0f;
+#pragma unroll 4
+            for (int k = 0; k < ksplit; ++k) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(part + k * plane + at));
+                const float4 y = __ldg(reinterpret_cast<const float4 *>(part + k * plane + at) + 1);
+                f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
+                f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
+            }
+            *reinterpret_cast<float4 *>(V + at) = make_float4(f[0], f[1], f[2], f[3]);
+            *reinterpret_cast<float4 *>(V + at + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        } else {
+            const float4 x = *reinterpret_cast<const float4 *>(V + at);
+            const float4 y = *reinterpret_cast<const float4 *>(V + at + 4);
+            f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
+            f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
+        }
+        *reinterpret_cast<uint4 *>(sA + (c * 16 + (row >> 3)) * 128 + (row & 7) * 16) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                       pack_bf16(f[6], f[7]));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int u = threadIdx.x + 128 * j;
+        const int n = n_inner ? u % kLyW : u / 8, c = n_inner ? u / kLyW : u % 8;
+        *reinterpret_cast<uint4 *>(sB + (c * 8 + (n >> 3)) * 128 + (n & 7) * 16) =
+            make_uint4(pack_bf16(r[j][0], r[j][1]), pack_bf16(r[j][2], r[j][3]),
+                       pack_bf16(r[j][4], r[j][5]), pack_bf16(r[j][6], r[j][7]));
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < kLyW / 16; ++k)
+            mma_bf16(tmem, smem_desc(smem_addr(sA) + k * 2 * 2048, 2048, 128),
+                     smem_desc(smem_addr(sB) + k * 2 * 1024, 1024, 128), k > 0 ? 1u : 0u);
+        mma_commit(smem_addr(&bar));
+    }
+    __syncwarp();
+    const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_addr(&bar), 0));
+    if (ok) {
+        tc_fence_after();
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {   // 16 rows x 32 columns each
+            const int hf = p & 1, col = (p >> 1) * 32;
+            if (warp * 32 + hf * 16 >= rows) continue;
+            float v[16];
+            tmem_ld_16x32(tmem + ((uint32_t)(warp * 32 + hf * 16) << 16) + (uint32_t)col, v);
+            tmem_ld_wait(v);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int row = warp * 32 + hf * 16 + t * 8 + (lane >> 2);
+                if (row >= rows) continue;
+                const long long b = b0 + row;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int n = col + 8 * j + 2 * (lane & 3);
+                    const float2 s =
+                        make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
+                    *reinterpret_cast<float2 *>(U + (b * kLyQ + q) * kLyW + n) = s;
+                    __nv_bfloat16 *im = u_img + b * (kLyQ * kLyW) + ((q >> 3) * kLyW + n) * 8 +
+                                        (q & 7);
+                    im[0] = __float2bfloat16_rn(s.x);
+                    im[8] = __float2bfloat16_rn(s.y);
+                }
+            }
+        }
+    } else if (threadIdx.x == 0) {
+        atomicExch(&g_gemm_wait_fail, 1);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
+}  // namespace

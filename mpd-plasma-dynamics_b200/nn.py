@@ -47,14 +47,25 @@ def basis_image(A, rows, K, s_row, s_k, block_k=256):
     return img
 
 
-def layer(h, w, w_sn, w_sk, out0, P, B, n_out=64, epilogue=FORWARD, basis=None, U=None,
-          u_work=None, bias=None, z_in=None, out1=None):
+def spectral(h, basis, R, r_sn, r_sk, V, U, u_image, P, B, work=None):
+    """V[b] = basis h[b], U[b, q] = V[b, q] R[q], u_image = U as layer() reads it:
+    mpd_nn_spectral in include/mpd_b200.h."""
+    lib = N.load()
+    d = N.SpectralDesc(P, B, h.data_ptr(), basis.data_ptr(), R.data_ptr(), r_sn, r_sk,
+                       V.data_ptr(), U.data_ptr(), u_image.data_ptr(),
+                       work.data_ptr() if work is not None else None,
+                       work.numel() if work is not None else 0)
+    N.check(lib.mpd_nn_spectral(C.byref(d), _stream()), lib)
+
+
+def layer(h, w, w_sn, w_sk, out0, P, B, n_out=64, epilogue=FORWARD, basis=None, u_image=None,
+          bias=None, z_in=None, out1=None):
     """out0 = h W + basis U[b] (+ bias), out1 = GELU(out0); or the backward forms
     of it: mpd_nn_layer in include/mpd_b200.h."""
     lib = N.load()
     ptr = lambda t: None if t is None else t.data_ptr()
     d = N.LayerDesc(P, B, n_out, epilogue, h.data_ptr(), w.data_ptr(), w_sn, w_sk, ptr(basis),
-                    ptr(U), ptr(u_work), ptr(bias), ptr(z_in), out0.data_ptr(), ptr(out1))
+                    ptr(u_image), ptr(bias), ptr(z_in), out0.data_ptr(), ptr(out1))
     N.check(lib.mpd_nn_layer(C.byref(d), _stream()), lib)
 
 

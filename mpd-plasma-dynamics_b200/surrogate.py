@@ -143,10 +143,12 @@ class SpectralOperator:
         Fq, G = bases(H, W)
         self.F = torch.from_numpy(Fq.astype(np.float32)).to(dev)
         self.G = torch.from_numpy(G.astype(np.float32)).to(dev)
-        # the synthesis and its transpose as the layer kernel reads them
+        # the bases and their transposes as the tensor cores read them
         self.G_img = nn.basis_image(self.G, self.P, self.Q, self.Q, 1)
         self.Ft_img = nn.basis_image(self.F, self.P, self.Q, 1, self.P)
-        self.u_work = torch.empty(batch * self.Q * WIDTH, device=dev, dtype=torch.bfloat16)
+        self.F_img = nn.basis_image(self.F, self.Q, self.P, self.P, 1, block_k=32)
+        self.Gt_img = nn.basis_image(self.G, self.Q, self.P, 1, self.Q, block_k=32)
+        self.u_image = torch.empty(batch * self.Q * WIDTH, device=dev, dtype=torch.bfloat16)
         rows = batch * self.P
         self.x = torch.zeros(rows, N_IN, **f32)
         self.z = [torch.zeros(rows, WIDTH, **f32) for _ in range(LAYERS + 1)]
@@ -227,21 +229,18 @@ class SpectralOperator:
         self.x.copy_(self.torch.from_numpy(x.reshape(-1, N_IN).astype(np.float32)))
 
     def forward(self):
-        B, P, Q, Cw = self.B, self.P, self.Q, WIDTH
+        B, P, Cw = self.B, self.P, WIDTH
         p = self.p
         self._linear(self.x, N_IN, p["W_in"], Cw, self.z[0])
         self._bias_act(self.z[0], p["b_in"], self.h[0], act=False)
         for l in range(LAYERS):
             h, z = self.h[l], self.z[l + 1]
-            # V[b] = F h[b]  (Q x C)
-            nn.gemm(self.F, h, self.V[l], Q, Cw, P, B, sa=(P, 1, 0), sb=(1, Cw, P * Cw),
-                    sc=(Cw, 1, Q * Cw), work=self.work)
-            # U[b, q] = V[b, q] R[q]   (batched over q)
-            nn.gemm(self.V[l], p[f"R{l}"], self.U, B, Cw, Cw, Q, sa=(Q * Cw, 1, Cw),
-                    sb=(1, Cw, Cw * Cw), sc=(Q * Cw, 1, Cw))
+            # V[b] = F h[b] (Q x C), U[b, q] = V[b, q] R[q]
+            nn.spectral(h, self.F_img, p[f"R{l}"], 1, Cw, self.V[l], self.U, self.u_image, P, B,
+                        work=self.work)
             # z[b] = h W + G U[b] + bias, h' = GELU(z) (z itself after the last layer)
-            nn.layer(h, p[f"W{l}"], 1, Cw, z, P, B, basis=self.G_img, U=self.U,
-                     u_work=self.u_work, bias=p[f"b{l}"],
+            nn.layer(h, p[f"W{l}"], 1, Cw, z, P, B, basis=self.G_img, u_image=self.u_image,
+                     bias=p[f"b{l}"],
                      out1=self.h[l + 1] if l < LAYERS - 1 else None)
         nn.layer(self.h[LAYERS], p["W_p1"], 1, HIDDEN, self.zp, B * P, 1, n_out=HIDDEN,
                  bias=p["b_p1"], out1=self.y1)
@@ -281,19 +280,16 @@ class SpectralOperator:
             h = self.h[l]
             self._wgrad(h, Cw, gz, Cw, g[f"W{l}"])
             self._colsum(gz, g[f"b{l}"])
-            # gU[b] = G^T gz[b]
-            nn.gemm(self.G, gz, self.gU, Q, Cw, P, B, sa=(1, Q, 0), sb=(1, Cw, P * Cw),
-                    sc=(Cw, 1, Q * Cw), work=self.work)
+            # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T
+            nn.spectral(gz, self.Gt_img, p[f"R{l}"], Cw, 1, self.gU, self.gV, self.u_image, P, B,
+                        work=self.work)
             # dR[q] = sum_b V[b, q]^T gU[b, q]
             nn.gemm(self.V[l], self.gU, g[f"R{l}"], Cw, Cw, B, Q, sa=(1, Q * Cw, Cw),
                     sb=(1, Q * Cw, Cw), sc=(Cw, 1, Cw * Cw))
-            # gV[b, q] = gU[b, q] R[q]^T
-            nn.gemm(self.gU, p[f"R{l}"], self.gV, B, Cw, Cw, Q, sa=(Q * Cw, 1, Cw),
-                    sb=(Cw, 1, Cw * Cw), sc=(Q * Cw, 1, Cw))
             # gh = gz W^T + F^T gV, and through the activation of the layer below
             gh = self.gh[1] if gz is self.gh[0] else self.gh[0]
-            nn.layer(gz, p[f"W{l}"], Cw, 1, gh, P, B, basis=self.Ft_img, U=self.gV,
-                     u_work=self.u_work, epilogue=nn.ACT_BWD if l else nn.PLAIN,
+            nn.layer(gz, p[f"W{l}"], Cw, 1, gh, P, B, basis=self.Ft_img,
+                     u_image=self.u_image, epilogue=nn.ACT_BWD if l else nn.PLAIN,
                      z_in=self.z[l] if l else None)
             gz = gh
         # lift (the input needs no gradient)

@@ -14,8 +14,13 @@ def _operands(P, B, seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     return dict(h=rnd(B * P, 64), W=rnd(64, 64) / 8, G=rnd(P, 256), U=rnd(B, 256, 64) / 16,
-                bias=rnd(64), z=2 * rnd(B * P, 64),
-                u_work=torch.empty(B * 256 * 64, dtype=torch.bfloat16, device="cuda"))
+                bias=rnd(64), z=2 * rnd(B * P, 64))
+
+
+def _u_image(U):
+    """U[b] (256 x 64) in 16-byte units of 8 coefficients, unit (q / 8, column)."""
+    import torch
+    return U.to(torch.bfloat16).view(-1, 32, 8, 64).transpose(2, 3).contiguous()
 
 
 def _ptr(t):
@@ -43,7 +48,7 @@ def test_layer_is_the_separate_launches(pkg, P, B):
     out = torch.empty_like(z)
     assert lib.mpd_nn_bias_act(_ptr(z), _ptr(o["bias"]), _ptr(out), B * P, 64, 1, stream) == 0
     got0, got1 = torch.full_like(z, 7.0), torch.full_like(z, 7.0)
-    args = dict(basis=img, U=o["U"], u_work=o["u_work"])
+    args = dict(basis=img, u_image=_u_image(o["U"]))
     nn.layer(o["h"], o["W"], 1, 64, got0, P, B, bias=o["bias"], out1=got1, **args)
     assert torch.equal(got0, z) and torch.equal(got1, out)
     got0.fill_(7.0)
@@ -82,7 +87,34 @@ def test_refused_operands(pkg):
     nn, o = pkg.nn, _operands(8, 1, 0)
     out = torch.empty(8, 64, device="cuda")
     img = nn.basis_image(o["G"], 8, 256, 256, 1)
-    for bad in (dict(basis=img, U=o["U"]), dict(basis=img, U=o["U"], u_work=o["u_work"]),
+    for bad in (dict(basis=img), dict(basis=img, u_image=_u_image(o["U"])),
                 dict(bias=o["bias"])):
         with pytest.raises(pkg._native.MpdError):
             nn.layer(o["h"], o["W"], 1, 64, out, 8, 1, **bad)
+
+
+@pytest.mark.parametrize("P,B,room", [(1, 1, 16), (31, 2, 16), (33, 3, 16), (255, 2, 16),
+                                      (300, 2, 0), (1001, 16, 16), (4100, 1, 16), (70, 130, 2),
+                                      (40000, 2, 16)])
+def test_spectral_half_is_the_separate_launches(pkg, P, B, room):
+    """Both directions (R and R^T), split and unsplit K, more samples than a tile."""
+    import torch
+    nn, o = pkg.nn, _operands(P, B, 7 * P + B)
+    Fq = o["G"].t().contiguous()
+    R = torch.randn(256, 64, 64, device="cuda") / 8
+    n = B * 256 * 64
+    work = torch.empty(room * n, device="cuda") if room else None
+    img = nn.basis_image(Fq, 256, P, P, 1, block_k=32)
+    assert torch.equal(img, nn.basis_image(o["G"], 256, P, 1, 256, block_k=32))
+    new = lambda: torch.full((B, 256, 64), 7.0, device="cuda")
+    for r_sn, r_sk in ((1, 64), (64, 1)):
+        V, U, gV, gU = new(), new(), new(), new()
+        nn.gemm(Fq, o["h"], V, 256, 64, P, B, sa=(P, 1, 0), sb=(1, 64, P * 64),
+                sc=(64, 1, 256 * 64), work=work)
+        nn.gemm(V, R, U, B, 64, 64, 256, sa=(256 * 64, 1, 64), sb=(r_sn, r_sk, 4096),
+                sc=(256 * 64, 1, 64))
+        image = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+        nn.spectral(o["h"], img, R, r_sn, r_sk, gV, gU, image, P, B, work=work)
+        assert torch.equal(gV, V) and torch.equal(gU, U)
+        assert torch.equal(image, _u_image(U).view(-1))
+    nn.wait_status()
