@@ -397,9 +397,10 @@ int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream);
  *   MPD_NN_FORWARD  out0 = s + bias; out1 = GELU(out0) (out1 may be NULL)
  *   MPD_NN_ACT_BWD  out0 = s * GELU'(z_in)
  *   MPD_NN_PLAIN    out0 = s
- * With basis == NULL: s = h W with n_out = 128 columns, MPD_NN_FORWARD only
- * (B = 1, P = all rows).  h, out0, out1, z_in, basis and u_image start on
- * 16-byte boundaries. */
+ * With basis == NULL: the projection, s = h W with n_out = 128 columns and
+ *   MPD_NN_FORWARD  (out1 not NULL), and out2 = out1 W2 + bias2 with 8 columns,
+ *                   W2(k, n) at w2[k * 8 + n]
+ * h, out0, out1, out2, z_in, basis and u_image start on 16-byte boundaries. */
 enum { MPD_NN_FORWARD = 0, MPD_NN_ACT_BWD = 1, MPD_NN_PLAIN = 2 };
 typedef struct mpd_layer_desc {
     int P, B, n_out, epilogue;
@@ -408,9 +409,16 @@ typedef struct mpd_layer_desc {
     const void *basis, *u_image;
     const float *bias, *z_in;
     float *out0, *out1;
+    const float *w2, *bias2;
+    float *out2;
 } mpd_layer_desc;
 
 int mpd_nn_layer(const mpd_layer_desc *d, void *stream);
+
+/* z = x W + bias with the GEMM's roundings: x rows x 6, W 6 x 64 (both dense),
+ * z rows x 64 on a 16-byte boundary. */
+int mpd_nn_lift(const float *x, const float *w, const float *bias, float *z, long long rows,
+                void *stream);
 
 /* Element-wise and reduction kernels of the network (FP32, deterministic sums):
  * z += bias (per column), out = GELU(z) (act != 0) or z;  g_z = g_out GELU'(z);

@@ -108,7 +108,8 @@ class LayerDesc(C.Structure):
                 ("h", C.c_void_p), ("w", C.c_void_p), ("w_sn", C.c_longlong),
                 ("w_sk", C.c_longlong), ("basis", C.c_void_p), ("u_image", C.c_void_p),
                 ("bias", C.c_void_p), ("z_in", C.c_void_p),
-                ("out0", C.c_void_p), ("out1", C.c_void_p)]
+                ("out0", C.c_void_p), ("out1", C.c_void_p), ("w2", C.c_void_p),
+                ("bias2", C.c_void_p), ("out2", C.c_void_p)]
 
 
 class SpectralDesc(C.Structure):
@@ -170,6 +171,7 @@ SIGNATURES = [
                                      _VP, _VP]),
     ("mpd_nn_spectral", C.c_int, [C.POINTER(SpectralDesc), _VP]),
     ("mpd_nn_layer", C.c_int, [C.POINTER(LayerDesc), _VP]),
+    ("mpd_nn_lift", C.c_int, [_VP, _VP, _VP, _VP, C.c_longlong, _VP]),
     ("mpd_nn_bias_act", C.c_int, [_VP, _VP, _VP, C.c_longlong, C.c_int, C.c_int, _VP]),
     ("mpd_nn_act_bwd", C.c_int, [_VP, _VP, _VP, C.c_longlong, _VP]),
     ("mpd_nn_colsum", C.c_int, [_VP, C.c_longlong, C.c_int, _VP, _VP, _VP]),

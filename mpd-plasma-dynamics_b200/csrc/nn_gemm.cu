@@ -469,13 +469,13 @@ int NnLaunched(const char *what) {
     return MPD_ERR_CUDA;
 }
 
-template <int K2, int NB, int EPI>
+template <int K2, int NB, int EPI, bool HEAD>
 int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
-    constexpr int smem = layer_smem<K2, NB>();
+    constexpr int smem = layer_smem<K2, NB, HEAD>();
     static bool attr_set = false;  // per process; the attribute is per function
     if (!attr_set) {
         const cudaError_t e = cudaFuncSetAttribute(
-            nn_layer_kernel<K2, NB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            nn_layer_kernel<K2, NB, EPI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) {
             mpd::SetLastError(std::string("mpd_nn_layer: ") + cudaGetErrorString(e));
             return MPD_ERR_CUDA;
@@ -483,7 +483,7 @@ int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
         attr_set = true;
     }
     const long long items = (long long)a.tiles * a.B;
-    nn_layer_kernel<K2, NB, EPI>
+    nn_layer_kernel<K2, NB, EPI, HEAD>
         <<<(int)(items < 148 ? items : 148), kLyThreads, smem, st>>>(a);
     return NnLaunched("mpd_nn_layer");
 }
@@ -504,6 +504,19 @@ int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int row
     basis_image_kernel<<<148 * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         src, s_row, s_k, rows, K, mt, block_k, nkb, static_cast<uint4 *>(image));
     return NnLaunched("mpd_nn_basis_image");
+}
+
+int mpd_nn_lift(const float *x, const float *w, const float *bias, float *z, long long rows,
+                void *stream) {
+    if (!x || !w || !bias || !z || rows < 0 || !Aligned16(z)) {
+        mpd::SetLastError("mpd_nn_lift: bad arguments");
+        return MPD_ERR_INVALID;
+    }
+    if (rows == 0) return MPD_OK;
+    const long long tiles = (rows + kLyRows - 1) / kLyRows;
+    nn_lift_kernel<<<(int)(tiles < 4 * 148 ? tiles : 4 * 148), 128, 0,
+                     static_cast<cudaStream_t>(stream)>>>(x, w, bias, rows, z);
+    return NnLaunched("mpd_nn_lift");
 }
 
 int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream) {
@@ -550,13 +563,14 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
         return MPD_ERR_INVALID;
     }
     const bool spectral = d->basis != nullptr;
-    const bool shape_ok = spectral ? d->n_out == 64 && d->u_image : d->n_out == 128;
+    const bool shape_ok = spectral ? d->n_out == 64 && d->u_image
+                                   : d->n_out == 128 && d->out1 && d->w2 && d->bias2 && d->out2;
     const bool epi_ok = d->epilogue == MPD_NN_FORWARD ? d->bias != nullptr
                         : !spectral                   ? false
                         : d->epilogue == MPD_NN_ACT_BWD ? d->z_in != nullptr
                                                         : d->epilogue == MPD_NN_PLAIN;
     if (!shape_ok || !epi_ok || !Aligned16(d->h) || !Aligned16(d->out0) || !Aligned16(d->out1) ||
-        !Aligned16(d->z_in) || !Aligned16(d->basis) || !Aligned16(d->u_image)) {
+        !Aligned16(d->z_in) || !Aligned16(d->out2) || !Aligned16(d->basis) || !Aligned16(d->u_image)) {
         mpd::SetLastError("mpd_nn_layer: unsupported widths, epilogue or alignment");
         return MPD_ERR_INVALID;
     }
@@ -575,15 +589,18 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     a.u_img = static_cast<const unsigned char *>(d->u_image);
     a.bias = d->bias;
     a.z_in = d->z_in;
+    a.w2 = d->w2;
+    a.bias2 = d->bias2;
+    a.out2 = d->out2;
     a.out0 = d->out0;
     a.out1 = d->out1;
     a.P = d->P;
     a.B = d->B;
     a.tiles = (d->P + kLyRows - 1) / kLyRows;
-    if (!spectral) return LaunchLayer<0, 2, kEpiForward>(a, st);
-    if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyQ, 1, kEpiForward>(a, st);
-    if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyQ, 1, kEpiActBwd>(a, st);
-    return LaunchLayer<kLyQ, 1, kEpiPlain>(a, st);
+    if (!spectral) return LaunchLayer<0, 2, kEpiForward, true>(a, st);
+    if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyQ, 1, kEpiForward, false>(a, st);
+    if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyQ, 1, kEpiActBwd, false>(a, st);
+    return LaunchLayer<kLyQ, 1, kEpiPlain, false>(a, st);
 }
 
 int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream) {

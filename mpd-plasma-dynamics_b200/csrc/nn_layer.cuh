@@ -40,6 +40,10 @@ constexpr int kLyHBytes = kLyRows * kLyW * 4;     // 32 KB
 constexpr int kLyHbBytes = kLyRows * kLyW * 2;    // 16 KB
 constexpr int kLyWBytes = kLyW * kLyW * 2;        // 8 KB per 64 output columns
 constexpr uint32_t kLyTmem = 256;
+// The 128-wide projection with the 8 outputs after it (HEAD):
+constexpr int kLyOut = 8;
+constexpr int kLyYBytes = kLyRows * 128 * 2;      // 32 KB: GELU(z) in BF16
+constexpr int kLyW2Bytes = 64 * 128 * 2;          // 16 KB: 8 columns, the rest zero
 
 enum LayerEpilogue { kEpiForward = 0, kEpiActBwd = 1, kEpiPlain = 2 };
 
@@ -52,6 +56,8 @@ struct LayerArgs {
     const float *bias;           // forward
     const float *z_in;           // kEpiActBwd: GELU' is taken at these
     float *out0, *out1;          // out1: GELU(out0), or NULL
+    const float *w2, *bias2;     // HEAD: (k, n) at w2[k * 8 + n]
+    float *out2;                 // HEAD: rows x 8
     int P, B, tiles;             // rows of one sample, samples, 128-row tiles of one sample
 };
 
@@ -110,23 +116,32 @@ __device__ __forceinline__ float layer_dgelu(float x) {
     return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
 }
 
-template <int K2, int NB>
+template <int K2, int NB, bool HEAD>
 constexpr int layer_smem() {
-    return (K2 ? kLyGBytes + 2 * kLyUBytes : 0) + 2 * kLyHBytes + kLyHbBytes + NB * kLyWBytes;
+    return (K2 ? kLyGBytes + 2 * kLyUBytes : 0) + 2 * kLyHBytes + kLyHbBytes + NB * kLyWBytes +
+           (HEAD ? 2 * kLyYBytes + kLyW2Bytes : 0);
 }
 
-template <int K2, int NB, int EPI>
+// HEAD (with NB == 2, forward): out2 = GELU(z) W2 + bias2, while GELU(z) is in
+// registers: the epilogue also leaves it in BF16 as the A operand of a third
+// product, whose result it stores one item later.  As its own launch it read
+// the 528 MB of out1 back (16 x 64400 rows).
+template <int K2, int NB, int EPI, bool HEAD>
 __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs a) {
     static_assert(K2 == 0 || NB == 1, "one accumulator pair of 64 columns each");
+    static_assert(!HEAD || (K2 == 0 && NB == 2 && EPI == kEpiForward), "after the projection");
+    constexpr uint32_t kTmem = HEAD ? 512 : kLyTmem;
     extern __shared__ __align__(1024) unsigned char gemm_smem[];
     __shared__ __align__(8) uint64_t h_full[2], h_free[2], u_full[2], acc_full[2], acc_free[2],
-        g_full, hb_full, hb_free;
+        g_full, hb_full, hb_free, y_full[2], o_full[2];
     __shared__ uint32_t tmem_slot;
     unsigned char *sG = gemm_smem;
     unsigned char *sU = sG + (K2 ? kLyGBytes : 0);
     unsigned char *sH = sU + (K2 ? 2 * kLyUBytes : 0);
     unsigned char *sHb = sH + 2 * kLyHBytes;
     unsigned char *sW = sHb + kLyHbBytes;
+    unsigned char *sY = sW + NB * kLyWBytes;
+    unsigned char *sW2 = sY + 2 * kLyYBytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = (long long)a.tiles * a.B;
     const long long first = layer_first(total, blockIdx.x, gridDim.x);
@@ -135,7 +150,7 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_addr(&tmem_slot)),
-                     "r"(kLyTmem)
+                     "r"(kTmem)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -146,6 +161,8 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
             mbar_init(smem_addr(&u_full[i]), 1);
             mbar_init(smem_addr(&acc_full[i]), 1);
             mbar_init(smem_addr(&acc_free[i]), kLyEpiWarps);
+            mbar_init(smem_addr(&y_full[i]), kLyEpiWarps);
+            mbar_init(smem_addr(&o_full[i]), 1);
         }
         mbar_init(smem_addr(&g_full), 1);
         mbar_init(smem_addr(&hb_full), kLyCvtWarps);
@@ -162,6 +179,18 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                                    (nl & 7) * 16) =
             make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                        pack_bf16(f[6], f[7]));
+    }
+    if (HEAD) {
+        for (int u = threadIdx.x; u < 64 * (128 / 8); u += kLyThreads) {
+            const int n = u % 64, c = u / 64;
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                f[e] = n < kLyOut ? __ldg(a.w2 + (8 * c + e) * kLyOut + n) : 0.0f;
+            *reinterpret_cast<uint4 *>(sW2 + (c * 8 + (n >> 3)) * 128 + (n & 7) * 16) =
+                make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                           pack_bf16(f[6], f[7]));
+        }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -183,6 +212,36 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                     bias[nb][j] = make_float2(bp[0], bp[1]);
                 }
         }
+        // the 8 outputs of item k: 16 rows a warp
+        auto head_out = [&](int k) {
+            if (!mbar_wait_bounded(smem_addr(&o_full[k & 1]), (k >> 1) & 1)) return false;
+            tc_fence_after();
+            uint32_t r[4];
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                         : "r"(tmem + ((uint32_t)(quad * 32 + (warp >> 2) * 16) << 16) +
+                               (uint32_t)(256 + (k & 1) * 64)));
+            asm volatile("tcgen05.wait::ld.sync.aligned;"
+                         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])
+                         :
+                         : "memory");
+            tc_fence_before();
+            const long long it = first + k;
+            const int tile = (int)(it / a.B), b = (int)(it % a.B);
+            const int nrows = min(kLyRows, a.P - tile * kLyRows);
+            const float2 bias2 =
+                make_float2(__ldg(a.bias2 + 2 * (lane & 3)), __ldg(a.bias2 + 2 * (lane & 3) + 1));
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int row = quad * 32 + (warp >> 2) * 16 + t * 8 + (lane >> 2);
+                if (row < nrows)
+                    *reinterpret_cast<float2 *>(
+                        a.out2 + ((long long)b * a.P + (long long)tile * kLyRows + row) * kLyOut +
+                        2 * (lane & 3)) = make_float2(__uint_as_float(r[2 * t]) + bias2.x,
+                                                      __uint_as_float(r[2 * t + 1]) + bias2.y);
+            }
+            return true;
+        };
         for (int i = 0; i < items; ++i) {
             const long long it = first + i;
             const int tile = (int)(it / a.B), b = (int)(it % a.B), buf = i & 1;
@@ -232,7 +291,8 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                 }
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                    if (r0 + 8 * t >= nrows) continue;
+                    const bool in = r0 + 8 * t < nrows;
+                    if (!HEAD && !in) continue;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         float2 v = make_float2(s[t >> 1][4 * j + 2 * (t & 1)],
@@ -245,14 +305,31 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                             v.x *= layer_dgelu(zin[t][j].x);
                             v.y *= layer_dgelu(zin[t][j].y);
                         }
-                        *reinterpret_cast<float2 *>(a.out0 + e) = v;
-                        if (EPI == kEpiForward && a.out1)
-                            *reinterpret_cast<float2 *>(a.out1 + e) =
-                                make_float2(layer_gelu(v.x), layer_gelu(v.y));
+                        if (in) *reinterpret_cast<float2 *>(a.out0 + e) = v;
+                        if (EPI == kEpiForward && (HEAD || a.out1)) {
+                            const float2 y = make_float2(layer_gelu(v.x), layer_gelu(v.y));
+                            if (in) *reinterpret_cast<float2 *>(a.out1 + e) = y;
+                            if (HEAD) {   // 8 rows x 4 lanes: 128 bytes in a row
+                                const int c = (nb * 64 + col0) / 8 + j, row = r0 + 8 * t;
+                                *reinterpret_cast<uint32_t *>(
+                                    sY + buf * kLyYBytes + (c * (kLyRows / 8) + (row >> 3)) * 128 +
+                                    (row & 7) * 16 + 4 * (lane & 3)) = pack_bf16(y.x, y.y);
+                            }
+                        }
                     }
                 }
             }
+            if (HEAD) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_addr(&y_full[buf]));
+                if (i >= 1) {
+                    ok = __all_sync(0xffffffffu, head_out(i - 1));
+                    if (!ok) break;
+                }
+            }
         }
+        if (HEAD && ok && items > 0) ok = __all_sync(0xffffffffu, head_out(items - 1));
     } else if (warp < kLyEpiWarps + kLyCvtWarps) {
         // ---- round h: 8 rows x 8 chunks of 8 columns per step of a warp; the
         // chunk and the half read first rotate with the row, so the 16-byte
@@ -331,7 +408,20 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
     } else {
         // ---- products
         if (lane == 0) {
-            int tile_now = -1, gloads = 0, done = 0;
+            int tile_now = -1, gloads = 0, done = 0, heads = 0;
+            auto head = [&](int k) {   // the third product of item k
+                if (!mbar_wait_bounded(smem_addr(&y_full[k & 1]), (k >> 1) & 1)) return false;
+                tc_fence_after();
+#pragma unroll
+                for (int s = 0; s < 128 / 16; ++s)
+                    mma_bf16(tmem + 256 + (k & 1) * 64,
+                             smem_desc(smem_addr(sY + (k & 1) * kLyYBytes) + s * 2 * 2048, 2048,
+                                       128),
+                             smem_desc(smem_addr(sW2) + s * 2 * 1024, 1024, 128), s > 0 ? 1u : 0u);
+                mma_commit(smem_addr(&o_full[k & 1]));
+                ++heads;
+                return true;
+            };
             for (int i = 0; i < items; ++i) {
                 const int tile = (int)((first + i) / a.B), buf = i & 1;
                 if (i >= 2)
@@ -377,11 +467,19 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                 }
                 mma_commit(smem_addr(&acc_full[buf]));
                 ++done;
+                if (HEAD && i >= 1) {
+                    ok = head(i - 1);
+                    if (!ok) break;
+                }
             }
+            if (HEAD && ok && items > 0) ok = head(items - 1);
             // TMEM and shared memory are given back only after every product
             if (done)
                 ok = mbar_wait_bounded(smem_addr(&acc_full[(done - 1) & 1]),
                                        ((done - 1) >> 1) & 1) && ok;
+            if (heads)
+                ok = mbar_wait_bounded(smem_addr(&o_full[(heads - 1) & 1]),
+                                       ((heads - 1) >> 1) & 1) && ok;
         }
     }
     if (!ok) atomicExch(&g_gemm_wait_fail, 1);
@@ -391,7 +489,7 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(kLyTmem)
+                     "r"(kTmem)
                      : "memory");
     }
 }
@@ -419,6 +517,139 @@ __global__ void basis_image_kernel(const float *src, long long s_row, long long 
         }
         img[u] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                             pack_bf16(f[6], f[7]));
+    }
+}
+
+}  // namespace
+
+namespace {
+
+// The lift z = x W + bias (x: rows x 6, 64 columns).  One MMA of K 16 a tile and
+// 24 bytes a row in for 256 out: bound by the stores.  Four CTAs of 128 threads
+// per SM (their TMEM is 2 x 64 columns each) take even shares of the 128-row
+// tiles; the rows of tile i + 1 are fetched into registers and the product of
+// tile i runs while tile i - 1 is stored.
+constexpr int kLiftK = 6;
+
+__global__ void __launch_bounds__(128, 4) nn_lift_kernel(const float *x, const float *w,
+                                                         const float *bias, long long rows,
+                                                         float *z) {
+    __shared__ __align__(1024) unsigned char sA[2][kLyRows * 16 * 2];
+    __shared__ __align__(1024) unsigned char sB[kLyW * 16 * 2];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = (rows + kLyRows - 1) / kLyRows;
+    const long long first = layer_first(total, blockIdx.x, gridDim.x);
+    const int items = (int)(layer_first(total, blockIdx.x + 1, gridDim.x) - first);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "r"(128)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        mbar_init(smem_addr(&bar[0]), 1);
+        mbar_init(smem_addr(&bar[1]), 1);
+        mbar_init_fence();
+    }
+    // K 6 .. 15 of both operands stay zero
+    for (int u = threadIdx.x; u < 2 * kLyRows * 2; u += 128)
+        reinterpret_cast<uint4 *>(sA)[u] = make_uint4(0, 0, 0, 0);
+    {
+        const int n = threadIdx.x & 63, c = threadIdx.x >> 6;
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            f[e] = 8 * c + e < kLiftK ? __ldg(w + (8 * c + e) * kLyW + n) : 0.0f;
+        *reinterpret_cast<uint4 *>(sB + (c * 8 + (n >> 3)) * 128 + (n & 7) * 16) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+                       pack_bf16(f[6], f[7]));
+    }
+    float2 bs[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        bs[j] = make_float2(__ldg(bias + 8 * j + 2 * (lane & 3)),
+                            __ldg(bias + 8 * j + 2 * (lane & 3) + 1));
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    // element e = thread + 128 j of a tile's 768: row e / 6, k e % 6
+    float v[kLiftK];
+    auto load = [&](int i) {
+        const long long base = (first + i) * (kLyRows * kLiftK);
+#pragma unroll
+        for (int j = 0; j < kLiftK; ++j) {
+            const long long e = base + threadIdx.x + 128 * j;
+            v[j] = e < rows * kLiftK ? __ldg(x + e) : 0.0f;
+        }
+    };
+    auto store = [&](int i) {
+        if (!mbar_wait_bounded(smem_addr(&bar[i & 1]), (i >> 1) & 1)) return false;
+        tc_fence_after();
+        const long long r0 = (first + i) * kLyRows + warp * 32 + (lane >> 2);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {   // 16 rows x 32 columns each
+            const int hf = p >> 1, col = (p & 1) * 32;
+            float s[16];
+            tmem_ld_16x32(tmem + ((uint32_t)(warp * 32 + hf * 16) << 16) +
+                              (uint32_t)((i & 1) * 64 + col),
+                          s);
+            tmem_ld_wait(s);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const long long row = r0 + hf * 16 + t * 8;
+                if (row >= rows) continue;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 b = bs[col / 8 + j];
+                    *reinterpret_cast<float2 *>(z + row * kLyW + col + 8 * j + 2 * (lane & 3)) =
+                        make_float2(s[4 * j + 2 * t] + b.x, s[4 * j + 2 * t + 1] + b.y);
+                }
+            }
+        }
+        tc_fence_before();
+        return true;
+    };
+    bool ok = true;
+    int issued = 0;
+    if (items > 0) load(0);
+    for (int i = 0; i < items; ++i) {
+#pragma unroll
+        for (int j = 0; j < kLiftK; ++j) {
+            const int e = threadIdx.x + 128 * j, row = e / kLiftK, k = e % kLiftK;
+            *reinterpret_cast<__nv_bfloat16 *>(sA[i & 1] + (row >> 3) * 128 + (row & 7) * 16 +
+                                               2 * k) = __float2bfloat16_rn(v[j]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tc_fence_before();
+        if (!__syncthreads_and(ok)) break;
+        if (threadIdx.x == 0) {
+            tc_fence_after();
+            mma_bf16(tmem + (i & 1) * 64, smem_desc(smem_addr(sA[i & 1]), 2048, 128),
+                     smem_desc(smem_addr(sB), 1024, 128), 0u);
+            mma_commit(smem_addr(&bar[i & 1]));
+        }
+        issued = i + 1;
+        __syncwarp();
+        if (i + 1 < items) load(i + 1);
+        if (i >= 1) ok = __all_sync(0xffffffffu, store(i - 1));
+    }
+    if (issued == items && ok) {
+        if (items > 0) ok = __all_sync(0xffffffffu, store(items - 1));
+    } else if (issued) {   // a wait gave up: TMEM goes back only after every product
+        ok = false;
+        mbar_wait_bounded(smem_addr(&bar[(issued - 1) & 1]), ((issued - 1) >> 1) & 1);
+    }
+    if (!ok && lane == 0) atomicExch(&g_gemm_wait_fail, 1);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128)
+                     : "memory");
     }
 }
 

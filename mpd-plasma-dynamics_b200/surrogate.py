@@ -160,7 +160,6 @@ class SpectralOperator:
         self.zp = torch.zeros(rows, HIDDEN, **f32)
         self.y1 = torch.zeros(rows, HIDDEN, **f32)
         self.out = torch.zeros(rows, N_OUT, **f32)
-        self.zo = torch.zeros(rows, N_OUT, **f32)
         # backward scratch
         self.g_a = torch.zeros(rows, max(WIDTH, HIDDEN), **f32)
         self.g_b = torch.zeros(rows, max(WIDTH, HIDDEN), **f32)
@@ -197,17 +196,6 @@ class SpectralOperator:
     def _chk(self, rc):
         N.check(rc, self.lib)
 
-    def _linear(self, x, k_in, Wt, n_out, out, beta=0.0):
-        """out[rows, n_out] (+)= x[rows, k_in] @ Wt[k_in, n_out]."""
-        rows = x.shape[0]
-        nn.gemm(x, Wt, out, rows, n_out, k_in, 1, sa=(x.stride(0), 1, 0), sb=(1, n_out, 0),
-                sc=(out.stride(0), 1, 0), beta=beta)
-
-    def _bias_act(self, z, b, out, act):
-        self._chk(self.lib.mpd_nn_bias_act(C.c_void_p(z.data_ptr()), C.c_void_p(b.data_ptr()),
-                                           C.c_void_p(out.data_ptr()), z.shape[0], z.shape[1],
-                                           int(act), self._s()))
-
     def _wgrad(self, a, k_in, gz, n_out, dst):
         """dst[k_in, n_out] = sum over rows of a[:, :k_in]^T gz, split by sample."""
         B, P = self.B, self.P
@@ -231,8 +219,7 @@ class SpectralOperator:
     def forward(self):
         B, P, Cw = self.B, self.P, WIDTH
         p = self.p
-        self._linear(self.x, N_IN, p["W_in"], Cw, self.z[0])
-        self._bias_act(self.z[0], p["b_in"], self.h[0], act=False)
+        nn.lift(self.x, p["W_in"], p["b_in"], self.z[0])
         for l in range(LAYERS):
             h, z = self.h[l], self.z[l + 1]
             # V[b] = F h[b] (Q x C), U[b, q] = V[b, q] R[q]
@@ -243,9 +230,7 @@ class SpectralOperator:
                      bias=p[f"b{l}"],
                      out1=self.h[l + 1] if l < LAYERS - 1 else None)
         nn.layer(self.h[LAYERS], p["W_p1"], 1, HIDDEN, self.zp, B * P, 1, n_out=HIDDEN,
-                 bias=p["b_p1"], out1=self.y1)
-        self._linear(self.y1, HIDDEN, p["W_p2"], N_OUT, self.zo)
-        self._bias_act(self.zo, p["b_p2"], self.out, act=False)
+                 bias=p["b_p1"], out1=self.y1, w2=p["W_p2"], bias2=p["b_p2"], out2=self.out)
         return self.out
 
     def loss_and_grad(self, target) -> None:

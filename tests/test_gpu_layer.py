@@ -68,7 +68,7 @@ def test_layer_is_the_separate_launches(pkg, P, B):
 
 
 @pytest.mark.parametrize("rows", [1, 128, 1001, 40000])
-def test_wide_linear_is_the_separate_launches(pkg, rows):
+def test_projection_is_the_separate_launches(pkg, rows):
     import torch
     nn, lib, o = pkg.nn, pkg._native.load(), _operands(rows, 1, rows)
     W = torch.randn(64, 128, device="cuda") / 8
@@ -76,9 +76,29 @@ def test_wide_linear_is_the_separate_launches(pkg, rows):
     z, out = torch.empty(rows, 128, device="cuda"), torch.empty(rows, 128, device="cuda")
     nn.gemm(o["h"], W, z, rows, 128, 64, 1, sa=(64, 1, 0), sb=(1, 128, 0), sc=(128, 1, 0))
     assert lib.mpd_nn_bias_act(_ptr(z), _ptr(bias), _ptr(out), rows, 128, 1, nn._stream()) == 0
-    got0, got1 = torch.full_like(z, 7.0), torch.full_like(z, 7.0)
-    nn.layer(o["h"], W, 1, 128, got0, rows, 1, n_out=128, bias=bias, out1=got1)
-    assert torch.equal(got0, z) and torch.equal(got1, out)
+    W2, bias2 = torch.randn(128, 8, device="cuda") / 11, torch.randn(8, device="cuda")
+    zo, y = torch.empty(rows, 8, device="cuda"), torch.empty(rows, 8, device="cuda")
+    nn.gemm(out, W2, zo, rows, 8, 128, 1, sa=(128, 1, 0), sb=(1, 8, 0), sc=(8, 1, 0))
+    assert lib.mpd_nn_bias_act(_ptr(zo), _ptr(bias2), _ptr(y), rows, 8, 0, nn._stream()) == 0
+    got0, got1, got2 = (torch.full_like(t, 7.0) for t in (z, out, y))
+    nn.layer(o["h"], W, 1, 128, got0, rows, 1, n_out=128, bias=bias, out1=got1, w2=W2,
+             bias2=bias2, out2=got2)
+    assert torch.equal(got0, z) and torch.equal(got1, out) and torch.equal(got2, y)
+    nn.wait_status()
+
+
+@pytest.mark.parametrize("rows", [1, 127, 129, 75777, 300000])
+def test_lift_is_the_separate_launches(pkg, rows):
+    import torch
+    nn, lib = pkg.nn, pkg._native.load()
+    x, W = torch.randn(rows, 6, device="cuda"), torch.randn(6, 64, device="cuda")
+    bias = torch.randn(64, device="cuda")
+    z, h = torch.empty(rows, 64, device="cuda"), torch.empty(rows, 64, device="cuda")
+    nn.gemm(x, W, z, rows, 64, 6, 1, sa=(6, 1, 0), sb=(1, 64, 0), sc=(64, 1, 0))
+    assert lib.mpd_nn_bias_act(_ptr(z), _ptr(bias), _ptr(h), rows, 64, 0, nn._stream()) == 0
+    got = torch.full_like(z, 7.0)
+    nn.lift(x, W, bias, got)
+    assert torch.equal(got, z)
     nn.wait_status()
 
 
