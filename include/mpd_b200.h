@@ -397,9 +397,10 @@ int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream);
  *   MPD_NN_FORWARD  out0 = s + bias; out1 = GELU(out0) (out1 may be NULL)
  *   MPD_NN_ACT_BWD  out0 = s * GELU'(z_in)
  *   MPD_NN_PLAIN    out0 = s
- * With basis == NULL: the projection, s = h W with n_out = 128 columns and
- *   MPD_NN_FORWARD  (out1 not NULL), and out2 = out1 W2 + bias2 with 8 columns,
- *                   W2(k, n) at w2[k * 8 + n]
+ * With basis == NULL: the projection, s = h W with n_out = 128 columns, and
+ * the product after it, W2(n, k) at w2[n * w2_sn + k * w2_sk]:
+ *   MPD_NN_FORWARD  (out1 not NULL), out2 = out1 W2 + bias2 with 8 columns
+ *   MPD_NN_ACT_BWD  h: rows x 8, out2 = out0 W2 with 64 columns
  * h, out0, out1, out2, z_in, basis and u_image start on 16-byte boundaries. */
 enum { MPD_NN_FORWARD = 0, MPD_NN_ACT_BWD = 1, MPD_NN_PLAIN = 2 };
 typedef struct mpd_layer_desc {
@@ -410,6 +411,7 @@ typedef struct mpd_layer_desc {
     const float *bias, *z_in;
     float *out0, *out1;
     const float *w2, *bias2;
+    long long w2_sn, w2_sk;
     float *out2;
 } mpd_layer_desc;
 

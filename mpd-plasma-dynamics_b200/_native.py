@@ -109,7 +109,8 @@ class LayerDesc(C.Structure):
                 ("w_sk", C.c_longlong), ("basis", C.c_void_p), ("u_image", C.c_void_p),
                 ("bias", C.c_void_p), ("z_in", C.c_void_p),
                 ("out0", C.c_void_p), ("out1", C.c_void_p), ("w2", C.c_void_p),
-                ("bias2", C.c_void_p), ("out2", C.c_void_p)]
+                ("bias2", C.c_void_p), ("w2_sn", C.c_longlong), ("w2_sk", C.c_longlong),
+                ("out2", C.c_void_p)]
 
 
 class SpectralDesc(C.Structure):

@@ -469,13 +469,13 @@ int NnLaunched(const char *what) {
     return MPD_ERR_CUDA;
 }
 
-template <int K2, int NB, int EPI, bool HEAD>
+template <int K1, int K2, int NB, int EPI, int OUT2>
 int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
-    constexpr int smem = layer_smem<K2, NB, HEAD>();
+    constexpr int smem = layer_smem<K2, NB, OUT2>();
     static bool attr_set = false;  // per process; the attribute is per function
     if (!attr_set) {
         const cudaError_t e = cudaFuncSetAttribute(
-            nn_layer_kernel<K2, NB, EPI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            nn_layer_kernel<K1, K2, NB, EPI, OUT2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) {
             mpd::SetLastError(std::string("mpd_nn_layer: ") + cudaGetErrorString(e));
             return MPD_ERR_CUDA;
@@ -483,7 +483,7 @@ int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
         attr_set = true;
     }
     const long long items = (long long)a.tiles * a.B;
-    nn_layer_kernel<K2, NB, EPI, HEAD>
+    nn_layer_kernel<K1, K2, NB, EPI, OUT2>
         <<<(int)(items < 148 ? items : 148), kLyThreads, smem, st>>>(a);
     return NnLaunched("mpd_nn_layer");
 }
@@ -563,12 +563,13 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
         return MPD_ERR_INVALID;
     }
     const bool spectral = d->basis != nullptr;
+    const bool fwd = d->epilogue == MPD_NN_FORWARD, bwd = d->epilogue == MPD_NN_ACT_BWD;
     const bool shape_ok = spectral ? d->n_out == 64 && d->u_image
-                                   : d->n_out == 128 && d->out1 && d->w2 && d->bias2 && d->out2;
-    const bool epi_ok = d->epilogue == MPD_NN_FORWARD ? d->bias != nullptr
-                        : !spectral                   ? false
-                        : d->epilogue == MPD_NN_ACT_BWD ? d->z_in != nullptr
-                                                        : d->epilogue == MPD_NN_PLAIN;
+                                   : d->n_out == 128 && d->w2 && d->out2 &&
+                                         (!fwd || (d->out1 && d->bias2));
+    const bool epi_ok = fwd   ? d->bias != nullptr
+                        : bwd ? d->z_in != nullptr
+                              : spectral && d->epilogue == MPD_NN_PLAIN;
     if (!shape_ok || !epi_ok || !Aligned16(d->h) || !Aligned16(d->out0) || !Aligned16(d->out1) ||
         !Aligned16(d->z_in) || !Aligned16(d->out2) || !Aligned16(d->basis) || !Aligned16(d->u_image)) {
         mpd::SetLastError("mpd_nn_layer: unsupported widths, epilogue or alignment");
@@ -590,6 +591,8 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     a.bias = d->bias;
     a.z_in = d->z_in;
     a.w2 = d->w2;
+    a.w2_sn = d->w2_sn;
+    a.w2_sk = d->w2_sk;
     a.bias2 = d->bias2;
     a.out2 = d->out2;
     a.out0 = d->out0;
@@ -597,10 +600,12 @@ int mpd_nn_layer(const mpd_layer_desc *d, void *stream) {
     a.P = d->P;
     a.B = d->B;
     a.tiles = (d->P + kLyRows - 1) / kLyRows;
-    if (!spectral) return LaunchLayer<0, 2, kEpiForward, true>(a, st);
-    if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyQ, 1, kEpiForward, false>(a, st);
-    if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyQ, 1, kEpiActBwd, false>(a, st);
-    return LaunchLayer<kLyQ, 1, kEpiPlain, false>(a, st);
+    if (!spectral && d->epilogue == MPD_NN_FORWARD)
+        return LaunchLayer<kLyW, 0, 2, kEpiForward, 8>(a, st);
+    if (!spectral) return LaunchLayer<8, 0, 2, kEpiActBwd, kLyW>(a, st);
+    if (d->epilogue == MPD_NN_FORWARD) return LaunchLayer<kLyW, kLyQ, 1, kEpiForward, 0>(a, st);
+    if (d->epilogue == MPD_NN_ACT_BWD) return LaunchLayer<kLyW, kLyQ, 1, kEpiActBwd, 0>(a, st);
+    return LaunchLayer<kLyW, kLyQ, 1, kEpiPlain, 0>(a, st);
 }
 
 int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream) {

@@ -40,10 +40,9 @@ constexpr int kLyHBytes = kLyRows * kLyW * 4;     // 32 KB
 constexpr int kLyHbBytes = kLyRows * kLyW * 2;    // 16 KB
 constexpr int kLyWBytes = kLyW * kLyW * 2;        // 8 KB per 64 output columns
 constexpr uint32_t kLyTmem = 256;
-// The 128-wide projection with the 8 outputs after it (HEAD):
-constexpr int kLyOut = 8;
+// The 128-wide projection with another product after it (OUT2 columns):
 constexpr int kLyYBytes = kLyRows * 128 * 2;      // 32 KB: GELU(z) in BF16
-constexpr int kLyW2Bytes = 64 * 128 * 2;          // 16 KB: 8 columns, the rest zero
+constexpr int kLyW2Bytes = 64 * 128 * 2;          // 16 KB: columns past OUT2 are zero
 
 enum LayerEpilogue { kEpiForward = 0, kEpiActBwd = 1, kEpiPlain = 2 };
 
@@ -56,8 +55,9 @@ struct LayerArgs {
     const float *bias;           // forward
     const float *z_in;           // kEpiActBwd: GELU' is taken at these
     float *out0, *out1;          // out1: GELU(out0), or NULL
-    const float *w2, *bias2;     // HEAD: (k, n) at w2[k * 8 + n]
-    float *out2;                 // HEAD: rows x 8
+    const float *w2, *bias2;     // OUT2: (n, k) at w2[n * w2_sn + k * w2_sk]
+    long long w2_sn, w2_sk;
+    float *out2;                 // rows x OUT2
     int P, B, tiles;             // rows of one sample, samples, 128-row tiles of one sample
 };
 
@@ -116,20 +116,30 @@ __device__ __forceinline__ float layer_dgelu(float x) {
     return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * c * (1.0f + 3.0f * 0.044715f * x * x);
 }
 
-template <int K2, int NB, bool HEAD>
+template <int K2, int NB, int OUT2>
 constexpr int layer_smem() {
     return (K2 ? kLyGBytes + 2 * kLyUBytes : 0) + 2 * kLyHBytes + kLyHbBytes + NB * kLyWBytes +
-           (HEAD ? 2 * kLyYBytes + kLyW2Bytes : 0);
+           (OUT2 ? 2 * kLyYBytes + kLyW2Bytes : 0);
 }
 
-// HEAD (with NB == 2, forward): out2 = GELU(z) W2 + bias2, while GELU(z) is in
-// registers: the epilogue also leaves it in BF16 as the A operand of a third
-// product, whose result it stores one item later.  As its own launch it read
-// the 528 MB of out1 back (16 x 64400 rows).
-template <int K2, int NB, int EPI, bool HEAD>
+// OUT2 (with NB == 2) is the projection and what follows it, while its values are
+// in registers: the epilogue also leaves them in BF16 as the A operand of a third
+// product, whose result it stores one item later.
+//   forward, OUT2 8:    out2 = GELU(z) W2 + bias2
+//   backward, OUT2 64:  out0 = (h W) GELU'(z_in) with h of K1 = 8 columns (the
+//                       gradient of the outputs), out2 = out0 W2
+// As its own launches the forward form read the 528 MB of out1 back (16 x 64400
+// rows: 230 + 340 us, here 268 where memory alone takes 207), the backward one
+// moved its 128 columns five times (96 us at 65600 rows, here 33).  The
+// epilogue's tanh and 32-byte stores bound both; 16 epilogue warps instead of 8
+// gave 285 and 33.
+template <int K1, int K2, int NB, int EPI, int OUT2>
 __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs a) {
     static_assert(K2 == 0 || NB == 1, "one accumulator pair of 64 columns each");
-    static_assert(!HEAD || (K2 == 0 && NB == 2 && EPI == kEpiForward), "after the projection");
+    constexpr bool HEAD = OUT2 != 0;
+    static_assert(!HEAD || (K2 == 0 && NB == 2 && EPI != kEpiPlain), "after the projection");
+    static_assert(K1 == kLyW || K1 == 8, "whole chunks of h, one product of K 16 at least");
+    constexpr int kHRow = K1 * 4;   // bytes of a row of h
     constexpr uint32_t kTmem = HEAD ? 512 : kLyTmem;
     extern __shared__ __align__(1024) unsigned char gemm_smem[];
     __shared__ __align__(8) uint64_t h_full[2], h_free[2], u_full[2], acc_full[2], acc_free[2],
@@ -170,23 +180,28 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
         mbar_init_fence();
     }
     // W rounded once: (n, k) of 64-column block n / 64
-    for (int u = threadIdx.x; u < NB * kLyW * (kLyW / 8); u += kLyThreads) {
+    constexpr int kK1 = K1 < 16 ? 16 : K1;   // zero past K1
+    for (int u = threadIdx.x; u < NB * kLyW * (kK1 / 8); u += kLyThreads) {
         const int n = u % (NB * kLyW), c = u / (NB * kLyW), nl = n % kLyW;
         float f[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = __ldg(a.w + n * a.w_sn + (8 * c + e) * a.w_sk);
+        for (int e = 0; e < 8; ++e)
+            f[e] = 8 * c + e < K1 ? __ldg(a.w + n * a.w_sn + (8 * c + e) * a.w_sk) : 0.0f;
         *reinterpret_cast<uint4 *>(sW + (n / kLyW) * kLyWBytes + (c * (kLyW / 8) + (nl >> 3)) * 128 +
                                    (nl & 7) * 16) =
             make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                        pack_bf16(f[6], f[7]));
     }
+    if (K1 < 16)   // the second chunk of K
+        for (int u = threadIdx.x; u < kLyRows; u += kLyThreads)
+            reinterpret_cast<uint4 *>(sHb + 2048)[u] = make_uint4(0, 0, 0, 0);
     if (HEAD) {
         for (int u = threadIdx.x; u < 64 * (128 / 8); u += kLyThreads) {
             const int n = u % 64, c = u / 64;
             float f[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                f[e] = n < kLyOut ? __ldg(a.w2 + (8 * c + e) * kLyOut + n) : 0.0f;
+                f[e] = n < OUT2 ? __ldg(a.w2 + n * a.w2_sn + (8 * c + e) * a.w2_sk) : 0.0f;
             *reinterpret_cast<uint4 *>(sW2 + (c * 8 + (n >> 3)) * 128 + (n & 7) * 16) =
                 make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                            pack_bf16(f[6], f[7]));
@@ -212,34 +227,54 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                     bias[nb][j] = make_float2(bp[0], bp[1]);
                 }
         }
-        // the 8 outputs of item k: 16 rows a warp
+        // the third product of item k: 16 rows a warp
         auto head_out = [&](int k) {
             if (!mbar_wait_bounded(smem_addr(&o_full[k & 1]), (k >> 1) & 1)) return false;
             tc_fence_after();
-            uint32_t r[4];
-            asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                         : "r"(tmem + ((uint32_t)(quad * 32 + (warp >> 2) * 16) << 16) +
-                               (uint32_t)(256 + (k & 1) * 64)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;"
-                         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])
-                         :
-                         : "memory");
-            tc_fence_before();
+            const int rw = quad * 32 + (warp >> 2) * 16;
+            const uint32_t ta = tmem + ((uint32_t)rw << 16) + (uint32_t)(256 + (k & 1) * 64);
             const long long it = first + k;
             const int tile = (int)(it / a.B), b = (int)(it % a.B);
             const int nrows = min(kLyRows, a.P - tile * kLyRows);
-            const float2 bias2 =
-                make_float2(__ldg(a.bias2 + 2 * (lane & 3)), __ldg(a.bias2 + 2 * (lane & 3) + 1));
+            float *o = a.out2 + ((long long)b * a.P + (long long)tile * kLyRows) * OUT2;
+            if constexpr (OUT2 == 8) {
+                uint32_t r[4];
+                asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                             : "r"(ta));
+                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                             : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])
+                             :
+                             : "memory");
+                const int n = 2 * (lane & 3);
+                const float2 bias2 = make_float2(__ldg(a.bias2 + n), __ldg(a.bias2 + n + 1));
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const int row = quad * 32 + (warp >> 2) * 16 + t * 8 + (lane >> 2);
-                if (row < nrows)
-                    *reinterpret_cast<float2 *>(
-                        a.out2 + ((long long)b * a.P + (long long)tile * kLyRows + row) * kLyOut +
-                        2 * (lane & 3)) = make_float2(__uint_as_float(r[2 * t]) + bias2.x,
-                                                      __uint_as_float(r[2 * t + 1]) + bias2.y);
+                for (int t = 0; t < 2; ++t) {
+                    const int row = rw + t * 8 + (lane >> 2);
+                    if (row < nrows)
+                        *reinterpret_cast<float2 *>(o + row * OUT2 + n) =
+                            make_float2(__uint_as_float(r[2 * t]) + bias2.x,
+                                        __uint_as_float(r[2 * t + 1]) + bias2.y);
+                }
+            } else if constexpr (OUT2 == 64) {
+#pragma unroll
+                for (int col = 0; col < 64; col += 32) {
+                    float v[16];
+                    tmem_ld_16x32(ta + col, v);
+                    tmem_ld_wait(v);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const int row = rw + t * 8 + (lane >> 2);
+                        if (row >= nrows) continue;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            *reinterpret_cast<float2 *>(o + row * OUT2 + col + 8 * j +
+                                                        2 * (lane & 3)) =
+                                make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
+                    }
+                }
             }
+            tc_fence_before();
             return true;
         };
         for (int i = 0; i < items; ++i) {
@@ -251,22 +286,24 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                 ((long long)b * a.P + (long long)tile * kLyRows + r0) * (NB * 64) + col0 +
                 2 * (lane & 3);
             float2 zin[4][4];
-            if (EPI == kEpiActBwd) {
+            auto load_z = [&](int nb) {
 #pragma unroll
                 for (int t = 0; t < 4; ++t)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         zin[t][j] = r0 + 8 * t < nrows
                                         ? __ldg(reinterpret_cast<const float2 *>(
-                                              a.z_in + at + t * 8 * (NB * 64) + 8 * j))
+                                              a.z_in + at + t * 8 * (NB * 64) + nb * 64 + 8 * j))
                                         : make_float2(0.0f, 0.0f);
-            }
+            };
+            if (EPI == kEpiActBwd) load_z(0);
             ok = mbar_wait_bounded(smem_addr(&acc_full[buf]), (i >> 1) & 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
+                if (EPI == kEpiActBwd && nb > 0) load_z(nb);
                 float s[2][16];
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
@@ -306,9 +343,12 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                             v.y *= layer_dgelu(zin[t][j].y);
                         }
                         if (in) *reinterpret_cast<float2 *>(a.out0 + e) = v;
-                        if (EPI == kEpiForward && (HEAD || a.out1)) {
-                            const float2 y = make_float2(layer_gelu(v.x), layer_gelu(v.y));
-                            if (in) *reinterpret_cast<float2 *>(a.out1 + e) = y;
+                        if (HEAD || (EPI == kEpiForward && a.out1)) {
+                            float2 y = v;
+                            if (EPI == kEpiForward) {
+                                y = make_float2(layer_gelu(v.x), layer_gelu(v.y));
+                                if (in) *reinterpret_cast<float2 *>(a.out1 + e) = y;
+                            }
                             if (HEAD) {   // 8 rows x 4 lanes: 128 bytes in a row
                                 const int c = (nb * 64 + col0) / 8 + j, row = r0 + 8 * t;
                                 *reinterpret_cast<uint32_t *>(
@@ -342,8 +382,16 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const unsigned char *src = sH + buf * kLyHBytes;
+            if (K1 < 16) {
+                const int row = cw * 32 + lane;
+                const float4 x = *reinterpret_cast<const float4 *>(src + row * kHRow);
+                const float4 y = *reinterpret_cast<const float4 *>(src + row * kHRow + 16);
+                *reinterpret_cast<uint4 *>(sHb + row * 16) =
+                    make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y),
+                               pack_bf16(y.z, y.w));
+            }
 #pragma unroll
-            for (int st = 0; st < 8; ++st) {
+            for (int st = 0; st < (K1 < 16 ? 0 : 8); ++st) {
                 const int row = cw * 32 + (st >> 1) * 8 + rl;
                 const int c = ((st & 1) * 4 + cg + rl) & 7;
                 const int swap = (rl >> 2) & 1;
@@ -372,12 +420,12 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                 const long long it = first + i;
                 const int tile = (int)(it / a.B), b = (int)(it % a.B), buf = i & 1;
                 const uint32_t hbytes =
-                    (uint32_t)min(kLyRows, a.P - tile * kLyRows) * (kLyW * 4);
+                    (uint32_t)min(kLyRows, a.P - tile * kLyRows) * kHRow;
                 if (i >= 2) ok = mbar_wait_bounded(smem_addr(&h_free[buf]), ((i - 2) >> 1) & 1);
                 if (!ok) break;
                 mbar_expect_tx(smem_addr(&h_full[buf]), hbytes);
                 bulk_load(smem_addr(sH + buf * kLyHBytes),
-                          a.h + ((long long)b * a.P + (long long)tile * kLyRows) * kLyW, hbytes,
+                          a.h + ((long long)b * a.P + (long long)tile * kLyRows) * K1, hbytes,
                           smem_addr(&h_full[buf]));
                 ++nh;
                 if (!K2) continue;
@@ -431,7 +479,7 @@ __global__ void __launch_bounds__(kLyThreads, 1) nn_layer_kernel(const LayerArgs
                 tc_fence_after();
                 const uint32_t d1 = tmem + (uint32_t)(buf * 128);
 #pragma unroll
-                for (int s = 0; s < kLyW / 16; ++s) {
+                for (int s = 0; s < kK1 / 16; ++s) {
                     const uint64_t ad = smem_desc(smem_addr(sHb) + s * 2 * (kLyRows / 8) * 128,
                                                   (kLyRows / 8) * 128, 128);
 #pragma unroll

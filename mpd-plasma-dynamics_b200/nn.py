@@ -59,15 +59,16 @@ def spectral(h, basis, R, r_sn, r_sk, V, U, u_image, P, B, work=None):
 
 
 def layer(h, w, w_sn, w_sk, out0, P, B, n_out=64, epilogue=FORWARD, basis=None, u_image=None,
-          bias=None, z_in=None, out1=None, w2=None, bias2=None, out2=None):
+          bias=None, z_in=None, out1=None, w2=None, bias2=None, out2=None,
+          w2_sn=0, w2_sk=0):
     """out0 = h W + basis U[b] (+ bias), out1 = GELU(out0); or the backward forms
-    of it; or the projection (n_out 128) with out2 = out1 W2 + bias2:
+    of it; or the projection (n_out 128) and the product after it, out2:
     mpd_nn_layer in include/mpd_b200.h."""
     lib = N.load()
     ptr = lambda t: None if t is None else t.data_ptr()
     d = N.LayerDesc(P, B, n_out, epilogue, h.data_ptr(), w.data_ptr(), w_sn, w_sk, ptr(basis),
                     ptr(u_image), ptr(bias), ptr(z_in), out0.data_ptr(), ptr(out1),
-                    ptr(w2), ptr(bias2), ptr(out2))
+                    ptr(w2), ptr(bias2), w2_sn, w2_sk, ptr(out2))
     N.check(lib.mpd_nn_layer(C.byref(d), _stream()), lib)
 
 

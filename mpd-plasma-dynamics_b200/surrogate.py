@@ -161,8 +161,7 @@ class SpectralOperator:
         self.y1 = torch.zeros(rows, HIDDEN, **f32)
         self.out = torch.zeros(rows, N_OUT, **f32)
         # backward scratch
-        self.g_a = torch.zeros(rows, max(WIDTH, HIDDEN), **f32)
-        self.g_b = torch.zeros(rows, max(WIDTH, HIDDEN), **f32)
+        self.gzp = torch.zeros(rows, HIDDEN, **f32)
         self.g_out = torch.zeros(rows, N_OUT, **f32)
         self.gh = [torch.zeros(rows, WIDTH, **f32) for _ in range(2)]
         self.gU = torch.zeros(batch, self.Q, WIDTH, **f32)
@@ -230,7 +229,8 @@ class SpectralOperator:
                      bias=p[f"b{l}"],
                      out1=self.h[l + 1] if l < LAYERS - 1 else None)
         nn.layer(self.h[LAYERS], p["W_p1"], 1, HIDDEN, self.zp, B * P, 1, n_out=HIDDEN,
-                 bias=p["b_p1"], out1=self.y1, w2=p["W_p2"], bias2=p["b_p2"], out2=self.out)
+                 bias=p["b_p1"], out1=self.y1, w2=p["W_p2"], w2_sn=1, w2_sk=N_OUT,
+                 bias2=p["b_p2"], out2=self.out)
         return self.out
 
     def loss_and_grad(self, target) -> None:
@@ -249,21 +249,15 @@ class SpectralOperator:
         # projection
         self._wgrad(self.y1, HIDDEN, self.g_out, N_OUT, g["W_p2"])
         self._colsum(self.g_out, g["b_p2"])
-        gy1 = self.g_a[:, :HIDDEN]
-        nn.gemm(self.g_out, p["W_p2"], gy1, rows, HIDDEN, N_OUT, 1, sa=(N_OUT, 1, 0),
-                sb=(N_OUT, 1, 0), sc=(self.g_a.stride(0), 1, 0))
-        gzp = self.g_b[:, :HIDDEN]
-        self._chk(self.lib.mpd_nn_act_bwd(C.c_void_p(gy1.data_ptr()), C.c_void_p(self.zp.data_ptr()),
-                                          C.c_void_p(gzp.data_ptr()), rows * HIDDEN, self._s()))
+        # gzp = (g_out W_p2^T) GELU'(zp), gh = gzp W_p1^T
+        gzp, gh = self.gzp, self.gh[0]
+        nn.layer(self.g_out, p["W_p2"], N_OUT, 1, gzp, rows, 1, n_out=HIDDEN,
+                 epilogue=nn.ACT_BWD, z_in=self.zp, w2=p["W_p1"], w2_sn=HIDDEN, w2_sk=1, out2=gh)
         self._wgrad(self.h[LAYERS], Cw, gzp, HIDDEN, g["W_p1"])
         self._colsum(gzp, g["b_p1"])
-        gh = self.gh[0]
-        nn.gemm(gzp, p["W_p1"], gh, rows, Cw, HIDDEN, 1, sa=(HIDDEN, 1, 0), sb=(HIDDEN, 1, 0),
-                sc=(Cw, 1, 0))
         gz = gh   # the last layer has no activation
         for l in reversed(range(LAYERS)):
-            h = self.h[l]
-            self._wgrad(h, Cw, gz, Cw, g[f"W{l}"])
+            self._wgrad(self.h[l], Cw, gz, Cw, g[f"W{l}"])
             self._colsum(gz, g[f"b{l}"])
             # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T
             nn.spectral(gz, self.Gt_img, p[f"R{l}"], Cw, 1, self.gU, self.gV, self.u_image, P, B,

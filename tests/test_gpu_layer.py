@@ -82,8 +82,17 @@ def test_projection_is_the_separate_launches(pkg, rows):
     assert lib.mpd_nn_bias_act(_ptr(zo), _ptr(bias2), _ptr(y), rows, 8, 0, nn._stream()) == 0
     got0, got1, got2 = (torch.full_like(t, 7.0) for t in (z, out, y))
     nn.layer(o["h"], W, 1, 128, got0, rows, 1, n_out=128, bias=bias, out1=got1, w2=W2,
-             bias2=bias2, out2=got2)
+             w2_sn=1, w2_sk=8, bias2=bias2, out2=got2)
     assert torch.equal(got0, z) and torch.equal(got1, out) and torch.equal(got2, y)
+    # backward: from the gradient of the 8 outputs to the 64 columns of h
+    gz, gh = torch.empty_like(z), torch.empty(rows, 64, device="cuda")
+    nn.gemm(y, W2, out, rows, 128, 8, 1, sa=(8, 1, 0), sb=(8, 1, 0), sc=(128, 1, 0))
+    assert lib.mpd_nn_act_bwd(_ptr(out), _ptr(z), _ptr(gz), gz.numel(), nn._stream()) == 0
+    nn.gemm(gz, W, gh, rows, 64, 128, 1, sa=(128, 1, 0), sb=(128, 1, 0), sc=(64, 1, 0))
+    got2 = torch.full_like(gh, 7.0)
+    nn.layer(y, W2, 8, 1, got0, rows, 1, n_out=128, epilogue=nn.ACT_BWD, z_in=z, w2=W,
+             w2_sn=128, w2_sk=1, out2=got2)
+    assert torch.equal(got0, gz) and torch.equal(got2, gh)
     nn.wait_status()
 
 
