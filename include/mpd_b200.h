@@ -417,6 +417,14 @@ typedef struct mpd_layer_desc {
 
 int mpd_nn_layer(const mpd_layer_desc *d, void *stream);
 
+/* dw(m, n) = sum over rows of a(r, m) g(r, n) and db(n) = sum over rows of
+ * g(r, n) for B samples of P rows, with the roundings, the split of K and the
+ * orders of the GEMM, mpd_nn_sum_parts and mpd_nn_colsum: (k_in, n_out) of (6, 64),
+ * (64, 64), (64, 128) or (128, 8), all dense.  work: at least B * k_in * n_out
+ * floats (K is split as far as it has room for), colwork: 128 * n_out floats. */
+int mpd_nn_wgrad(const float *a, const float *g, int k_in, int n_out, int P, int B, float *dw,
+                 float *db, float *work, long long work_floats, float *colwork, void *stream);
+
 /* z = x W + bias with the GEMM's roundings: x rows x 6, W 6 x 64 (both dense),
  * z rows x 64 on a 16-byte boundary. */
 int mpd_nn_lift(const float *x, const float *w, const float *bias, float *z, long long rows,

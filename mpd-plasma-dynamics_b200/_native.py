@@ -172,6 +172,8 @@ SIGNATURES = [
                                      _VP, _VP]),
     ("mpd_nn_spectral", C.c_int, [C.POINTER(SpectralDesc), _VP]),
     ("mpd_nn_layer", C.c_int, [C.POINTER(LayerDesc), _VP]),
+    ("mpd_nn_wgrad", C.c_int, [_VP, _VP, C.c_int, C.c_int, C.c_int, C.c_int, _VP, _VP, _VP,
+                               C.c_longlong, _VP, _VP]),
     ("mpd_nn_lift", C.c_int, [_VP, _VP, _VP, _VP, C.c_longlong, _VP]),
     ("mpd_nn_bias_act", C.c_int, [_VP, _VP, _VP, C.c_longlong, C.c_int, C.c_int, _VP]),
     ("mpd_nn_act_bwd", C.c_int, [_VP, _VP, _VP, C.c_longlong, _VP]),

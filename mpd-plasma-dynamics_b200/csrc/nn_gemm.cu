@@ -440,6 +440,7 @@ __global__ void nn_gemm_reduce_kernel(const mpd_gemm_desc d, int ksplit) {
 
 #include "nn_layer.cuh"
 #include "nn_spectral.cuh"
+#include "nn_wgrad.cuh"
 
 namespace {
 
@@ -488,6 +489,31 @@ int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
     return NnLaunched("mpd_nn_layer");
 }
 
+template <int KA, int N>
+int LaunchWgrad(WgradArgs a, long long work_floats, cudaStream_t st) {
+    constexpr int smem = wg_smem<KA, N>();
+    SplitK(KA, N, a.P, a.B, work_floats, &a.ksplit, &a.kspan);
+    if ((long long)a.B * a.ksplit > 65535 ||
+        (long long)a.ksplit * a.B * KA * N > work_floats) {
+        mpd::SetLastError("mpd_nn_wgrad: batch too large for one launch or for its scratch");
+        return MPD_ERR_INVALID;
+    }
+    static bool attr_set = false;  // per process; the attribute is per function
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            nn_wgrad_kernel<KA, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) {
+            mpd::SetLastError(std::string("mpd_nn_wgrad: ") + cudaGetErrorString(e));
+            return MPD_ERR_CUDA;
+        }
+        attr_set = true;
+    }
+    nn_wgrad_kernel<KA, N><<<a.B * a.ksplit + ((N + 31) / 32) * kWgColSlices, kWgThreads, smem,
+                             st>>>(a);
+    nn_wgrad_sum_kernel<<<(KA * N + 31) / 32 + (N + 255) / 256, 256, 0, st>>>(a, KA * N, N);
+    return NnLaunched("mpd_nn_wgrad");
+}
+
 bool Aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -504,6 +530,32 @@ int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int row
     basis_image_kernel<<<148 * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         src, s_row, s_k, rows, K, mt, block_k, nkb, static_cast<uint4 *>(image));
     return NnLaunched("mpd_nn_basis_image");
+}
+
+int mpd_nn_wgrad(const float *a, const float *g, int k_in, int n_out, int P, int B, float *dw,
+                 float *db, float *work, long long work_floats, float *colwork, void *stream) {
+    if (!a || !g || !dw || !db || !work || !colwork || P < 1 || B < 0 || !Aligned16(work)) {
+        mpd::SetLastError("mpd_nn_wgrad: bad arguments");
+        return MPD_ERR_INVALID;
+    }
+    if (B == 0) return MPD_OK;
+    WgradArgs w;
+    w.a = a;
+    w.g = g;
+    w.P = P;
+    w.B = B;
+    w.ksplit = w.kspan = 0;
+    w.part = work;
+    w.colpart = colwork;
+    w.dw = dw;
+    w.db = db;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (k_in == kLiftK && n_out == 64) return LaunchWgrad<kLiftK, 64>(w, work_floats, st);
+    if (k_in == 64 && n_out == 64) return LaunchWgrad<64, 64>(w, work_floats, st);
+    if (k_in == 64 && n_out == 128) return LaunchWgrad<64, 128>(w, work_floats, st);
+    if (k_in == 128 && n_out == 8) return LaunchWgrad<128, 8>(w, work_floats, st);
+    mpd::SetLastError("mpd_nn_wgrad: widths are 6 x 64, 64 x 64, 64 x 128 or 128 x 8");
+    return MPD_ERR_INVALID;
 }
 
 int mpd_nn_lift(const float *x, const float *w, const float *bias, float *z, long long rows,

@@ -80,6 +80,16 @@ def lift(x, w, bias, z):
                             _stream()), lib)
 
 
+def wgrad(a, g, P, B, dw, db, work, colwork):
+    """dw = a^T g and db = column sums of g over B samples of P rows:
+    mpd_nn_wgrad in include/mpd_b200.h."""
+    lib = N.load()
+    N.check(lib.mpd_nn_wgrad(C.c_void_p(a.data_ptr()), C.c_void_p(g.data_ptr()), a.shape[1],
+                             g.shape[1], P, B, C.c_void_p(dw.data_ptr()),
+                             C.c_void_p(db.data_ptr()), C.c_void_p(work.data_ptr()), work.numel(),
+                             C.c_void_p(colwork.data_ptr()), _stream()), lib)
+
+
 def wait_status():
     lib = N.load()
     N.check(lib.mpd_nn_wait_status(_stream()), lib)

@@ -166,7 +166,6 @@ class SpectralOperator:
         self.gh = [torch.zeros(rows, WIDTH, **f32) for _ in range(2)]
         self.gU = torch.zeros(batch, self.Q, WIDTH, **f32)
         self.gV = torch.zeros(batch, self.Q, WIDTH, **f32)
-        self.parts = torch.zeros(batch * max(WIDTH, HIDDEN) * max(WIDTH, HIDDEN), **f32)
         self.partial = torch.zeros(148 * 32, device=dev, dtype=torch.float64)
         self.colwork = torch.zeros(128 * max(WIDTH, HIDDEN), **f32)
         # split-K partial sums of the long-K products (grid sums, weight gradients)
@@ -195,20 +194,9 @@ class SpectralOperator:
     def _chk(self, rc):
         N.check(rc, self.lib)
 
-    def _wgrad(self, a, k_in, gz, n_out, dst):
-        """dst[k_in, n_out] = sum over rows of a[:, :k_in]^T gz, split by sample."""
-        B, P = self.B, self.P
-        parts = self.parts[:B * k_in * n_out]
-        nn.gemm(a, gz, parts, k_in, n_out, P, B, sa=(1, a.stride(0), P * a.stride(0)),
-                sb=(1, gz.stride(0), P * gz.stride(0)), sc=(n_out, 1, k_in * n_out),
-                work=self.work)
-        self._chk(self.lib.mpd_nn_sum_parts(C.c_void_p(parts.data_ptr()), B, k_in * n_out,
-                                            C.c_void_p(dst.data_ptr()), 0, self._s()))
-
-    def _colsum(self, x, dst):
-        self._chk(self.lib.mpd_nn_colsum(C.c_void_p(x.data_ptr()), x.shape[0], x.shape[1],
-                                         C.c_void_p(dst.data_ptr()),
-                                         C.c_void_p(self.colwork.data_ptr()), self._s()))
+    def _wgrad(self, a, gz, weight, bias):
+        """Gradients of a linear layer's weight (a^T gz) and bias (column sums of gz)."""
+        nn.wgrad(a, gz, self.P, self.B, self.g[weight], self.g[bias], self.work, self.colwork)
 
     # --------------------------------------------------------------- forward
     def load_inputs(self, x: np.ndarray):
@@ -247,18 +235,15 @@ class SpectralOperator:
         p, g = self.p, self.g
         rows = B * P
         # projection
-        self._wgrad(self.y1, HIDDEN, self.g_out, N_OUT, g["W_p2"])
-        self._colsum(self.g_out, g["b_p2"])
+        self._wgrad(self.y1, self.g_out, "W_p2", "b_p2")
         # gzp = (g_out W_p2^T) GELU'(zp), gh = gzp W_p1^T
         gzp, gh = self.gzp, self.gh[0]
         nn.layer(self.g_out, p["W_p2"], N_OUT, 1, gzp, rows, 1, n_out=HIDDEN,
                  epilogue=nn.ACT_BWD, z_in=self.zp, w2=p["W_p1"], w2_sn=HIDDEN, w2_sk=1, out2=gh)
-        self._wgrad(self.h[LAYERS], Cw, gzp, HIDDEN, g["W_p1"])
-        self._colsum(gzp, g["b_p1"])
+        self._wgrad(self.h[LAYERS], gzp, "W_p1", "b_p1")
         gz = gh   # the last layer has no activation
         for l in reversed(range(LAYERS)):
-            self._wgrad(self.h[l], Cw, gz, Cw, g[f"W{l}"])
-            self._colsum(gz, g[f"b{l}"])
+            self._wgrad(self.h[l], gz, f"W{l}", f"b{l}")
             # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T
             nn.spectral(gz, self.Gt_img, p[f"R{l}"], Cw, 1, self.gU, self.gV, self.u_image, P, B,
                         work=self.work)
@@ -272,8 +257,7 @@ class SpectralOperator:
                      z_in=self.z[l] if l else None)
             gz = gh
         # lift (the input needs no gradient)
-        self._wgrad(self.x, N_IN, gh, Cw, g["W_in"])
-        self._colsum(gh, g["b_in"])
+        self._wgrad(self.x, gh, "W_in", "b_in")
 
     # ------------------------------------------------------ captured iteration
     def capture(self) -> None:

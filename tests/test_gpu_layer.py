@@ -111,6 +111,29 @@ def test_lift_is_the_separate_launches(pkg, rows):
     nn.wait_status()
 
 
+@pytest.mark.parametrize("k_in,n_out", [(6, 64), (64, 64), (64, 128), (128, 8)])
+@pytest.mark.parametrize("P,B,room", [(1, 1, 1), (63, 2, 64), (257, 3, 64), (1300, 16, 64),
+                                      (4100, 2, 3), (1001, 9, 1)])
+def test_weight_gradients_are_the_separate_launches(pkg, k_in, n_out, P, B, room):
+    import torch
+    nn, lib = pkg.nn, pkg._native.load()
+    a, g = torch.randn(B * P, k_in, device="cuda"), torch.randn(B * P, n_out, device="cuda")
+    mn = k_in * n_out
+    work = torch.empty(room * B * mn, device="cuda")
+    colwork = torch.empty(128 * n_out, device="cuda")
+    parts, dw = torch.empty(B * mn, device="cuda"), torch.empty(k_in, n_out, device="cuda")
+    db = torch.empty(n_out, device="cuda")
+    nn.gemm(a, g, parts, k_in, n_out, P, B, sa=(1, k_in, P * k_in), sb=(1, n_out, P * n_out),
+            sc=(n_out, 1, mn), work=work)
+    assert lib.mpd_nn_sum_parts(_ptr(parts), B, mn, _ptr(dw), 0, nn._stream()) == 0
+    assert lib.mpd_nn_colsum(_ptr(g), B * P, n_out, _ptr(db), _ptr(colwork), nn._stream()) == 0
+    got_w, got_b = torch.full_like(dw, 7.0), torch.full_like(db, 7.0)
+    work.fill_(7.0), colwork.fill_(7.0)
+    nn.wgrad(a, g, P, B, got_w, got_b, work, colwork)
+    assert torch.equal(got_w, dw) and torch.equal(got_b, db)
+    nn.wait_status()
+
+
 def test_refused_operands(pkg):
     import torch
     nn, o = pkg.nn, _operands(8, 1, 0)
