@@ -374,7 +374,11 @@ int mpd_nn_basis_image(const float *src, long long s_row, long long s_k, int row
  * GEMMs it stands for: V[b] = basis h[b] (256 x 64 sums over P points; basis:
  * image of 256 x P with block_k 32), U[b, q] = V[b, q] R[q] with R[q](n, k) at
  * R[q * 4096 + n * r_sn + k * r_sk], and U as the image mpd_nn_layer reads
- * (B * 32 KB).  All operands but R start on 16-byte boundaries. */
+ * (B * 32 KB).  With dR (B <= MPD_NN_MIX_GRAD_MAX_B only) also
+ * dR[q](k, n) = sum_b V_fwd[b, q, k] V[b, q, n], the gradient of R[q] when V is
+ * the gradient of the U that V_fwd gave.  All operands but R and V_fwd start on
+ * 16-byte boundaries. */
+#define MPD_NN_MIX_GRAD_MAX_B 32
 typedef struct mpd_spectral_desc {
     int P, B;
     const float *h;
@@ -385,6 +389,8 @@ typedef struct mpd_spectral_desc {
     void *u_image;
     float *work;           /* optional scratch for split-K partial sums (or NULL) */
     long long work_floats;
+    const float *V_fwd;    /* B x 256 x 64, with dR */
+    float *dR;             /* 256 x 64 x 64 (or NULL) */
 } mpd_spectral_desc;
 
 int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream);

@@ -117,7 +117,8 @@ class SpectralDesc(C.Structure):
     _fields_ = [("P", C.c_int), ("B", C.c_int), ("h", C.c_void_p), ("basis", C.c_void_p),
                 ("R", C.c_void_p), ("r_sn", C.c_longlong), ("r_sk", C.c_longlong),
                 ("V", C.c_void_p), ("U", C.c_void_p), ("u_image", C.c_void_p),
-                ("work", C.c_void_p), ("work_floats", C.c_longlong)]
+                ("work", C.c_void_p), ("work_floats", C.c_longlong), ("V_fwd", C.c_void_p),
+                ("dR", C.c_void_p)]
 
 
 class MpdError(RuntimeError):

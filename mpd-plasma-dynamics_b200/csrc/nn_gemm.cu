@@ -510,7 +510,7 @@ int LaunchWgrad(WgradArgs a, long long work_floats, cudaStream_t st) {
     }
     nn_wgrad_kernel<KA, N><<<a.B * a.ksplit + ((N + 31) / 32) * kWgColSlices, kWgThreads, smem,
                              st>>>(a);
-    nn_wgrad_sum_kernel<<<(KA * N + 31) / 32 + (N + 255) / 256, 256, 0, st>>>(a, KA * N, N);
+    nn_wgrad_sum_kernel<<<(KA * N + 31) / 32 + 1, kWgSumWarps * 32, 0, st>>>(a, KA * N, N);
     return NnLaunched("mpd_nn_wgrad");
 }
 
@@ -582,6 +582,10 @@ int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream) {
         mpd::SetLastError("mpd_nn_spectral: operands must start on 16-byte boundaries");
         return MPD_ERR_INVALID;
     }
+    if (d->dR && (!d->V_fwd || d->B > MPD_NN_MIX_GRAD_MAX_B || !Aligned16(d->dR))) {
+        mpd::SetLastError("mpd_nn_spectral: dR needs V_fwd and at most 32 samples");
+        return MPD_ERR_INVALID;
+    }
     if (d->B == 0) return MPD_OK;
     int ksplit, kspan;
     SplitK(kLyQ, kLyW, d->P, d->B, d->work ? d->work_floats : 0, &ksplit, &kspan);
@@ -603,9 +607,17 @@ int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream) {
     nn_project_kernel<<<d->B * ksplit, kPjThreads, kPjSmem, st>>>(
         static_cast<const unsigned char *>(d->basis), d->h, d->P, d->B, kspan,
         ksplit > 1 ? d->work : d->V);
-    nn_mix_kernel<<<dim3(kLyQ, (d->B + 127) / 128), 128, 0, st>>>(
-        d->work, ksplit, d->B, d->R, d->r_sn, d->r_sk, d->V, d->U,
-        static_cast<__nv_bfloat16 *>(d->u_image));
+    const dim3 grid(kLyQ, (d->B + 127) / 128);
+    if (d->dR)
+        nn_mix_kernel<true><<<grid, 128, 0, st>>>(d->work, ksplit, d->B, d->R, d->r_sn, d->r_sk,
+                                                  d->V, d->U,
+                                                  static_cast<__nv_bfloat16 *>(d->u_image),
+                                                  d->V_fwd, d->dR);
+    else
+        nn_mix_kernel<false><<<grid, 128, 0, st>>>(d->work, ksplit, d->B, d->R, d->r_sn, d->r_sk,
+                                                   d->V, d->U,
+                                                   static_cast<__nv_bfloat16 *>(d->u_image),
+                                                   nullptr, nullptr);
     return NnLaunched("mpd_nn_spectral");
 }
 

@@ -188,10 +188,20 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
 // (16 KB of R, ksplit x 256 B a sample), so what it costs is one trip to memory
 // for both, taken together, the product and the stores.  U also leaves as the
 // image the layer kernel copies (element (q, n) of sample b: 16-byte unit q / 8).
+// GRAD (one CTA of samples, at most 32: K of one block of the general kernel) adds
+// the gradient of R[q] = V_fwd[., q]^T V[., q], whose second operand is at hand:
+// as a launch of its own it took 13.6 us, here it is within the trip.
+constexpr int kMixGradK = MPD_NN_MIX_GRAD_MAX_B;
+constexpr uint32_t kMixTmem = 128;
+
+template <bool GRAD>
 __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int ksplit, int B,
                                                      const float *R, long long r_sn,
                                                      long long r_sk, float *V, float *U,
-                                                     __nv_bfloat16 *u_img) {
+                                                     __nv_bfloat16 *u_img, const float *V_fwd,
+                                                     float *dR) {
+    __shared__ __align__(1024) unsigned char sA2[GRAD ? 128 * kMixGradK * 2 : 16];
+    __shared__ __align__(1024) unsigned char sB2[GRAD ? kLyW * kMixGradK * 2 : 16];
     __shared__ __align__(1024) unsigned char sA[128 * kLyW * 2];
     __shared__ __align__(1024) unsigned char sB[kLyW * kLyW * 2];
     __shared__ __align__(8) uint64_t bar;
@@ -201,7 +211,7 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_addr(&tmem_slot)),
-                     "r"(kTmemCols)
+                     "r"(kMixTmem)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -219,6 +229,23 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[j][e] = __ldg(Rq + n * r_sn + (8 * c + e) * r_sk);
     }
+    // the first operand of the gradient: 8 samples of one row k of V_fwd's transpose
+    float vf[2][8];
+    if (GRAD) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int u = threadIdx.x + 128 * j, k = u % kLyW, c = u / kLyW;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                vf[j][e] = 8 * c + e < B
+                               ? __ldg(V_fwd + ((long long)(8 * c + e) * kLyQ + q) * kLyW + k)
+                               : 0.0f;
+        }
+        // samples past B are zero in both operands
+        for (int u = threadIdx.x; u < (int)sizeof(sB2) / 16; u += 128)
+            reinterpret_cast<uint4 *>(sB2)[u] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+    }
     const long long plane = (long long)B * kLyQ * kLyW;
     for (int u = threadIdx.x; u < rows * 8; u += 128) {
         const int row = u >> 3, c = u & 7;
@@ -227,7 +254,7 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
         if (ksplit > 1) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) f[e] = 0.0f;
-#pragma unroll 4
+#pragma unroll 8
             for (int k = 0; k < ksplit; ++k) {
                 const float4 x = __ldg(reinterpret_cast<const float4 *>(part + k * plane + at));
                 const float4 y = __ldg(reinterpret_cast<const float4 *>(part + k * plane + at) + 1);
@@ -245,6 +272,21 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
         *reinterpret_cast<uint4 *>(sA + (c * 16 + (row >> 3)) * 128 + (row & 7) * 16) =
             make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
                        pack_bf16(f[6], f[7]));
+        if (GRAD) {   // element (n, sample)
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                *reinterpret_cast<__nv_bfloat16 *>(sB2 + ((row >> 3) * 8 + c) * 128 + e * 16 +
+                                                   (row & 7) * 2) = __float2bfloat16_rn(f[e]);
+        }
+    }
+    if (GRAD) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int u = threadIdx.x + 128 * j, k = u % kLyW, c = u / kLyW;
+            *reinterpret_cast<uint4 *>(sA2 + (c * 16 + (k >> 3)) * 128 + (k & 7) * 16) =
+                make_uint4(pack_bf16(vf[j][0], vf[j][1]), pack_bf16(vf[j][2], vf[j][3]),
+                           pack_bf16(vf[j][4], vf[j][5]), pack_bf16(vf[j][6], vf[j][7]));
+        }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -264,6 +306,12 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
         for (int k = 0; k < kLyW / 16; ++k)
             mma_bf16(tmem, smem_desc(smem_addr(sA) + k * 2 * 2048, 2048, 128),
                      smem_desc(smem_addr(sB) + k * 2 * 1024, 1024, 128), k > 0 ? 1u : 0u);
+        if (GRAD) {
+#pragma unroll
+            for (int k = 0; k < kMixGradK / 16; ++k)
+                mma_bf16(tmem + 64, smem_desc(smem_addr(sA2) + k * 2 * 2048, 2048, 128),
+                         smem_desc(smem_addr(sB2) + k * 2 * 1024, 1024, 128), k > 0 ? 1u : 0u);
+        }
         mma_commit(smem_addr(&bar));
     }
     __syncwarp();
@@ -295,6 +343,25 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
                 }
             }
         }
+        if (GRAD && warp < 2) {   // rows k of dR[q]
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int hf = p & 1, col = (p >> 1) * 32;
+                float v[16];
+                tmem_ld_16x32(tmem + ((uint32_t)(warp * 32 + hf * 16) << 16) +
+                                  (uint32_t)(64 + col),
+                              v);
+                tmem_ld_wait(v);
+                float *o = dR + (long long)q * (kLyW * kLyW) +
+                           (warp * 32 + hf * 16 + (lane >> 2)) * kLyW + col + 2 * (lane & 3);
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        *reinterpret_cast<float2 *>(o + t * 8 * kLyW + 8 * j) =
+                            make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
+            }
+        }
     } else if (threadIdx.x == 0) {
         atomicExch(&g_gemm_wait_fail, 1);
     }
@@ -303,7 +370,7 @@ __global__ void __launch_bounds__(128) nn_mix_kernel(const float *part, int kspl
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(kTmemCols)
+                     "r"(kMixTmem)
                      : "memory");
     }
 }

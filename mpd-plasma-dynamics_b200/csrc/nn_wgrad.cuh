@@ -212,18 +212,20 @@ __global__ void __launch_bounds__(kWgThreads, 2) nn_wgrad_kernel(const WgradArgs
     }
 }
 
-// 32 elements of dW a block: a warp takes samples warp, warp + 8, ... and adds
-// their splits (all loads in flight together); the first warp adds the samples.
+// 32 elements of dW a block: a warp takes samples warp, warp + 16, ... and adds
+// their splits (16 loads in flight at a time); the first warp adds the samples.
 // The blocks after them finish db, a column a thread.
-__global__ void __launch_bounds__(256) nn_wgrad_sum_kernel(const WgradArgs a, int n_dw, int N) {
-    __shared__ float red[8][32];
+constexpr int kWgSumWarps = 16;
+__global__ void __launch_bounds__(kWgSumWarps * 32) nn_wgrad_sum_kernel(const WgradArgs a,
+                                                                        int n_dw, int N) {
+    __shared__ float red[kWgSumWarps][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int dw_blocks = (n_dw + 31) / 32;
     if (blockIdx.x >= dw_blocks) {
-        const int c = (blockIdx.x - dw_blocks) * 256 + threadIdx.x;
+        const int c = (blockIdx.x - dw_blocks) * (kWgSumWarps * 32) + threadIdx.x;
         if (c >= N) return;
         float t = 0.0f;
-#pragma unroll 16
+#pragma unroll 32
         for (int k = 0; k < kWgColSlices; ++k) t += a.colpart[k * N + c];
         a.db[c] = t;
         return;
@@ -231,18 +233,18 @@ __global__ void __launch_bounds__(256) nn_wgrad_sum_kernel(const WgradArgs a, in
     const int e = blockIdx.x * 32 + lane;
     const long long plane = (long long)a.B * n_dw;
     float sum = 0.0f;
-    for (int b0 = 0; b0 < a.B; b0 += 8) {
+    for (int b0 = 0; b0 < a.B; b0 += kWgSumWarps) {
         const int b = b0 + warp;
         float s = 0.0f;
         if (b < a.B && e < n_dw) {
             const float *p = a.part + (long long)b * n_dw + e;
-#pragma unroll 8
+#pragma unroll 16
             for (int k = 0; k < a.ksplit; ++k) s += __ldg(p + k * plane);
         }
         red[warp][lane] = s;
         __syncthreads();
         if (warp == 0)
-            for (int k = 0; k < 8 && b0 + k < a.B; ++k) sum += red[k][lane];
+            for (int k = 0; k < kWgSumWarps && b0 + k < a.B; ++k) sum += red[k][lane];
         __syncthreads();
     }
     if (warp == 0 && e < n_dw) a.dw[e] = sum;

@@ -33,6 +33,7 @@ def gemm(A, B, Cout, M, N_, K, batch=1, sa=None, sb=None, sc=None, alpha=1.0, be
 
 
 FORWARD, ACT_BWD, PLAIN = 0, 1, 2   # epilogues of layer()
+MIX_GRAD_MAX_B = 32                 # samples up to which spectral() also makes dR
 
 
 def basis_image(A, rows, K, s_row, s_k, block_k=256):
@@ -47,14 +48,18 @@ def basis_image(A, rows, K, s_row, s_k, block_k=256):
     return img
 
 
-def spectral(h, basis, R, r_sn, r_sk, V, U, u_image, P, B, work=None):
-    """V[b] = basis h[b], U[b, q] = V[b, q] R[q], u_image = U as layer() reads it:
-    mpd_nn_spectral in include/mpd_b200.h."""
+def spectral(h, basis, R, r_sn, r_sk, V, U, u_image, P, B, work=None, V_fwd=None,
+             dR=None):
+    """V[b] = basis h[b], U[b, q] = V[b, q] R[q], u_image = U as layer() reads it,
+    dR[q] = sum over b of V_fwd[b, q]^T V[b, q]: mpd_nn_spectral in
+    include/mpd_b200.h."""
     lib = N.load()
     d = N.SpectralDesc(P, B, h.data_ptr(), basis.data_ptr(), R.data_ptr(), r_sn, r_sk,
                        V.data_ptr(), U.data_ptr(), u_image.data_ptr(),
                        work.data_ptr() if work is not None else None,
-                       work.numel() if work is not None else 0)
+                       work.numel() if work is not None else 0,
+                       V_fwd.data_ptr() if V_fwd is not None else None,
+                       dR.data_ptr() if dR is not None else None)
     N.check(lib.mpd_nn_spectral(C.byref(d), _stream()), lib)
 
 

@@ -244,12 +244,13 @@ class SpectralOperator:
         gz = gh   # the last layer has no activation
         for l in reversed(range(LAYERS)):
             self._wgrad(self.h[l], gz, f"W{l}", f"b{l}")
-            # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T
+            # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T, dR[q] = sum_b V[b, q]^T gU[b, q]
+            fused = B <= nn.MIX_GRAD_MAX_B
             nn.spectral(gz, self.Gt_img, p[f"R{l}"], Cw, 1, self.gU, self.gV, self.u_image, P, B,
-                        work=self.work)
-            # dR[q] = sum_b V[b, q]^T gU[b, q]
-            nn.gemm(self.V[l], self.gU, g[f"R{l}"], Cw, Cw, B, Q, sa=(1, Q * Cw, Cw),
-                    sb=(1, Q * Cw, Cw), sc=(Cw, 1, Cw * Cw))
+                        work=self.work, V_fwd=self.V[l], dR=g[f"R{l}"] if fused else None)
+            if not fused:
+                nn.gemm(self.V[l], self.gU, g[f"R{l}"], Cw, Cw, B, Q, sa=(1, Q * Cw, Cw),
+                        sb=(1, Q * Cw, Cw), sc=(Cw, 1, Cw * Cw))
             # gh = gz W^T + F^T gV, and through the activation of the layer below
             gh = self.gh[1] if gz is self.gh[0] else self.gh[0]
             nn.layer(gz, p[f"W{l}"], Cw, 1, gh, P, B, basis=self.Ft_img,

@@ -147,7 +147,7 @@ def test_refused_operands(pkg):
 
 @pytest.mark.parametrize("P,B,room", [(1, 1, 16), (31, 2, 16), (33, 3, 16), (255, 2, 16),
                                       (300, 2, 0), (1001, 16, 16), (4100, 1, 16), (70, 130, 2),
-                                      (40000, 2, 16)])
+                                      (40000, 2, 16), (90, 17, 16), (90, 32, 16)])
 def test_spectral_half_is_the_separate_launches(pkg, P, B, room):
     """Both directions (R and R^T), split and unsplit K, more samples than a tile."""
     import torch
@@ -169,4 +169,12 @@ def test_spectral_half_is_the_separate_launches(pkg, P, B, room):
         nn.spectral(o["h"], img, R, r_sn, r_sk, gV, gU, image, P, B, work=work)
         assert torch.equal(gV, V) and torch.equal(gU, U)
         assert torch.equal(image, _u_image(U).view(-1))
+        if B <= nn.MIX_GRAD_MAX_B:
+            Vf = torch.randn(B, 256, 64, device="cuda")
+            dR, gR = torch.empty_like(R), torch.full_like(R, 7.0)
+            nn.gemm(Vf, V, dR, 64, 64, B, 256, sa=(1, 256 * 64, 64), sb=(1, 256 * 64, 64),
+                    sc=(64, 1, 4096))
+            nn.spectral(o["h"], img, R, r_sn, r_sk, gV, gU, image, P, B, work=work, V_fwd=Vf,
+                        dR=gR)
+            assert torch.equal(gR, dR) and torch.equal(gV, V) and torch.equal(gU, U)
     nn.wait_status()
