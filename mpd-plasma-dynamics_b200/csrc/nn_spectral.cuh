@@ -10,25 +10,25 @@
 // general kernel: once per tile, with the basis rounded again per sample, and
 // 320 CTAs in two waves at two per SM).  The basis is an image of the tensor
 // core's layout in blocks of 32 points (basis_image_kernel), so a stage of the
-// four-stage ring is two bulk copies (16 KB of basis, 8 KB of h); four warps
-// transpose and round h, one thread issues the products.  104 KB of shared
-// memory: two CTAs per SM.  The split of K, the order of the products in an
+// four-stage ring is two bulk copies (16 KB of basis, 8 KB of h); two sets of
+// four warps transpose and round h, one thread issues the products.  112 KB of
+// shared memory: two CTAs per SM.  The split of K, the order of the products in an
 // accumulator and the order of the partial sums are the general kernel's, so
 // the values are too.  Both kernels together, measured against the general one
-// (B200): 450 -> 112 us at 16 samples of 64400 points (the copies: 264 MB of h
-// from memory and 530 MB of the basis from L2), 53.5 -> 21.5 us at 16 of 4100
-// and 146 -> 60 us at 1 of 64400 (one trip through the ring per CTA and a
-// quarter of the SMs busy: bound by latency).
+// (B200): 455 -> 104 us at 16 samples of 64400 points (the copies: 264 MB of h
+// from memory and 530 MB of the basis from L2; with one set of converting warps
+// 113), 53 -> 21 us at 16 of 4100 and 146 -> 60 us at 1 of 64400 (16 CTAs, each
+// waiting for its ring: bound by latency).
 #pragma once
 
 namespace {
 
 constexpr int kPjK = 32, kPjStages = 4;
-constexpr int kPjThreads = 6 * 32;
+constexpr int kPjCvtWarps = 8, kPjThreads = (kPjCvtWarps + 2) * 32;
 constexpr int kPjFBytes = 2 * 128 * kPjK * 2;    // 16 KB: both tiles of a block
 constexpr int kPjHBytes = kPjK * kLyW * 4;       // 8 KB
 constexpr int kPjHbBytes = kPjK * kLyW * 2;      // 4 KB
-constexpr int kPjSmem = kPjStages * (kPjFBytes + kPjHBytes) + 2 * kPjHbBytes;
+constexpr int kPjSmem = kPjStages * (kPjFBytes + kPjHBytes) + kPjStages * kPjHbBytes;
 constexpr uint32_t kPjTmem = 128;
 
 // out: ksplit == 1 ? V (B x 256 x 64) : the partial sums (ksplit x B x 256 x 64)
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
                                                                 const float *h, int P, int B,
                                                                 int kspan, float *out) {
     extern __shared__ __align__(1024) unsigned char gemm_smem[];
-    __shared__ __align__(8) uint64_t full[kPjStages], done[kPjStages], hb_full[2];
+    __shared__ __align__(8) uint64_t full[kPjStages], done[kPjStages], hb_full[kPjStages];
     __shared__ uint32_t tmem_slot;
     unsigned char *sF = gemm_smem, *sH = sF + kPjStages * kPjFBytes,
                   *sHb = sH + kPjStages * kPjHBytes;
@@ -56,8 +56,8 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
         for (int i = 0; i < kPjStages; ++i) {
             mbar_init(smem_addr(&full[i]), 1);
             mbar_init(smem_addr(&done[i]), 1);
+            mbar_init(smem_addr(&hb_full[i]), 4);
         }
-        for (int i = 0; i < 2; ++i) mbar_init(smem_addr(&hb_full[i]), 4);
         mbar_init_fence();
     }
     tc_fence_before();
@@ -66,19 +66,19 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
     const uint32_t tmem = tmem_slot;
     bool ok = true;
 
-    if (warp < 4) {
-        // ---- h (points x columns) to its transpose in BF16, zero past K's end
-        const int n = threadIdx.x & 63, cb = threadIdx.x >> 6;
-        for (int i = 0; i < n_chunks; ++i) {
+    if (warp < kPjCvtWarps) {
+        // ---- h (points x columns) to its transpose in BF16, zero past K's end;
+        // four warps take the even chunks, four the odd ones.  The copies of
+        // chunk i were issued after the products of chunk i - kPjStages, so its
+        // buffer is free as well.
+        const int n = threadIdx.x & 63, cb = (threadIdx.x >> 6) & 1;
+        for (int i = warp >> 2; i < n_chunks; i += 2) {
             const int s = i % kPjStages;
             ok = mbar_wait_bounded(smem_addr(&full[s]), (i / kPjStages) & 1);
-            if (ok && i >= 2)   // the products of chunk i - 2 read this buffer
-                ok = mbar_wait_bounded(smem_addr(&done[(i - 2) % kPjStages]),
-                                       ((i - 2) / kPjStages) & 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const float *src = reinterpret_cast<const float *>(sH + s * kPjHBytes);
-            unsigned char *dst = sHb + (i & 1) * kPjHbBytes;
+            unsigned char *dst = sHb + s * kPjHbBytes;
             const int left = k_end - k_begin - i * kPjK;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -94,35 +94,32 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_addr(&hb_full[i & 1]));
+            if (lane == 0) mbar_arrive(smem_addr(&hb_full[s]));
         }
         if (ok) ok = mbar_wait_bounded(smem_addr(&done[(n_chunks - 1) % kPjStages]),
                                        ((n_chunks - 1) / kPjStages) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             tc_fence_after();
-            float *o = out + ((long long)blockIdx.x * kLyQ + warp * 32 + (lane >> 2)) * kLyW +
+            const int mt = warp >> 2, r0 = (warp & 3) * 32;   // a tile per four warps
+            float *o = out + ((long long)blockIdx.x * kLyQ + mt * 128 + r0 + (lane >> 2)) * kLyW +
                        2 * (lane & 3);
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+            for (int q = 0; q < 4; ++q) {   // 16 rows x 32 columns each
+                const int hf = q & 1, col = (q >> 1) * 32;
+                float v[16];
+                tmem_ld_16x32(tmem + ((uint32_t)(r0 + hf * 16) << 16) + (uint32_t)(mt * 64 + col),
+                              v);
+                tmem_ld_wait(v);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {   // 16 rows x 32 columns each
-                    const int hf = q & 1, col = (q >> 1) * 32;
-                    float v[16];
-                    tmem_ld_16x32(tmem + ((uint32_t)(warp * 32 + hf * 16) << 16) +
-                                      (uint32_t)(mt * 64 + col),
-                                  v);
-                    tmem_ld_wait(v);
+                for (int t = 0; t < 2; ++t)
 #pragma unroll
-                    for (int t = 0; t < 2; ++t)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            *reinterpret_cast<float2 *>(
-                                o + (mt * 128 + hf * 16 + t * 8) * kLyW + col + 8 * j) =
-                                make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
-                }
+                    for (int j = 0; j < 4; ++j)
+                        *reinterpret_cast<float2 *>(o + (hf * 16 + t * 8) * kLyW + col + 8 * j) =
+                            make_float2(v[4 * j + 2 * t] + 0.0f, v[4 * j + 2 * t + 1] + 0.0f);
+            }
         }
-    } else if (warp == 4) {
+    } else if (warp == kPjCvtWarps) {
         // ---- copies
         if (lane == 0) {
             int n = 0;
@@ -149,7 +146,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             for (; n < n_chunks; ++n) {
                 const int s = n % kPjStages;
                 ok = mbar_wait_bounded(smem_addr(&full[s]), (n / kPjStages) & 1) &&
-                     mbar_wait_bounded(smem_addr(&hb_full[n & 1]), (n >> 1) & 1);
+                     mbar_wait_bounded(smem_addr(&hb_full[s]), (n / kPjStages) & 1);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
@@ -160,7 +157,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
                             smem_addr(sF + s * kPjFBytes) + mt * (kPjFBytes / 2) + k * 2 * 2048,
                             2048, 128);
                         const uint64_t bd = smem_desc(
-                            smem_addr(sHb + (n & 1) * kPjHbBytes) + k * 2 * 1024, 1024, 128);
+                            smem_addr(sHb + s * kPjHbBytes) + k * 2 * 1024, 1024, 128);
                         mma_bf16(tmem + mt * 64, ad, bd, (n > 0 || k > 0) ? 1u : 0u);
                     }
                 mma_commit(smem_addr(&done[s]));
