@@ -80,6 +80,7 @@ def layer(h, w, w_sn, w_sk, out0, P, B, n_out=64, epilogue=FORWARD, basis=None, 
 def lift(x, w, bias, z):
     """z = x W + bias (rows x 6 to rows x 64), rounded as gemm() rounds."""
     lib = N.load()
+    x = x.contiguous()
     N.check(lib.mpd_nn_lift(C.c_void_p(x.data_ptr()), C.c_void_p(w.data_ptr()),
                             C.c_void_p(bias.data_ptr()), C.c_void_p(z.data_ptr()), x.shape[0],
                             _stream()), lib)
@@ -89,6 +90,7 @@ def wgrad(a, g, P, B, dw, db, work, colwork):
     """dw = a^T g and db = column sums of g over B samples of P rows:
     mpd_nn_wgrad in include/mpd_b200.h."""
     lib = N.load()
+    a, g = a.contiguous(), g.contiguous()
     N.check(lib.mpd_nn_wgrad(C.c_void_p(a.data_ptr()), C.c_void_p(g.data_ptr()), a.shape[1],
                              g.shape[1], P, B, C.c_void_p(dw.data_ptr()),
                              C.c_void_p(db.data_ptr()), C.c_void_p(work.data_ptr()), work.numel(),
