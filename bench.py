@@ -723,7 +723,7 @@ def run_batch(args, rank=0, world=1, local_rank=0):
 
 def run_profile(args):
     """Lean run for profilers: the exact first step, --warmup graph steps, then
-    --steps eagerly launched steps (interior + boundary kernel each)."""
+    --steps eagerly launched steps."""
     import __graft_entry__
     pkg = __graft_entry__.load_package()
     case = _case()
