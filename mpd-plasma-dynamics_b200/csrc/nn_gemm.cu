@@ -514,6 +514,25 @@ int LaunchWgrad(WgradArgs a, long long work_floats, cudaStream_t st) {
     return NnLaunched("mpd_nn_wgrad");
 }
 
+template <int TILES>
+int LaunchProject(const mpd_spectral_desc &d, int ksplit, int kspan, cudaStream_t st) {
+    static bool attr_set = false;  // per process; the attribute is per function
+    if (!attr_set) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(nn_project_kernel<TILES>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmem<TILES>);
+        if (e != cudaSuccess) {
+            mpd::SetLastError(std::string("mpd_nn_spectral: ") + cudaGetErrorString(e));
+            return MPD_ERR_CUDA;
+        }
+        attr_set = true;
+    }
+    nn_project_kernel<TILES><<<d.B * ksplit * (2 / TILES), kPjThreads, kPjSmem<TILES>, st>>>(
+        static_cast<const unsigned char *>(d.basis), d.h, d.P, d.B, kspan,
+        ksplit > 1 ? d.work : d.V);
+    return MPD_OK;
+}
+
 bool Aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -593,20 +612,17 @@ int mpd_nn_spectral(const mpd_spectral_desc *d, void *stream) {
         mpd::SetLastError("mpd_nn_spectral: batch too large for one launch");
         return MPD_ERR_INVALID;
     }
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(
-            nn_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmem);
-        if (e != cudaSuccess) {
-            mpd::SetLastError(std::string("mpd_nn_spectral: ") + cudaGetErrorString(e));
-            return MPD_ERR_CUDA;
-        }
-        attr_set = true;
-    }
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    nn_project_kernel<<<d->B * ksplit, kPjThreads, kPjSmem, st>>>(
-        static_cast<const unsigned char *>(d->basis), d->h, d->P, d->B, kspan,
-        ksplit > 1 ? d->work : d->V);
+    // Few CTAs are bound by what one SM can take in (24 KB of basis and h a chunk
+    // at 63 GB/s), so while two CTAs per (sample, split) still have an SM each,
+    // each takes one row tile (16 KB a chunk): projection and mix of 1 sample of
+    // 64400 points 58 -> 51 us, 4 of them 63.6 -> 54, 4 of 4100 18.9 -> 17.2 (a
+    // deeper ring alone gave nothing: 59.1).  Beyond that both tiles share one
+    // fetch and one rounding of h, two CTAs to an SM: 160 CTAs at 16 samples are
+    // one wave, 320 were two (438 us of the general kernel).
+    const int rc = 2LL * d->B * ksplit <= 148 ? LaunchProject<1>(*d, ksplit, kspan, st)
+                                              : LaunchProject<2>(*d, ksplit, kspan, st);
+    if (rc != MPD_OK) return rc;
     const dim3 grid(kLyQ, (d->B + 127) / 128);
     if (d->dR)
         nn_mix_kernel<true><<<grid, 128, 0, st>>>(d->work, ksplit, d->B, d->R, d->r_sn, d->r_sk,

@@ -6,7 +6,8 @@
 //                      sums over the split of K before it
 //
 // nn_project_kernel: one CTA per (sample, split of K), both 128-row tiles of the
-// basis as two TMEM accumulators, so a row of h is fetched and rounded once (the
+// basis as two TMEM accumulators (a CTA per tile where that many have an SM
+// each), so a row of h is fetched and rounded once (the
 // general kernel: once per tile, with the basis rounded again per sample, and
 // 320 CTAs in two waves at two per SM).  The basis is an image of the tensor
 // core's layout in blocks of 32 points (basis_image_kernel), so a stage of the
@@ -17,31 +18,38 @@
 // the values are too.  Both kernels together, measured against the general one
 // (B200): 455 -> 104 us at 16 samples of 64400 points (the copies: 264 MB of h
 // from memory and 530 MB of the basis from L2; with one set of converting warps
-// 113), 53 -> 21 us at 16 of 4100 and 146 -> 60 us at 1 of 64400 (16 CTAs, each
-// waiting for its ring: bound by latency).
+// 113), 53 -> 21 us at 16 of 4100 and 146 -> 51 us at 1 of 64400 (32 CTAs of one
+// tile each, bound by what one SM takes in).
 #pragma once
 
 namespace {
 
-constexpr int kPjK = 32, kPjStages = 4;
+constexpr int kPjK = 32;
 constexpr int kPjCvtWarps = 8, kPjThreads = (kPjCvtWarps + 2) * 32;
-constexpr int kPjFBytes = 2 * 128 * kPjK * 2;    // 16 KB: both tiles of a block
+constexpr int kPjFTile = 128 * kPjK * 2;         // 8 KB: a row tile of a block
 constexpr int kPjHBytes = kPjK * kLyW * 4;       // 8 KB
 constexpr int kPjHbBytes = kPjK * kLyW * 2;      // 4 KB
-constexpr int kPjSmem = kPjStages * (kPjFBytes + kPjHBytes) + kPjStages * kPjHbBytes;
+// TILES (row tiles of the basis per CTA): 2 with 4 stages, or 1 with 8.
+template <int TILES>
+constexpr int kPjStages = 8 / TILES;
+template <int TILES>
+constexpr int kPjSmem = kPjStages<TILES> * (TILES * kPjFTile + kPjHBytes + kPjHbBytes);
 constexpr uint32_t kPjTmem = 128;
 
 // out: ksplit == 1 ? V (B x 256 x 64) : the partial sums (ksplit x B x 256 x 64)
+template <int TILES>
 __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned char *f_img,
                                                                 const float *h, int P, int B,
                                                                 int kspan, float *out) {
+    constexpr int STAGES = kPjStages<TILES>, kPjFBytes = TILES * kPjFTile;
     extern __shared__ __align__(1024) unsigned char gemm_smem[];
-    __shared__ __align__(8) uint64_t full[kPjStages], done[kPjStages], hb_full[kPjStages];
+    __shared__ __align__(8) uint64_t full[STAGES], done[STAGES], hb_full[STAGES];
     __shared__ uint32_t tmem_slot;
-    unsigned char *sF = gemm_smem, *sH = sF + kPjStages * kPjFBytes,
-                  *sHb = sH + kPjStages * kPjHBytes;
+    unsigned char *sF = gemm_smem, *sH = sF + STAGES * kPjFBytes,
+                  *sHb = sH + STAGES * kPjHBytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x % B, split = blockIdx.x / B;
+    const int part = blockIdx.x / (2 / TILES), tile0 = blockIdx.x % (2 / TILES);
+    const int b = part % B, split = part / B;
     const int k_begin = split * kspan, k_end = min(P, k_begin + kspan);
     const int n_chunks = (k_end - k_begin + kPjK - 1) / kPjK;
 
@@ -53,7 +61,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kPjStages; ++i) {
+        for (int i = 0; i < STAGES; ++i) {
             mbar_init(smem_addr(&full[i]), 1);
             mbar_init(smem_addr(&done[i]), 1);
             mbar_init(smem_addr(&hb_full[i]), 4);
@@ -69,12 +77,12 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
     if (warp < kPjCvtWarps) {
         // ---- h (points x columns) to its transpose in BF16, zero past K's end;
         // four warps take the even chunks, four the odd ones.  The copies of
-        // chunk i were issued after the products of chunk i - kPjStages, so its
+        // chunk i were issued after the products of chunk i - STAGES, so its
         // buffer is free as well.
         const int n = threadIdx.x & 63, cb = (threadIdx.x >> 6) & 1;
         for (int i = warp >> 2; i < n_chunks; i += 2) {
-            const int s = i % kPjStages;
-            ok = mbar_wait_bounded(smem_addr(&full[s]), (i / kPjStages) & 1);
+            const int s = i % STAGES;
+            ok = mbar_wait_bounded(smem_addr(&full[s]), (i / STAGES) & 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const float *src = reinterpret_cast<const float *>(sH + s * kPjHBytes);
@@ -96,13 +104,13 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&hb_full[s]));
         }
-        if (ok) ok = mbar_wait_bounded(smem_addr(&done[(n_chunks - 1) % kPjStages]),
-                                       ((n_chunks - 1) / kPjStages) & 1);
+        if (ok) ok = mbar_wait_bounded(smem_addr(&done[(n_chunks - 1) % STAGES]),
+                                       ((n_chunks - 1) / STAGES) & 1);
         ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
+        if (ok && (warp >> 2) < TILES) {
             tc_fence_after();
             const int mt = warp >> 2, r0 = (warp & 3) * 32;   // a tile per four warps
-            float *o = out + ((long long)blockIdx.x * kLyQ + mt * 128 + r0 + (lane >> 2)) * kLyW +
+            float *o = out + ((long long)part * kLyQ + (tile0 + mt) * 128 + r0 + (lane >> 2)) * kLyW +
                        2 * (lane & 3);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {   // 16 rows x 32 columns each
@@ -124,37 +132,38 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
         if (lane == 0) {
             int n = 0;
             for (; n < n_chunks; ++n) {
-                const int s = n % kPjStages, k0 = k_begin + n * kPjK;
-                if (n >= kPjStages)
-                    ok = mbar_wait_bounded(smem_addr(&done[s]), (n / kPjStages - 1) & 1);
+                const int s = n % STAGES, k0 = k_begin + n * kPjK;
+                if (n >= STAGES)
+                    ok = mbar_wait_bounded(smem_addr(&done[s]), (n / STAGES - 1) & 1);
                 if (!ok) break;
                 const uint32_t hbytes = (uint32_t)min(kPjK, k_end - k0) * (kLyW * 4);
                 mbar_expect_tx(smem_addr(&full[s]), kPjFBytes + hbytes);
-                bulk_load(smem_addr(sF + s * kPjFBytes), f_img + (size_t)(k0 / kPjK) * kPjFBytes,
-                          kPjFBytes, smem_addr(&full[s]));
+                bulk_load(smem_addr(sF + s * kPjFBytes),
+                          f_img + ((size_t)(k0 / kPjK) * 2 + tile0) * kPjFTile, kPjFBytes,
+                          smem_addr(&full[s]));
                 bulk_load(smem_addr(sH + s * kPjHBytes), h + ((long long)b * P + k0) * kLyW,
                           hbytes, smem_addr(&full[s]));
             }
             // no copy may still land after the CTA exits
-            for (int k = max(0, n - kPjStages); k < n; ++k)
-                ok = mbar_wait_bounded(smem_addr(&full[k % kPjStages]), (k / kPjStages) & 1) && ok;
+            for (int k = max(0, n - STAGES); k < n; ++k)
+                ok = mbar_wait_bounded(smem_addr(&full[k % STAGES]), (k / STAGES) & 1) && ok;
         }
     } else {
         // ---- products
         if (lane == 0) {
             int n = 0;
             for (; n < n_chunks; ++n) {
-                const int s = n % kPjStages;
-                ok = mbar_wait_bounded(smem_addr(&full[s]), (n / kPjStages) & 1) &&
-                     mbar_wait_bounded(smem_addr(&hb_full[s]), (n / kPjStages) & 1);
+                const int s = n % STAGES;
+                ok = mbar_wait_bounded(smem_addr(&full[s]), (n / STAGES) & 1) &&
+                     mbar_wait_bounded(smem_addr(&hb_full[s]), (n / STAGES) & 1);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
-                for (int mt = 0; mt < 2; ++mt)
+                for (int mt = 0; mt < TILES; ++mt)
 #pragma unroll
                     for (int k = 0; k < kPjK / 16; ++k) {
                         const uint64_t ad = smem_desc(
-                            smem_addr(sF + s * kPjFBytes) + mt * (kPjFBytes / 2) + k * 2 * 2048,
+                            smem_addr(sF + s * kPjFBytes) + mt * kPjFTile + k * 2 * 2048,
                             2048, 128);
                         const uint64_t bd = smem_desc(
                             smem_addr(sHb + s * kPjHbBytes) + k * 2 * 1024, 1024, 128);
@@ -164,8 +173,8 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             }
             // TMEM and shared memory are given back only after every product
             if (n)
-                ok = mbar_wait_bounded(smem_addr(&done[(n - 1) % kPjStages]),
-                                       ((n - 1) / kPjStages) & 1) && ok;
+                ok = mbar_wait_bounded(smem_addr(&done[(n - 1) % STAGES]),
+                                       ((n - 1) / STAGES) & 1) && ok;
         }
     }
     if (!ok) atomicExch(&g_gemm_wait_fail, 1);

@@ -147,7 +147,8 @@ def test_refused_operands(pkg):
 
 @pytest.mark.parametrize("P,B,room", [(1, 1, 16), (31, 2, 16), (33, 3, 16), (255, 2, 16),
                                       (300, 2, 0), (1001, 16, 16), (4100, 1, 16), (70, 130, 2),
-                                      (40000, 2, 16), (90, 17, 16), (90, 32, 16)])
+                                      (40000, 2, 16), (90, 17, 16), (90, 32, 16), (4100, 16, 16),
+                                      (500, 150, 1)])
 def test_spectral_half_is_the_separate_launches(pkg, P, B, room):
     """Both directions (R and R^T), split and unsplit K, more samples than a tile."""
     import torch
