@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
                                                                 int kspan, float *out) {
     constexpr int STAGES = kPjStages<TILES>, kPjFBytes = TILES * kPjFTile;
     extern __shared__ __align__(1024) unsigned char gemm_smem[];
-    __shared__ __align__(8) uint64_t full[STAGES], done[STAGES], hb_full[STAGES];
+    __shared__ __align__(8) uint64_t full[STAGES], done[STAGES], hb_full[STAGES], all_done;
     __shared__ uint32_t tmem_slot;
     unsigned char *sF = gemm_smem, *sH = sF + STAGES * kPjFBytes,
                   *sHb = sH + STAGES * kPjHBytes;
@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             mbar_init(smem_addr(&done[i]), 1);
             mbar_init(smem_addr(&hb_full[i]), 4);
         }
+        mbar_init(smem_addr(&all_done), 1);
         mbar_init_fence();
     }
     tc_fence_before();
@@ -104,8 +105,11 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&hb_full[s]));
         }
-        if (ok) ok = mbar_wait_bounded(smem_addr(&done[(n_chunks - 1) % STAGES]),
-                                       ((n_chunks - 1) / STAGES) & 1);
+        // A barrier of one phase.  The last chunk's done[] would not do: a set
+        // knows how far that barrier has come only from the chunks it converts
+        // itself, so the set that did not convert the last one could take the
+        // phase two before (the same parity) for the last.
+        if (ok) ok = mbar_wait_bounded(smem_addr(&all_done), 0);
         ok = __all_sync(0xffffffffu, ok);
         if (ok && (warp >> 2) < TILES) {
             tc_fence_after();
@@ -172,7 +176,10 @@ __global__ void __launch_bounds__(kPjThreads) nn_project_kernel(const unsigned c
                 mma_commit(smem_addr(&done[s]));
             }
             // TMEM and shared memory are given back only after every product
-            if (n)
+            if (n == n_chunks) {
+                mma_commit(smem_addr(&all_done));
+                ok = mbar_wait_bounded(smem_addr(&all_done), 0) && ok;
+            } else if (n)
                 ok = mbar_wait_bounded(smem_addr(&done[(n - 1) % STAGES]),
                                        ((n - 1) / STAGES) & 1) && ok;
         }
