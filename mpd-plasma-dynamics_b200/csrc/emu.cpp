@@ -35,6 +35,7 @@ struct EmuSolver {
     int len = 0;
     std::vector<double> cphys, wall[2];
     bool has_ring = false;  // the configuration has a ring table
+    bool walls_stale = false;  // as mpd_solver's
     mpd::CompiledRing ring;
 };
 
@@ -229,9 +230,14 @@ int mpd_emu_advance(void *h, double dt, int order) {
     v.bc = s->bc;
     if (order == 3 && s->has_ring && !first && s->precision == MPD_PRECISION_FAST) {
         RingFromTable(s, u0, u, dt);
+        s->walls_stale = true;
         s->step++;
         return MPD_OK;
     }
+    if (s->walls_stale)
+        for (int l = 1; l <= g.L; ++l)
+            mpd::wall_row_from_state(g, u0, s->wall[s->step & 1].data(), s->len, l);
+    s->walls_stale = false;
     const int nring = mpd::ring_count(g);
     std::vector<double> ring(8 * static_cast<size_t>(nring));
     for (int t = 0; t < nring; ++t) {

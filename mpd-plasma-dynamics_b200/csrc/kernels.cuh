@@ -1045,20 +1045,10 @@ __global__ void init_wall_kernel(Geo g, const double *ic, double *wall0, int len
     }
 }
 
-// The wall lines a boundary kernel reads, from the current state (steps >= 1,
-// fast precision): what it would have left after the last step.
+// The wall lines, from the current state.
 __global__ void wall_lines_kernel(Geo g, const double *u0, double *wall, int len) {
-    for (int l = 1 + blockIdx.x * blockDim.x + threadIdx.x; l <= g.L; l += gridDim.x * blockDim.x) {
-        BcView v;
-        v.g = g;
-        v.fast = 1;
-        for (int side = 0; side < 2; ++side) {
-            const int m = side ? g.M + 1 : 1;
-            double u[8];
-            load_cons(u0, g.ps, g.ix(l, m), u);
-            store_line_phys(wall, len, side, l, recon_bc(v, u, g.r(l, m)));
-        }
-    }
+    for (int l = 1 + blockIdx.x * blockDim.x + threadIdx.x; l <= g.L; l += gridDim.x * blockDim.x)
+        wall_row_from_state(g, u0, wall, len, l);
 }
 
 // Fields::InitConservative (src/fields.cpp:40-57) on the device: interior

@@ -737,6 +737,20 @@ MPD_HD Phys recon_bc(const BcView &v, const double u[8], double r) {
     return q;
 }
 
+// Row l of the wall lines, from the current state u (steps >= 1, fast
+// precision): what a boundary kernel would have left after the last step.
+MPD_HD void wall_row_from_state(const Geo &g, const double *u, double *wall, int len, int l) {
+    BcView v;
+    v.g = g;
+    v.fast = 1;
+    for (int side = 0; side < 2; ++side) {
+        const int m = side ? g.M + 1 : 1;
+        double c[8];
+        load_cons(u, g.ps, g.ix(l, m), c);
+        store_line_phys(wall, len, side, l, recon_bc(v, c, g.r(l, m)));
+    }
+}
+
 // Primitive values in evaluation order.
 struct Prim {
     double v[8];

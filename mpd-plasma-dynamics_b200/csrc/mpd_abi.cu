@@ -104,6 +104,7 @@ struct mpd_solver {
     double *partials = nullptr, *small = nullptr;
     double *cphys = nullptr;                 // central lines (boundary inputs)
     double *wall[2] = {nullptr, nullptr};    // wall lines, by step parity
+    bool walls_stale = false;                // steps since they were written took none of them along
     int len = 0;                             // line length
     int resid_blocks = 0;                    // residual_kernel: one resident wave
     CUtensorMap tmap[2];                     // conserved planes of buf[0] / buf[1]
@@ -284,6 +285,20 @@ int InitFromIc(mpd_solver *s) {
     MPD_CK(cudaStreamSynchronize(s->stream));
     RefreshMirror(s);
     s->host_step = 0;
+    s->walls_stale = false;
+    return MPD_OK;
+}
+
+// The wall lines of the current state (step steps taken) for an engine that
+// reads them: whole steps (lf_step_kernel) neither read nor write them.
+int RefreshWalls(mpd_solver *s, long long step) {
+    if (!s->walls_stale) return MPD_OK;
+    if (step > 0) {
+        mpd::wall_lines_kernel<<<(s->L + 127) / 128, 128, 0, s->stream>>>(
+            s->g, s->buf[step & 1], s->wall[step & 1], s->len);
+        MPD_CK(cudaGetLastError());
+    }
+    s->walls_stale = false;
     return MPD_OK;
 }
 
@@ -324,6 +339,7 @@ int LaunchInterior(mpd_solver *s, bool first, bool use_state_dt, double dt, bool
     s->whole_step = false;
     if (!first && !variant && WholeStep(s)) {
         s->whole_step = true;
+        s->walls_stale = true;
         return LaunchStep(s, use_state_dt, dt, want_ws, 0, (int)(s->host_step & 1));
     }
     if (first || s->precision == MPD_PRECISION_EXACT) {
@@ -884,6 +900,7 @@ static mpd::PersistArgs PersistArgsOf(const mpd_solver *s, int nstrips, int nban
 static int GraphLoop(mpd_solver *s, long long budget, int per_graph) {
     const long long cap = budget <= 0 ? 0 : (budget + per_graph - 1) / per_graph;
     if (cap == 0) return MPD_OK;
+    if (WholeStep(s)) s->walls_stale = true;
     long long launched = 0;
     int pending = 0;
     auto launch = [&](int slot) -> int {
@@ -997,6 +1014,8 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
     // (the persistent engine pays two grid barriers per step and runs the
     // boundary chains of every face inside one phase)
     if (p->engine == MPD_ENGINE_PERSISTENT) {
+        rc = RefreshWalls(s, step0);
+        if (rc != MPD_OK) return rc;
         // one cooperative launch per chunk of steps; the residual keeps the
         // graph path's schedule: after steps (step - base) % residual_every == 0
         const mpd::PersistArgs a =
@@ -1399,12 +1418,9 @@ int mpd_set_ring_overlap(mpd_solver *s, int on) {
     if (rc != MPD_OK) return rc;
     rc = SyncState(s);
     if (rc != MPD_OK) return rc;
-    if (on && WholeStep(s) && s->h_st->step > 0) {
-        // whole steps leave no wall lines; the boundary kernels start from them
-        const int par = static_cast<int>(s->h_st->step & 1);
-        mpd::wall_lines_kernel<<<(s->L + 127) / 128, 128, 0, s->stream>>>(s->g, s->buf[par],
-                                                                          s->wall[par], s->len);
-        MPD_CK(cudaGetLastError());
+    if (on) {
+        rc = RefreshWalls(s, s->h_st->step);
+        if (rc != MPD_OK) return rc;
         MPD_CK(cudaStreamSynchronize(s->stream));
     }
     s->ring_overlap = on ? 1 : 0;
@@ -1612,6 +1628,8 @@ int mpd_batch_run(mpd_batch *b, const mpd_run_params *p, int nteams, const int *
         mpd_run_params pi = *p;
         if (dt0) pi.dt = dt0[i];
         rc = PrepareRun(s, &pi, step0[i]);
+        if (rc != MPD_OK) return rc;
+        rc = RefreshWalls(s, step0[i]);
         if (rc != MPD_OK) return rc;
         MPD_CK(cudaEventRecord(s->ev0, s->stream));
         const bool first = !s->h_st->done && s->host_step == 0;

@@ -1,0 +1,72 @@
+"""One solver through several engines: the one-kernel steps of a graph run or of
+Advance, the persistent loop, a batch and the two-kernel form, each starting from
+what the one before it left.  Every plane, t, dt and wave speed must be those of
+a solver that took the two-kernel form throughout (its boundary kernel leaves
+the wall lines after every step)."""
+import numpy as np
+import pytest
+
+from tests import cases, ring_layouts
+
+pytestmark = pytest.mark.gpu
+
+LAYOUTS = [ring_layouts.thruster, ring_layouts.axis_mixed, ring_layouts.axis_everywhere,
+           ring_layouts.channel, ring_layouts.split]
+
+
+class Walk:
+    """A solver and the reference beside it, the same steps in both."""
+
+    def __init__(self, pkg, cfg):
+        case = cases.make_case(cfg)
+        self.pkg, self.dt = pkg, 1e-6
+        self.a = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast")
+        self.ref = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast")
+        self.ref.ring_overlap = True
+        self.batch = pkg.BatchSolver([self.a])
+
+    def _run(self, s, n, **kw):
+        return s.run(T=1e300, dt=self.dt, adaptive=True, max_steps=n, steps_per_graph=10, **kw)
+
+    def go(self, how, n):
+        want = None
+        if how == "advance":
+            for _ in range(n):
+                self.a.Advance(self.dt)
+                self.ref.Advance(self.dt)
+                dt = self.a.ComputeDt(self.dt)
+                assert dt == self.ref.ComputeDt(self.dt)
+                assert self.a.MaxWaveSpeed() == self.ref.MaxWaveSpeed()
+                self.dt = dt
+        else:
+            if how == "batch":
+                got = self.batch.run(self.pkg.BatchPlan([2], [0]), T=1e300, dt=self.dt,
+                                     adaptive=True, max_steps=n).runs[0]
+            elif how == "two kernels":
+                self.a.ring_overlap = True
+                got = self._run(self.a, n)
+                self.a.ring_overlap = False
+            else:
+                got = self._run(self.a, n, engine=how)
+            want = self._run(self.ref, n)
+            assert (got.steps, got.t, got.dt, got.max_wave_speed, got.residual) == \
+                (want.steps, want.t, want.dt, want.max_wave_speed, want.residual), (how, n)
+            self.dt = want.dt
+        np.testing.assert_array_equal(self.a.conserved(), self.ref.conserved(), err_msg=how)
+
+    def close(self):
+        self.batch.close()
+        self.a.close()
+        self.ref.close()
+
+
+@pytest.mark.parametrize("make", LAYOUTS, ids=lambda f: f.__name__)
+@pytest.mark.parametrize("lead", [3, 4])
+@pytest.mark.parametrize("whole", ["graph", "advance"])
+@pytest.mark.parametrize("other", ["persistent", "batch", "two kernels"])
+def test_boundary_after_whole_steps(pkg, make, lead, whole, other):
+    """The faces' old wall values, after an odd and an even number of whole steps."""
+    w = Walk(pkg, make(40, 31))
+    w.go(whole, lead)
+    w.go(other, 5)
+    w.close()

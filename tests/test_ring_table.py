@@ -50,3 +50,16 @@ def test_constant_parts_of_an_expression_fold_to_the_interpreters_bits():
             oracle.advance(1e-5)
             np.testing.assert_array_equal(b.conserved(), a.conserved())
             np.testing.assert_array_equal(exact.conserved(), oracle.conserved())
+
+
+@pytest.mark.parametrize("L,M", [(5, 4), (40, 31)])
+@pytest.mark.parametrize("make", ring_layouts.ACCEPTED, ids=lambda f: f.__name__)
+def test_general_ring_after_table_rings_bitwise(make, L, M):
+    """The general path starts from the walls' old values, which table rings
+    leave behind: they come from the state then, for either step parity."""
+    case = cases.make_case(make(L, M))
+    a, b = Emu(case, "fast"), Emu(case, "fast")
+    for order in (0, 3, 0, 3, 3, 0, 0, 3, 3, 3, 0):
+        a.advance(1e-5)
+        b.advance(1e-5, order=order)
+        np.testing.assert_array_equal(b.conserved(), a.conserved())
