@@ -82,8 +82,8 @@ struct alignas(128) StepCtl {
 
 // What the step kernels share: controller slots by launch parity; each step's
 // wave-speed maximum and non-finite flag by step count mod 3 (one being read,
-// one being accumulated, one being cleared) with the wait-failure flag, one
-// line; the run parameters (written by the host only), one line.
+// one being accumulated, one being cleared; all zero between sequences of
+// launches) with the wait-failure flag, one line; the run parameters (written by the host only), one line.
 struct StepHot {
     StepCtl ctl[2];
     struct alignas(128) Acc {

@@ -16,7 +16,8 @@
 // Launch i of a sequence takes slot = i & 1: it reads ctl[slot] and writes
 // ctl[slot ^ 1].  A stopped run's remaining launches copy the slot on.
 // finish_steps_kernel ends a sequence: it works out the last step's
-// controller, leaves the canonical DevState fields and slot 0 current.
+// controller, leaves the canonical DevState fields, slot 0 current and the
+// wave-speed maxima zero.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -345,6 +346,12 @@ __global__ void finish_steps_kernel(Geo g, DevState *st, int slot) {
     const int wait_fail = x.wait_fail();
     if (threadIdx.x != 0) return;
     st->hot.ctl[0] = c;
+    // the step has ended: no maximum is needed any more, and steps of another
+    // kernel may come before the next of these, so all three start from zero
+    for (int k = 0; k < 3; ++k) {
+        st->hot.acc.ws[k] = 0ull;
+        st->hot.acc.nf[k] = 0u;
+    }
     if (c.step == step0) {
         if (run.run_mode && c.done) st->done = 1;
         return;

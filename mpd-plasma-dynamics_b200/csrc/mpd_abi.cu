@@ -1510,7 +1510,8 @@ int mpd_profile_kernel(mpd_solver *s, int which, int launches, double dt, double
     if (which != MPD_KERNEL_RESIDUAL) {
         MPD_CK(cudaMemsetAsync(&s->st->ws_acc, 0, sizeof(unsigned long long), s->stream));
         MPD_CK(cudaMemsetAsync(&s->st->nf_acc, 0, sizeof(unsigned int), s->stream));
-        MPD_CK(cudaMemsetAsync(&s->st->hot.acc, 0, sizeof(s->st->hot.acc), s->stream));
+        MPD_CK(cudaMemsetAsync(&s->st->hot.acc, 0, offsetof(mpd::StepHot::Acc, wait_fail),
+                               s->stream));
         MPD_CK(cudaStreamSynchronize(s->stream));
     }
     return SyncState(s);

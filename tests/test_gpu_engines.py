@@ -70,3 +70,20 @@ def test_boundary_after_whole_steps(pkg, make, lead, whole, other):
     w.go(whole, lead)
     w.go(other, 5)
     w.close()
+
+
+@pytest.mark.parametrize("lead", [2, 3, 4])
+@pytest.mark.parametrize("between", [1, 2, 3])
+@pytest.mark.parametrize("other", ["persistent", "batch", "two kernels"])
+def test_wave_speed_of_whole_steps_after_others(pkg, lead, between, other):
+    """The thruster's start-up, its wave speed falling every few steps: a maximum
+    left from before the other engine's steps would show in the next one's."""
+    w = Walk(pkg, ring_layouts.thruster(40, 31))
+    speeds = []
+    for how, n in (("graph", lead), (other, between), ("graph", 1), ("advance", 2),
+                   (other, between), ("advance", 1), (other, between), ("graph", 12)):
+        w.go(how, n)
+        speeds.append(w.ref.MaxWaveSpeed())
+    assert all(b < a for a, b in zip(speeds, speeds[1:])), speeds
+    assert w.a.MaxWaveSpeed() == speeds[-1]
+    w.close()
