@@ -320,6 +320,7 @@ def run_ours(args, rank, world, local_rank):
     w = max(args.warmup, 1)
     wres = solver.run(T=1e300, dt=cfg.dt, adaptive=True, max_steps=w, steps_per_graph=per_graph)
     assert wres.steps == w, wres
+    graphs = solver.graph_builds()
 
     uuid = None
     try:
@@ -341,6 +342,7 @@ def run_ours(args, rank, world, local_rank):
         dist.barrier()
     clocks = sampler.stop()
     assert res.steps == args.steps, res
+    assert solver.graph_builds() == graphs, "a graph was captured inside the timed region"
     t_max = max_over_ranks(res.device_ms)
 
     # per-launch device time of the dominant kernel and of the residual pass:

@@ -254,6 +254,10 @@ int mpd_ring_overlap_active(mpd_solver *s, int *active);
 int mpd_get_stream(mpd_solver *s, void **stream);
 /* Bytes of device memory the handle holds. */
 int mpd_device_bytes(mpd_solver *s, size_t *bytes);
+/* Measurement support (new; no reference counterpart): how many CUDA graphs
+ * mpd_run has captured for the handle so far.  Runs of one kind (steps per
+ * graph, adaptive or not, residual and check interval) share them. */
+int mpd_graph_builds(mpd_solver *s, long long *builds);
 
 /* Measurement support (new; no reference counterpart): advance `steps` steps
  * with time step dt, launching eagerly with CUDA events around each kernel on

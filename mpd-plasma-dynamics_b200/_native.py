@@ -158,6 +158,7 @@ SIGNATURES = [
     ("mpd_set_ring_overlap", C.c_int, [_VP, C.c_int]),
     ("mpd_ring_overlap_active", C.c_int, [_VP, C.POINTER(C.c_int)]),
     ("mpd_device_bytes", C.c_int, [_VP, C.POINTER(C.c_size_t)]),
+    ("mpd_graph_builds", C.c_int, [_VP, C.POINTER(C.c_longlong)]),
     ("mpd_profile_kernels", C.c_int, [_VP, C.c_int, C.c_double, DP]),
     ("mpd_profile_kernel", C.c_int, [_VP, C.c_int, C.c_int, C.c_double, DP]),
     ("mpd_integrals_noalloc", C.c_int, [_VP, C.c_size_t, C.c_int, C.c_int, C.c_int, _VP, C.c_double,

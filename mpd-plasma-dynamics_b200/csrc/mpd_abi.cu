@@ -139,8 +139,22 @@ struct mpd_solver {
     int precision = MPD_PRECISION_EXACT;
     int with_prev = 0;
     long long host_step = 0;
-    cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0, graph_check = 0, graph_resid = 0, graph_every = 0, graph_at = 0;
+    // the run loop's captured graphs: of one kind of run (GraphKind), one for
+    // each offset of the change check met last (BuildGraph)
+    struct GraphKind {
+        int steps = 0, flags = 0, resid_every = 0, check_every = 0;
+        bool operator==(const GraphKind &o) const {
+            return steps == o.steps && flags == o.flags && resid_every == o.resid_every &&
+                   check_every == o.check_every;
+        }
+    } graph_kind;
+    struct RunGraph {
+        cudaGraphExec_t exec;
+        int check_at;
+    };
+    std::vector<RunGraph> graphs;
+    cudaGraphExec_t graph = nullptr;  // the one of `graphs` in use
+    long long graph_builds = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, snap_ev = nullptr, stage_ev = nullptr;
     bool snap_pending = false;
     size_t dev_bytes = 0;
@@ -176,7 +190,7 @@ void FreeAll(mpd_solver *s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->side) cudaStreamSynchronize(s->side);
-    if (s->graph) cudaGraphExecDestroy(s->graph);
+    for (const mpd_solver::RunGraph &r : s->graphs) cudaGraphExecDestroy(r.exec);
     cudaFree(s->buf[0]);
     cudaFree(s->buf[1]);
     cudaFree(s->ic);
@@ -320,7 +334,8 @@ bool WholeStep(const mpd_solver *s) {
     return s->ring_ok && !s->ring_overlap && !MPD_INTERIOR_PAIR;
 }
 
-// parity: that of the step count the launch starts from, -1 where unknown.
+// parity: that of the step count the launch starts from less the run's
+// (StepHot::Run::parity), -1 where unknown.
 int LaunchStep(mpd_solver *s, bool use_state_dt, double dt, bool want_ws, int slot, int parity) {
     MPD_CK(mpd::launch_lf_step(s->g, s->step_plan, s->tmap[0], s->tmap[1], s->buf[0], s->buf[1],
                                s->st, dt, use_state_dt ? 1 : 0, want_ws, s->ring, slot,
@@ -462,23 +477,41 @@ int CheckHandle(mpd_solver *s) {
     return MPD_OK;
 }
 
-// parity: that of the step count every launch of the graph starts from, -1
-// where it may vary (a hint: a launch that finds another count is only slower).
 // check_every / check_at: the relative-change check follows the steps i (from
 // 1) with i % check_every == check_at; check_at < 0: every step (the
 // controller's own due flag decides).
+// A handle keeps the graphs of its last kind of run.  Continued runs start at
+// other step counts: without a check one graph serves them all, with one there
+// is a graph per offset of the check, the last kRunGraphs of them kept.  (100
+// steps of 100 x 40, B200: 0.6 ms to capture and instantiate; a check's two
+// nodes and the controller after every step instead of where due, which any
+// offset could share, cost 0.3 ms a hundred steps.)
+constexpr size_t kRunGraphs = 16;
+
 int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resid_every,
-               int check_every, int check_at, int parity) {
-    const int key = (with_check ? 1 : 0) | (want_ws ? 2 : 0) | (s->ring_overlap ? 4 : 0) |
-                    (WholeStep(s) ? 8 * (parity + 2) : 0);
-    if (s->graph && s->graph_steps == steps && s->graph_check == key &&
-        s->graph_resid == resid_every &&
-        (!with_check || (s->graph_every == check_every && s->graph_at == check_at)))
-        return MPD_OK;
-    if (s->graph) {
-        cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
+               int check_every, int check_at) {
+    const mpd_solver::GraphKind kind{
+        steps, (with_check ? 1 : 0) | (want_ws ? 2 : 0) | (s->ring_overlap ? 4 : 0), resid_every,
+        with_check ? check_every : 0};
+    s->graph = nullptr;
+    if (!(kind == s->graph_kind)) {
+        for (const mpd_solver::RunGraph &r : s->graphs) cudaGraphExecDestroy(r.exec);
+        s->graphs.clear();
+        s->graph_kind = kind;
     }
+    auto cached = [&](int at) {
+        for (const mpd_solver::RunGraph &r : s->graphs)
+            if (r.check_at == at) s->graph = r.exec;
+        return s->graph != nullptr;
+    };
+    if (!with_check) check_at = -1;
+    if (cached(check_at)) return MPD_OK;
+    if (s->graphs.size() == kRunGraphs) {  // the stream is idle: no launch uses it
+        cudaGraphExecDestroy(s->graphs.front().exec);
+        s->graphs.erase(s->graphs.begin());
+    }
+    // consecutive launches start at one parity where a graph's steps are even
+    const bool parity_known = steps % 2 == 0;
     cudaGraph_t graph = nullptr;
     MPD_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int rc = MPD_OK;
@@ -490,7 +523,7 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
             rc = EnqueueStep(s, false, true, 0.0, check, want_ws, res);
             continue;
         }
-        rc = LaunchStep(s, true, 0.0, want_ws, slot, parity < 0 ? -1 : (parity + i) & 1);
+        rc = LaunchStep(s, true, 0.0, want_ws, slot, parity_known ? i & 1 : -1);
         slot ^= 1;
         if (rc == MPD_OK && (res || check || i == steps - 1)) {
             const cudaError_t ef = mpd::launch_finish_steps(s->g, s->st, want_ws, slot, s->stream);
@@ -505,14 +538,13 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
         return rc;
     }
     if (e != cudaSuccess) return Fail(MPD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    const cudaError_t e2 = cudaGraphInstantiate(&s->graph, graph, 0);
+    cudaGraphExec_t exec = nullptr;
+    const cudaError_t e2 = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e2 != cudaSuccess) return Fail(MPD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2));
-    s->graph_steps = steps;
-    s->graph_check = key;
-    s->graph_resid = resid_every;
-    s->graph_every = check_every;
-    s->graph_at = check_at;
+    s->graphs.push_back({exec, check_at});
+    s->graph = exec;
+    s->graph_builds++;
     return MPD_OK;
 }
 
@@ -798,6 +830,7 @@ static int FinishRun(mpd_solver *s, long long step0, mpd_run_stats *stats) {
     h.resid_every = 1;
     h.T = INFINITY;
     h.max_steps = LLONG_MAX;
+    h.hot.run.parity = 0;
     rc = PushState(s);
     if (rc != MPD_OK) return rc;
     if (nonfinite) return Fail(MPD_ERR_NONFINITE, "non-finite value in the state");
@@ -867,6 +900,8 @@ static int PrepareRun(mpd_solver *s, const mpd_run_params *p, long long &step0) 
     if (h.t + dt > h.T) dt = h.T - h.t;  // src/main.cpp:221-223
     h.dt = dt;
     if (!(h.t < h.T)) h.done = 1;
+    // graph launches start after the exact first step, where there is one
+    h.hot.run.parity = static_cast<int>((h.step + (s->host_step == 0 ? 1 : 0)) & 1);
     return PushState(s);
 }
 
@@ -1000,6 +1035,41 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
     if (rc != MPD_OK) return rc;
     mpd::DevState &h = *s->h_st;
 
+    const bool monitored = p->monitor && p->monitor_every > 0;
+    // Steps per graph launch: a multiple of the residual interval, so that the
+    // residual is evaluated every residual_every steps; with monitor reports,
+    // a divisor of monitor_every where the residual interval allows.
+    int per_graph = p->steps_per_graph > 0 ? p->steps_per_graph : 100;
+    if (monitored && p->monitor_every % per_graph != 0) {
+        int a = per_graph, b = p->monitor_every;
+        while (b) {
+            const int r = a % b;
+            a = b;
+            b = r;
+        }
+        per_graph = a;
+    }
+    if (with_check && p->check_frequency > 0 && per_graph % p->check_frequency != 0 &&
+        p->check_frequency < per_graph)
+        per_graph = (per_graph / p->check_frequency) * p->check_frequency;
+    if (p->residual_every > 0 && per_graph % p->residual_every != 0)
+        per_graph = (per_graph / p->residual_every + 1) * p->residual_every;
+    long long taken_before = (!h.done && s->host_step == 0) ? 1 : 0;  // the exact first step
+    // Every graph launch starts a multiple of per_graph steps after the run's
+    // first (the monitored loop stops in between and does not): where that is
+    // a multiple of the check interval, the check's nodes follow only the
+    // steps it is due after.
+    int check_at = -1;
+    if (with_check && !monitored && per_graph % p->check_frequency == 0)
+        check_at = static_cast<int>((p->check_frequency - (step0 + taken_before) %
+                                     p->check_frequency) % p->check_frequency);
+    // before the run's first event: a capture is no part of its device time
+    if (p->engine != MPD_ENGINE_PERSISTENT) {
+        rc = BuildGraph(s, per_graph, with_check, want_ws, p->residual_every, p->check_frequency,
+                        check_at);
+        if (rc != MPD_OK) return rc;
+    }
+
     s->ev_stop = nullptr;
     MPD_CK(cudaEventRecord(s->ev0, s->stream));
     if (!h.done && s->host_step == 0) {
@@ -1037,39 +1107,6 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
         }
         return FinishRun(s, step0, stats);
     }
-    const bool monitored = p->monitor && p->monitor_every > 0;
-    // Steps per graph launch: a multiple of the residual interval, so that the
-    // residual is evaluated every residual_every steps; with monitor reports,
-    // a divisor of monitor_every where the residual interval allows.
-    int per_graph = p->steps_per_graph > 0 ? p->steps_per_graph : 100;
-    if (monitored && p->monitor_every % per_graph != 0) {
-        int a = per_graph, b = p->monitor_every;
-        while (b) {
-            const int r = a % b;
-            a = b;
-            b = r;
-        }
-        per_graph = a;
-    }
-    if (with_check && p->check_frequency > 0 && per_graph % p->check_frequency != 0 &&
-        p->check_frequency < per_graph)
-        per_graph = (per_graph / p->check_frequency) * p->check_frequency;
-    if (p->residual_every > 0 && per_graph % p->residual_every != 0)
-        per_graph = (per_graph / p->residual_every + 1) * p->residual_every;
-    long long taken_before = (!h.done && s->host_step == 0) ? 1 : 0;  // the exact first step
-    // Every graph launch starts a multiple of per_graph steps after the run's
-    // first (the monitored loop stops in between and does not): where that is
-    // a multiple of the check interval, the check's nodes follow only the
-    // steps it is due after.
-    int check_at = -1;
-    if (with_check && !monitored && per_graph % p->check_frequency == 0)
-        check_at = static_cast<int>((p->check_frequency - (step0 + taken_before) %
-                                     p->check_frequency) % p->check_frequency);
-    const int parity =
-        monitored || per_graph % 2 != 0 ? -1 : static_cast<int>((step0 + taken_before) & 1);
-    rc = BuildGraph(s, per_graph, with_check, want_ws, p->residual_every, p->check_frequency,
-                    check_at, parity);
-    if (rc != MPD_OK) return rc;
     const long long end = step0 + p->max_steps;
     for (;;) {
         // steps this segment may take: to the controller's current stop
@@ -1095,6 +1132,7 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
         const long long next = (h.step / p->monitor_every + 1) * p->monitor_every;
         h.max_steps = next < end ? next : end;
         h.done = 0;
+        h.hot.run.parity = static_cast<int>(h.step & 1);
         rc = PushState(s);
         if (rc != MPD_OK) return rc;
     }
@@ -1515,6 +1553,12 @@ int mpd_profile_kernel(mpd_solver *s, int which, int launches, double dt, double
         MPD_CK(cudaStreamSynchronize(s->stream));
     }
     return SyncState(s);
+}
+
+int mpd_graph_builds(mpd_solver *s, long long *builds) {
+    if (!s || !builds) return Fail(MPD_ERR_INVALID, "bad arguments");
+    *builds = s->graph_builds;
+    return MPD_OK;
 }
 
 int mpd_device_bytes(mpd_solver *s, size_t *bytes) {

@@ -322,6 +322,12 @@ class GpuSolver:
         self._call("mpd_device_bytes", C.byref(b))
         return b.value
 
+    def graph_builds(self) -> int:
+        """CUDA graphs captured for this solver's runs so far."""
+        b = C.c_longlong()
+        self._call("mpd_graph_builds", C.byref(b))
+        return b.value
+
 
 def build_case(cfg: SimConfig, precision: str = "fast", with_prev: bool | None = None,
                ic: IInitialCondition | None = None) -> GpuSolver:

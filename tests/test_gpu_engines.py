@@ -87,3 +87,36 @@ def test_wave_speed_of_whole_steps_after_others(pkg, lead, between, other):
     assert all(b < a for a, b in zip(speeds, speeds[1:])), speeds
     assert w.a.MaxWaveSpeed() == speeds[-1]
     w.close()
+
+
+def test_continued_runs_reuse_their_graphs(pkg):
+    """Runs from odd and even steps, plain and monitored, and new initial states
+    need one graph; with a change check one for each offset, the last 16 kept."""
+    case = cases.make_case(ring_layouts.channel(40, 31))
+    a = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast", with_prev=True)
+    b = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast", with_prev=True)
+    b.ring_overlap = True
+
+    def both(**kw):
+        r = [s.run(T=1e300, dt=1e-6, adaptive=True, **kw) for s in (a, b)]
+        assert (r[0].steps, r[0].t, r[0].dt, r[0].change) == \
+            (r[1].steps, r[1].t, r[1].dt, r[1].change)
+        np.testing.assert_array_equal(a.conserved(), b.conserved())
+
+    for n in (100, 100, 31, 100, 7, 100):
+        both(max_steps=n, steps_per_graph=10)
+    a.run(T=1e300, dt=1e-6, max_steps=33, steps_per_graph=10, monitor=lambda rep: None,
+          monitor_every=20)
+    b.run(T=1e300, dt=1e-6, max_steps=33, steps_per_graph=10)
+    a.set_physical(case.phys)
+    b.set_physical(case.phys)
+    both(max_steps=100, steps_per_graph=10)
+    assert a.graph_builds() == 1
+    check = dict(steps_per_graph=20, convergence_threshold=1e-30, check_frequency=20)
+    for n in (60, 60, 47, 60, 13, 60, 60):   # two offsets
+        both(max_steps=n, **check)
+    assert a.graph_builds() == 3
+    for _ in range(40):                      # all 20 offsets, twice
+        both(max_steps=21, **check)
+    a.close()
+    b.close()
