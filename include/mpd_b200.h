@@ -366,6 +366,14 @@ typedef struct mpd_gemm_desc {
 int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream);
 int mpd_nn_wait_status(void *stream);
 
+/* Widths of the network the entry points below are made for: inputs per point,
+ * channels, basis functions, hidden columns of the projection, outputs. */
+#define MPD_NN_INPUTS 6
+#define MPD_NN_WIDTH 64
+#define MPD_NN_BASIS 256
+#define MPD_NN_HIDDEN 128
+#define MPD_NN_OUTPUTS 8
+
 /* A (rows x K) FP32 operand at src[row * s_row + k * s_k], rounded to BF16 as
  * the GEMM rounds it and laid out as the tensor core reads it, for operands
  * that stay the same over many calls: blocks of block_k (a multiple of 8)

@@ -29,8 +29,8 @@
 
 namespace {
 
-constexpr int kLyW = 64;             // network width: columns of h, K of the first product
-constexpr int kLyQ = 256;            // K of the second product (basis functions)
+constexpr int kLyW = MPD_NN_WIDTH;   // columns of h, K of the first product
+constexpr int kLyQ = MPD_NN_BASIS;   // K of the second product
 constexpr int kLyRows = 128;
 constexpr int kLyEpiWarps = 8, kLyCvtWarps = 4;
 constexpr int kLyThreads = (kLyEpiWarps + kLyCvtWarps + 2) * 32;
@@ -43,6 +43,10 @@ constexpr uint32_t kLyTmem = 256;
 // The 128-wide projection with another product after it (OUT2 columns):
 constexpr int kLyYBytes = kLyRows * 128 * 2;      // 32 KB: GELU(z) in BF16
 constexpr int kLyW2Bytes = 64 * 128 * 2;          // 16 KB: columns past OUT2 are zero
+
+static_assert(kLyW == 64 && kLyQ == 256 && MPD_NN_HIDDEN == 128 && MPD_NN_OUTPUTS == 8 &&
+                  MPD_NN_INPUTS <= 8,
+              "tiles, accumulators and operand layouts below are laid out for these");
 
 enum LayerEpilogue { kEpiForward = 0, kEpiActBwd = 1, kEpiPlain = 2 };
 
@@ -577,7 +581,7 @@ namespace {
 // per SM (their TMEM is 2 x 64 columns each) take even shares of the 128-row
 // tiles; the rows of tile i + 1 are fetched into registers and the product of
 // tile i runs while tile i - 1 is stored.
-constexpr int kLiftK = 6;
+constexpr int kLiftK = MPD_NN_INPUTS;
 
 __global__ void __launch_bounds__(128, 4) nn_lift_kernel(const float *x, const float *w,
                                                          const float *bias, long long rows,

@@ -124,6 +124,11 @@ class SpectralOperator:
         self.torch = torch
         self.H, self.W, self.P, self.B = H, W, H * W, batch
         self.Q = (2 * MODES) ** 2
+        net = (N_IN, WIDTH, self.Q, HIDDEN, N_OUT)
+        kernels = (nn.INPUTS, nn.WIDTH, nn.BASIS, nn.HIDDEN, nn.OUTPUTS)
+        if net != kernels:
+            raise ValueError(f"inputs, width, basis functions, hidden and output columns {net}: "
+                             f"the kernels are made for {kernels}")
         self.shapes = param_shapes()
         sizes = [int(np.prod(s)) for _, s in self.shapes]
         self.nparam = sum(sizes)
@@ -197,7 +202,8 @@ class SpectralOperator:
 
     def _wgrad(self, a, gz, weight, bias):
         """Gradients of a linear layer's weight (a^T gz) and bias (column sums of gz)."""
-        nn.wgrad(a, gz, self.P, self.B, self.g[weight], self.g[bias], self.work, self.colwork)
+        nn.wgrad(a, gz, self.P, self.B, self.g[weight], self.g[bias], self.work, self.colwork,
+                 check=False)
 
     # --------------------------------------------------------------- forward
     def load_inputs(self, x: np.ndarray):
@@ -207,19 +213,19 @@ class SpectralOperator:
     def forward(self):
         B, P, Cw = self.B, self.P, WIDTH
         p = self.p
-        nn.lift(self.x, p["W_in"], p["b_in"], self.z[0])
+        nn.lift(self.x, p["W_in"], p["b_in"], self.z[0], check=False)
         for l in range(LAYERS):
             h, z = self.h[l], self.z[l + 1]
             # V[b] = F h[b] (Q x C), U[b, q] = V[b, q] R[q]
             nn.spectral(h, self.F_img, p[f"R{l}"], 1, Cw, self.V[l], self.U, self.u_image, P, B,
-                        work=self.work)
+                        work=self.work, check=False)
             # z[b] = h W + G U[b] + bias, h' = GELU(z) (z itself after the last layer)
             nn.layer(h, p[f"W{l}"], 1, Cw, z, P, B, basis=self.G_img, u_image=self.u_image,
                      bias=p[f"b{l}"],
-                     out1=self.h[l + 1] if l < LAYERS - 1 else None)
+                     out1=self.h[l + 1] if l < LAYERS - 1 else None, check=False)
         nn.layer(self.h[LAYERS], p["W_p1"], 1, HIDDEN, self.zp, B * P, 1, n_out=HIDDEN,
                  bias=p["b_p1"], out1=self.y1, w2=p["W_p2"], w2_sn=1, w2_sk=N_OUT,
-                 bias2=p["b_p2"], out2=self.out)
+                 bias2=p["b_p2"], out2=self.out, check=False)
         return self.out
 
     def loss_and_grad(self, target) -> None:
@@ -240,7 +246,8 @@ class SpectralOperator:
         # gzp = (g_out W_p2^T) GELU'(zp), gh = gzp W_p1^T
         gzp, gh = self.gzp, self.gh[0]
         nn.layer(self.g_out, p["W_p2"], N_OUT, 1, gzp, rows, 1, n_out=HIDDEN,
-                 epilogue=nn.ACT_BWD, z_in=self.zp, w2=p["W_p1"], w2_sn=HIDDEN, w2_sk=1, out2=gh)
+                 epilogue=nn.ACT_BWD, z_in=self.zp, w2=p["W_p1"], w2_sn=HIDDEN, w2_sk=1, out2=gh,
+                 check=False)
         self._wgrad(self.h[LAYERS], gzp, "W_p1", "b_p1")
         gz = gh   # the last layer has no activation
         for l in reversed(range(LAYERS)):
@@ -248,7 +255,8 @@ class SpectralOperator:
             # gU[b] = G^T gz[b], gV[b, q] = gU[b, q] R[q]^T, dR[q] = sum_b V[b, q]^T gU[b, q]
             fused = B <= nn.MIX_GRAD_MAX_B
             nn.spectral(gz, self.Gt_img, p[f"R{l}"], Cw, 1, self.gU, self.gV, self.u_image, P, B,
-                        work=self.work, V_fwd=self.V[l], dR=g[f"R{l}"] if fused else None)
+                        work=self.work, V_fwd=self.V[l], dR=g[f"R{l}"] if fused else None,
+                        check=False)
             if not fused:
                 nn.gemm(self.V[l], self.gU, g[f"R{l}"], Cw, Cw, B, Q, sa=(1, Q * Cw, Cw),
                         sb=(1, Q * Cw, Cw), sc=(Cw, 1, Cw * Cw))
@@ -256,7 +264,7 @@ class SpectralOperator:
             gh = self.gh[1] if gz is self.gh[0] else self.gh[0]
             nn.layer(gz, p[f"W{l}"], Cw, 1, gh, P, B, basis=self.Ft_img,
                      u_image=self.u_image, epilogue=nn.ACT_BWD if l else nn.PLAIN,
-                     z_in=self.z[l] if l else None)
+                     z_in=self.z[l] if l else None, check=False)
             gz = gh
         # lift (the input needs no gradient)
         self._wgrad(self.x, gh, "W_in", "b_in")
