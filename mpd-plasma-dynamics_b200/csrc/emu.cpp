@@ -14,6 +14,7 @@
 #include "../../include/mpd_b200.h"
 #include "bc_compile.hpp"
 #include "lf_core.cuh"
+#include "once_per_device.hpp"
 
 namespace mpd {
 namespace {
@@ -288,6 +289,19 @@ int mpd_emu_download(void *h, int which, double *out) {
             out[g.ix(l, m)] = v[which - 8];
         }
     return MPD_OK;
+}
+
+// OncePerDevice over n calls: call i on devices[i], its work returning rc[i];
+// ran[i]: whether the work ran, ret[i]: what the call returned.
+void mpd_emu_once_per_device(const int *devices, const int *rc, int n, int *ran, int *ret) {
+    mpd::OncePerDevice once;
+    for (int i = 0; i < n; ++i) {
+        ran[i] = 0;
+        ret[i] = once(devices[i], [&] {
+            ran[i] = 1;
+            return rc[i];
+        });
+    }
 }
 
 int mpd_emu_has_ring(void *h) { return static_cast<EmuSolver *>(h)->has_ring ? 1 : 0; }

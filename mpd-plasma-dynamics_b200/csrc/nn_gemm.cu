@@ -36,6 +36,7 @@
 #include <string>
 
 #include "../../include/mpd_b200.h"
+#include "once_per_device.hpp"
 #include "tma.cuh"
 
 namespace mpd {
@@ -470,22 +471,29 @@ int NnLaunched(const char *what) {
     return MPD_ERR_CUDA;
 }
 
+// The kernel's opt-in to more than 48 KB of dynamic shared memory.
+template <class Kernel>
+int LargeSmem(mpd::OncePerDevice &once, Kernel kernel, int smem, const char *what) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess)
+        e = static_cast<cudaError_t>(once(device, [&] {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        }));
+    if (e == cudaSuccess) return MPD_OK;
+    mpd::SetLastError(std::string(what) + ": " + cudaGetErrorString(e));
+    return MPD_ERR_CUDA;
+}
+
 template <int K1, int K2, int NB, int EPI, int OUT2>
 int LaunchLayer(const LayerArgs &a, cudaStream_t st) {
     constexpr int smem = layer_smem<K2, NB, OUT2>();
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(
-            nn_layer_kernel<K1, K2, NB, EPI, OUT2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) {
-            mpd::SetLastError(std::string("mpd_nn_layer: ") + cudaGetErrorString(e));
-            return MPD_ERR_CUDA;
-        }
-        attr_set = true;
-    }
+    const auto kernel = nn_layer_kernel<K1, K2, NB, EPI, OUT2>;
+    static mpd::OncePerDevice once;
+    const int rc = LargeSmem(once, kernel, smem, "mpd_nn_layer");
+    if (rc != MPD_OK) return rc;
     const long long items = (long long)a.tiles * a.B;
-    nn_layer_kernel<K1, K2, NB, EPI, OUT2>
-        <<<(int)(items < 148 ? items : 148), kLyThreads, smem, st>>>(a);
+    kernel<<<(int)(items < 148 ? items : 148), kLyThreads, smem, st>>>(a);
     return NnLaunched("mpd_nn_layer");
 }
 
@@ -498,16 +506,9 @@ int LaunchWgrad(WgradArgs a, long long work_floats, cudaStream_t st) {
         mpd::SetLastError("mpd_nn_wgrad: batch too large for one launch or for its scratch");
         return MPD_ERR_INVALID;
     }
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(
-            nn_wgrad_kernel<KA, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) {
-            mpd::SetLastError(std::string("mpd_nn_wgrad: ") + cudaGetErrorString(e));
-            return MPD_ERR_CUDA;
-        }
-        attr_set = true;
-    }
+    static mpd::OncePerDevice once;
+    const int rc = LargeSmem(once, nn_wgrad_kernel<KA, N>, smem, "mpd_nn_wgrad");
+    if (rc != MPD_OK) return rc;
     nn_wgrad_kernel<KA, N><<<a.B * a.ksplit + ((N + 31) / 32) * kWgColSlices, kWgThreads, smem,
                              st>>>(a);
     nn_wgrad_sum_kernel<<<(KA * N + 31) / 32 + 1, kWgSumWarps * 32, 0, st>>>(a, KA * N, N);
@@ -516,17 +517,9 @@ int LaunchWgrad(WgradArgs a, long long work_floats, cudaStream_t st) {
 
 template <int TILES>
 int LaunchProject(const mpd_spectral_desc &d, int ksplit, int kspan, cudaStream_t st) {
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(nn_project_kernel<TILES>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmem<TILES>);
-        if (e != cudaSuccess) {
-            mpd::SetLastError(std::string("mpd_nn_spectral: ") + cudaGetErrorString(e));
-            return MPD_ERR_CUDA;
-        }
-        attr_set = true;
-    }
+    static mpd::OncePerDevice once;
+    const int rc = LargeSmem(once, nn_project_kernel<TILES>, kPjSmem<TILES>, "mpd_nn_spectral");
+    if (rc != MPD_OK) return rc;
     nn_project_kernel<TILES><<<d.B * ksplit * (2 / TILES), kPjThreads, kPjSmem<TILES>, st>>>(
         static_cast<const unsigned char *>(d.basis), d.h, d.P, d.B, kspan,
         ksplit > 1 ? d.work : d.V);
@@ -710,16 +703,9 @@ int mpd_nn_gemm(const mpd_gemm_desc *d, void *stream) {
     }
     const dim3 grid((d->M + kTileM - 1) / kTileM, (d->N + kTileN - 1) / kTileN,
                     d->batch * ksplit);
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        const cudaError_t ea = cudaFuncSetAttribute(
-            nn_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-        if (ea != cudaSuccess) {
-            mpd::SetLastError(std::string("mpd_nn_gemm: ") + cudaGetErrorString(ea));
-            return MPD_ERR_CUDA;
-        }
-        attr_set = true;
-    }
+    static mpd::OncePerDevice once;
+    const int rc = LargeSmem(once, nn_gemm_kernel, kGemmSmem, "mpd_nn_gemm");
+    if (rc != MPD_OK) return rc;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     nn_gemm_kernel<<<grid, kGemmThreads, kGemmSmem, st>>>(*d, ksplit, kspan);
     if (ksplit > 1) {

@@ -89,3 +89,16 @@ def test_wrong_operands_are_refused(monkeypatch, which):
             with pytest.raises(ValueError):
                 fn(**{**args, k: b})
     assert len(calls) == 1
+
+
+def test_attributes_are_set_once_on_each_device():
+    """A kernel's shared-memory opt-in: again on another device, and after a failure."""
+    import ctypes as C
+    calls = [(0, 0, 1), (0, 0, 0), (1, 5, 1), (1, 0, 1), (1, 0, 0), (0, 0, 0), (63, 0, 1),
+             (63, 0, 0), (64, 0, 1), (64, 0, 1)]
+    arr = lambda v: (C.c_int * len(calls))(*v)
+    ran, ret = arr([9] * len(calls)), arr([9] * len(calls))
+    pkg._native.load_emu().mpd_emu_once_per_device(arr(c[0] for c in calls),
+                                                   arr(c[1] for c in calls), len(calls), ran, ret)
+    assert list(ran) == [c[2] for c in calls]
+    assert list(ret) == [c[1] for c in calls]
