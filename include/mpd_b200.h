@@ -256,7 +256,9 @@ int mpd_get_stream(mpd_solver *s, void **stream);
 int mpd_device_bytes(mpd_solver *s, size_t *bytes);
 /* Measurement support (new; no reference counterpart): how many CUDA graphs
  * mpd_run has captured for the handle so far.  Runs of one kind (steps per
- * graph, adaptive or not, residual and check interval) share them. */
+ * graph, adaptive or not, residual and check interval) share them: one for
+ * starts from even and one from odd steps, and with a change check for each
+ * offset to its interval. */
 int mpd_graph_builds(mpd_solver *s, long long *builds);
 
 /* Measurement support (new; no reference counterpart): advance `steps` steps

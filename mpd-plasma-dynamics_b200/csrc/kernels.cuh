@@ -95,7 +95,6 @@ struct StepHot {
         double T, cfl, growth, dt_min, dt_max;
         long long max_steps;
         int run_mode, adaptive;
-        int parity;  // that of the step count a run's graph launches start from; else 0
     } run;
 };
 

@@ -140,7 +140,7 @@ struct mpd_solver {
     int with_prev = 0;
     long long host_step = 0;
     // the run loop's captured graphs: of one kind of run (GraphKind), one for
-    // each offset of the change check met last (BuildGraph)
+    // each kind of start met last (BuildGraph)
     struct GraphKind {
         int steps = 0, flags = 0, resid_every = 0, check_every = 0;
         bool operator==(const GraphKind &o) const {
@@ -150,7 +150,7 @@ struct mpd_solver {
     } graph_kind;
     struct RunGraph {
         cudaGraphExec_t exec;
-        int check_at;
+        int check_at, parity;
     };
     std::vector<RunGraph> graphs;
     cudaGraphExec_t graph = nullptr;  // the one of `graphs` in use
@@ -334,8 +334,7 @@ bool WholeStep(const mpd_solver *s) {
     return s->ring_ok && !s->ring_overlap && !MPD_INTERIOR_PAIR;
 }
 
-// parity: that of the step count the launch starts from less the run's
-// (StepHot::Run::parity), -1 where unknown.
+// parity: that of the step count the launch starts from, -1 where unknown.
 int LaunchStep(mpd_solver *s, bool use_state_dt, double dt, bool want_ws, int slot, int parity) {
     MPD_CK(mpd::launch_lf_step(s->g, s->step_plan, s->tmap[0], s->tmap[1], s->buf[0], s->buf[1],
                                s->st, dt, use_state_dt ? 1 : 0, want_ws, s->ring, slot,
@@ -480,16 +479,17 @@ int CheckHandle(mpd_solver *s) {
 // check_every / check_at: the relative-change check follows the steps i (from
 // 1) with i % check_every == check_at; check_at < 0: every step (the
 // controller's own due flag decides).
+// parity: that of the step count every launch of the graph starts from, -1
+// where it may vary (a hint: a launch that finds another count is only slower).
 // A handle keeps the graphs of its last kind of run.  Continued runs start at
-// other step counts: without a check one graph serves them all, with one there
-// is a graph per offset of the check, the last kRunGraphs of them kept.  (100
-// steps of 100 x 40, B200: 0.6 ms to capture and instantiate; a check's two
+// other step counts: there is a graph per parity and offset of the check, the
+// last kRunGraphs of them kept.  (100 steps of 100 x 40, B200: 0.6 ms to capture and instantiate; a check's two
 // nodes and the controller after every step instead of where due, which any
 // offset could share, cost 0.3 ms a hundred steps.)
 constexpr size_t kRunGraphs = 16;
 
 int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resid_every,
-               int check_every, int check_at) {
+               int check_every, int check_at, int parity) {
     const mpd_solver::GraphKind kind{
         steps, (with_check ? 1 : 0) | (want_ws ? 2 : 0) | (s->ring_overlap ? 4 : 0), resid_every,
         with_check ? check_every : 0};
@@ -499,19 +499,15 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
         s->graphs.clear();
         s->graph_kind = kind;
     }
-    auto cached = [&](int at) {
-        for (const mpd_solver::RunGraph &r : s->graphs)
-            if (r.check_at == at) s->graph = r.exec;
-        return s->graph != nullptr;
-    };
     if (!with_check) check_at = -1;
-    if (cached(check_at)) return MPD_OK;
+    if (!WholeStep(s)) parity = -1;
+    for (const mpd_solver::RunGraph &r : s->graphs)
+        if (r.check_at == check_at && r.parity == parity) s->graph = r.exec;
+    if (s->graph) return MPD_OK;
     if (s->graphs.size() == kRunGraphs) {  // the stream is idle: no launch uses it
         cudaGraphExecDestroy(s->graphs.front().exec);
         s->graphs.erase(s->graphs.begin());
     }
-    // consecutive launches start at one parity where a graph's steps are even
-    const bool parity_known = steps % 2 == 0;
     cudaGraph_t graph = nullptr;
     MPD_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int rc = MPD_OK;
@@ -523,7 +519,7 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
             rc = EnqueueStep(s, false, true, 0.0, check, want_ws, res);
             continue;
         }
-        rc = LaunchStep(s, true, 0.0, want_ws, slot, parity_known ? i & 1 : -1);
+        rc = LaunchStep(s, true, 0.0, want_ws, slot, parity < 0 ? -1 : (parity + i) & 1);
         slot ^= 1;
         if (rc == MPD_OK && (res || check || i == steps - 1)) {
             const cudaError_t ef = mpd::launch_finish_steps(s->g, s->st, want_ws, slot, s->stream);
@@ -542,7 +538,7 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
     const cudaError_t e2 = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e2 != cudaSuccess) return Fail(MPD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2));
-    s->graphs.push_back({exec, check_at});
+    s->graphs.push_back({exec, check_at, parity});
     s->graph = exec;
     s->graph_builds++;
     return MPD_OK;
@@ -830,7 +826,6 @@ static int FinishRun(mpd_solver *s, long long step0, mpd_run_stats *stats) {
     h.resid_every = 1;
     h.T = INFINITY;
     h.max_steps = LLONG_MAX;
-    h.hot.run.parity = 0;
     rc = PushState(s);
     if (rc != MPD_OK) return rc;
     if (nonfinite) return Fail(MPD_ERR_NONFINITE, "non-finite value in the state");
@@ -900,8 +895,6 @@ static int PrepareRun(mpd_solver *s, const mpd_run_params *p, long long &step0) 
     if (h.t + dt > h.T) dt = h.T - h.t;  // src/main.cpp:221-223
     h.dt = dt;
     if (!(h.t < h.T)) h.done = 1;
-    // graph launches start after the exact first step, where there is one
-    h.hot.run.parity = static_cast<int>((h.step + (s->host_step == 0 ? 1 : 0)) & 1);
     return PushState(s);
 }
 
@@ -1065,8 +1058,10 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
                                      p->check_frequency) % p->check_frequency);
     // before the run's first event: a capture is no part of its device time
     if (p->engine != MPD_ENGINE_PERSISTENT) {
+        const int parity =
+            monitored || per_graph % 2 != 0 ? -1 : static_cast<int>((step0 + taken_before) & 1);
         rc = BuildGraph(s, per_graph, with_check, want_ws, p->residual_every, p->check_frequency,
-                        check_at);
+                        check_at, parity);
         if (rc != MPD_OK) return rc;
     }
 
@@ -1132,7 +1127,6 @@ int mpd_run(mpd_solver *s, const mpd_run_params *p, mpd_run_stats *stats) {
         const long long next = (h.step / p->monitor_every + 1) * p->monitor_every;
         h.max_steps = next < end ? next : end;
         h.done = 0;
-        h.hot.run.parity = static_cast<int>(h.step & 1);
         rc = PushState(s);
         if (rc != MPD_OK) return rc;
     }

@@ -90,8 +90,9 @@ def test_wave_speed_of_whole_steps_after_others(pkg, lead, between, other):
 
 
 def test_continued_runs_reuse_their_graphs(pkg):
-    """Runs from odd and even steps, plain and monitored, and new initial states
-    need one graph; with a change check one for each offset, the last 16 kept."""
+    """Runs from odd and from even steps need a graph each, whatever the number of
+    them and the new initial states, monitored ones one more; with a change check
+    there is one for each offset too, the last 16 kept."""
     case = cases.make_case(ring_layouts.channel(40, 31))
     a = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast", with_prev=True)
     b = pkg.GpuSolver(case.cfg, case.grid, case.phys, precision="fast", with_prev=True)
@@ -111,11 +112,11 @@ def test_continued_runs_reuse_their_graphs(pkg):
     a.set_physical(case.phys)
     b.set_physical(case.phys)
     both(max_steps=100, steps_per_graph=10)
-    assert a.graph_builds() == 1
-    check = dict(steps_per_graph=20, convergence_threshold=1e-30, check_frequency=20)
-    for n in (60, 60, 47, 60, 13, 60, 60):   # two offsets
-        both(max_steps=n, **check)
     assert a.graph_builds() == 3
+    check = dict(steps_per_graph=20, convergence_threshold=1e-30, check_frequency=20)
+    for n in (60, 60, 47, 60, 13, 60, 60):   # two offsets, their parities with them
+        both(max_steps=n, **check)
+    assert a.graph_builds() == 5
     for _ in range(40):                      # all 20 offsets, twice
         both(max_steps=21, **check)
     a.close()
