@@ -296,6 +296,14 @@ int RingSymOf(int sym) {
     }
 }
 
+// Free indexes of each face's cells, L_LO, L_HI, M_LO, M_HI; (1, M+1) is
+// M_HI's, (L, M+1) is L_HI's.
+constexpr int kFaceLo[4] = {1, 1, 2, 1};
+int FaceHi(int f, int L, int M) {
+    const int hi[4] = {M, M + 1, L - 1, L - 1};
+    return hi[f];
+}
+
 bool ConstantField(const SegDesc &d, int j) {
     return d.type[j] == COND_DIRICHLET || (d.type[j] == COND_EXPR && d.form[j] == EF_CONST);
 }
@@ -339,10 +347,8 @@ bool CompileRing(const CompiledBc &bc, int L, int M, CompiledRing &out) {
     // the segment that decides each face cell: the last one that covers it
     out.len = line_len(L, M);
     out.cov.assign(4 * static_cast<size_t>(out.len), 0);
-    // L_LO, L_HI, M_LO, M_HI; (1, M+1) is M_HI's, (L, M+1) is L_HI's
-    const int lo[4] = {1, 1, 2, 1}, hi[4] = {M, M + 1, L - 1, L - 1};
     for (int f = 0; f < 4; ++f)
-        for (int k = lo[f]; k <= hi[f]; ++k) {
+        for (int k = kFaceLo[f]; k <= FaceHi(f, L, M); ++k) {
             int found = -1, n = 0;
             for (int t = 0; t < bc.nseg[f]; ++t) {
                 const SegDesc &d = bc.seg[bc.first[f] + t];
@@ -364,6 +370,26 @@ bool CompileRing(const CompiledBc &bc, int L, int M, CompiledRing &out) {
         for (int j : {Q_VZ, Q_HZ})
             if (d.type[j] != COND_AXIS_LF && !ConstantField(d, j)) return false;
     }
+    return true;
+}
+
+bool RingInRange(const CompiledRing &ring, int L, int M) {
+    const size_t n = ring.seg.size();
+    if (n > static_cast<size_t>(kRingSegments) || ring.len < line_len(L, M) ||
+        ring.cov.size() != 4 * static_cast<size_t>(ring.len))
+        return false;
+    for (const RingSeg &r : ring.seg) {
+        if (r.nbin < 0 || r.nbin > 8) return false;
+        for (int k = 0; k < r.nbin; ++k) {
+            const RingBin &b = r.bin[k];
+            if (b.j < 0 || b.j >= 8 || b.fa < RS_CONST || b.fa > RS_RZNB || b.fb < RS_CONST ||
+                b.fb > RS_RZNB)
+                return false;
+        }
+    }
+    for (int f = 0; f < 4; ++f)
+        for (int k = kFaceLo[f]; k <= FaceHi(f, L, M); ++k)
+            if (ring.cov[static_cast<size_t>(f) * ring.len + k] >= n) return false;
     return true;
 }
 

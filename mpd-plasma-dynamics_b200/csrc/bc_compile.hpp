@@ -38,6 +38,10 @@ struct CompiledRing {
 };
 bool CompileRing(const CompiledBc &bc, int L, int M, CompiledRing &out);
 
+// Whether every index that the ring's cells take from the table lies in its
+// range (they use them unchecked).
+bool RingInRange(const CompiledRing &ring, int L, int M);
+
 // Returns an MPD_* status; on failure `err` holds a message in the
 // reference's wording where the reference has one.
 int CompileBc(const mpd_config &cfg, CompiledBc &out, std::string &err);

@@ -291,6 +291,20 @@ int mpd_emu_download(void *h, int which, double *out) {
     return MPD_OK;
 }
 
+// Whether the ring table passes RingInRange with one index changed: what 0 cov
+// [at], 1 nbin of segment at, 2 / 3 / 4 j / fa / fb of the first field of segment
+// at; -1 nothing.
+int mpd_emu_ring_in_range(void *h, int what, int at, int value) {
+    auto *s = static_cast<EmuSolver *>(h);
+    mpd::CompiledRing r = s->ring;
+    if (what == 0) r.cov[at] = static_cast<unsigned char>(value);
+    if (what == 1) r.seg[at].nbin = value;
+    if (what == 2) r.seg[at].bin[0].j = value;
+    if (what == 3) r.seg[at].bin[0].fa = value;
+    if (what == 4) r.seg[at].bin[0].fb = value;
+    return mpd::RingInRange(r, s->g.L, s->g.M) ? 1 : 0;
+}
+
 // OncePerDevice over n calls: call i on devices[i], its work returning rc[i];
 // ran[i]: whether the work ran, ret[i]: what the call returned.
 void mpd_emu_once_per_device(const int *devices, const int *rc, int n, int *ran, int *ret) {

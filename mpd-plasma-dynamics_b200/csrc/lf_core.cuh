@@ -510,9 +510,10 @@ struct BcTable {
 };
 
 // The boundary ring in a form whose cells cost a few hundred instructions
-// each (ring_kernel, lf_step.cuh): a segment's fields without the interpreter,
-// and per face the segment that decides each cell.  CompileRing
-// (bc_compile.cpp) says which configurations have one.
+// each (ring_cell_new, which lf_step_kernel's ring warps run): a segment's fields
+// without the interpreter, and per face the segment that decides each cell.
+// CompileRing (bc_compile.cpp) says which configurations have one, RingInRange
+// there checks the indexes.
 constexpr int kRingSegments = 16;  // segments of all faces a ring table holds
 
 // Operands of a binary field: slots of the neighbour's and of the cell's own
@@ -951,7 +952,7 @@ template <class Slots>
 MPD_HD void ring_eval(const RingSeg &d, const RingGeo &x, const Slots &nb, const Slots &cur,
                       const double keep[8], double q[8]) {
     const unsigned int neu = d.neu, axis = d.axis;
-    const int nbin = d.nbin < 8 ? d.nbin : 8;
+    const int nbin = d.nbin;
 #pragma unroll
     for (int j = 0; j < 8; ++j) q[j] = nb.get(j);
 #pragma unroll
@@ -968,7 +969,7 @@ MPD_HD void ring_eval(const RingSeg &d, const RingGeo &x, const Slots &nb, const
         const RingBin &e = d.bin[b];
         const double a = ring_operand(x, e.fa, e.ca, nb, cur);
         const double c = ring_operand(x, e.fb, e.cb, nb, cur);
-        cur.set(e.j & 7, bc_binop(e.op, a, c));
+        cur.set(e.j, bc_binop(e.op, a, c));
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) q[j] = cur.get(j);
@@ -1300,12 +1301,12 @@ struct RingLane {
             face = m == 1 ? FACE_M_LO : FACE_M_HI, k = l1, ln = l1, mn = m == 1 ? 2 : M;
         }
         m_lo = face == FACE_M_LO;
-        is = t.cov[face * t.len + k] & (kRingSegments - 1);
+        is = t.cov[face * t.len + k];
         is2 = 0;
         x = ring_geo(g, l1, m1, ln, mn);
         if (two) {
             const int f2 = l == 1 ? FACE_M_HI : FACE_L_HI;
-            is2 = t.cov[f2 * t.len + (l == 1 ? 1 : m)] & (kRingSegments - 1);
+            is2 = t.cov[f2 * t.len + (l == 1 ? 1 : m)];
             x2 = ring_geo(g, l, m, l1, m1);
         }
         f.place(g, ln, old ? 2 : mn);
@@ -1406,7 +1407,7 @@ MPD_HD void ring_cell_new(const Geo &g, const RingTable &t, const RingSeg *seg,
     // (l-1, 1) as the segment loop leaves it: L_LO's corner, what the same
     // segment leaves (AxisLF keeps the old value), or an earlier segment's
     const int f3 = l == 2 ? FACE_L_LO : FACE_M_LO;
-    const int is3 = t.cov[f3 * t.len + (l == 2 ? 1 : l - 1)] & (kRingSegments - 1);
+    const int is3 = t.cov[f3 * t.len + (l == 2 ? 1 : l - 1)];
     if (l > 2 && is3 == c.is) {
         S.vz = (axis >> Q_VZ & 1u) ? os.vz : d.value[Q_VZ];
         S.Hz = (axis >> Q_HZ & 1u) ? os.Hz : d.value[Q_HZ];

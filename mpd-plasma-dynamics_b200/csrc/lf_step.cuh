@@ -123,8 +123,9 @@ __device__ __forceinline__ StepCtl step_resolve(const Geo &g, const StepWords &x
 static_assert(sizeof(RingSeg) % 16 == 0, "ring segments are copied as 16-byte words");
 
 // A shared-memory double at a 32-bit shared address: explicitly the shared
-// state space (an operand chosen at run time between these slots and global
-// arrays through one generic pointer faulted).
+// state space.  (An earlier form of the ring that picked operands between these
+// slots and global arrays through one pointer at run time faulted.  The cause
+// is not known; nothing is left of that form.)
 __device__ __forceinline__ double lds_f64(uint32_t a) {
     double v;
     asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");

@@ -117,7 +117,7 @@ struct mpd_solver {
     bool ring_beside = false;                // the interior just launched left the ring to it
     bool ring_ok = false;                    // the configuration has a ring table
     bool whole_step = false;                 // the kernel just launched was a whole step
-    mpd::RingTable ring{};                   // the ring inside the interior's rows
+    mpd::RingTable ring{};                   // the table, for lf_step_kernel
     mpd::StepPlan step_plan;                 // lf_step_kernel's one wave
     unsigned char *d_ring = nullptr;         // the table's segments and cover
     mpd::TmaPlan pplan;                      // persistent launch (cooperative wave)
@@ -708,9 +708,13 @@ int mpd_create(const mpd_config *cfg, const mpd_geometry *geom, const double *ph
             s->overlap_blocks = groups < sms ? groups : sms;
             s->overlap_ok = g.L >= 4 && s->overlap_blocks > 0;
         }
-        // the boundary ring inside the interior's rows, where the faces allow it
+        // the boundary ring in the interior's kernel, where the faces allow it
         mpd::CompiledRing cr;
         if (mpd::CompileRing(cbc, s->L, s->M, cr)) {
+            if (!mpd::RingInRange(cr, s->L, s->M)) {
+                FreeAll(s);
+                return Fail(MPD_ERR_INVALID, "boundary ring table out of range");
+            }
             const size_t nseg = cr.seg.size() * sizeof(mpd::RingSeg);
             STEP(DevAlloc(s, &s->d_ring, nseg + cr.cov.size()));
             if (cudaMemcpy(s->d_ring, cr.seg.data(), nseg, cudaMemcpyHostToDevice) !=

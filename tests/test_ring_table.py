@@ -63,3 +63,21 @@ def test_general_ring_after_table_rings_bitwise(make, L, M):
         a.advance(1e-5)
         b.advance(1e-5, order=order)
         np.testing.assert_array_equal(b.conserved(), a.conserved())
+
+
+@pytest.mark.parametrize("make", ring_layouts.ACCEPTED, ids=lambda f: f.__name__)
+def test_indexes_of_the_table_are_checked_on_the_host(make):
+    """The device takes them unchecked: every table in range, none with an index
+    past its end."""
+    L, M = 12, 9
+    emu = Emu(cases.make_case(make(L, M)), "fast")
+    ok = lambda *a: bool(emu.lib.mpd_emu_ring_in_range(emu.h, *a))
+    length, cfg = max(L + 2, M + 3), make(L, M)
+    nseg = sum(len(f.segments) for f in (cfg.bc_l_lo, cfg.bc_l_hi, cfg.bc_m_lo, cfg.bc_m_hi))
+    assert ok(-1, 0, 0)
+    for face, (lo, hi) in enumerate([(1, M), (1, M + 1), (2, L - 1), (1, L - 1)]):
+        for k in (lo, hi):
+            assert ok(0, face * length + k, nseg - 1) and not ok(0, face * length + k, nseg)
+    assert not ok(1, 0, 9) and not ok(1, 0, -1)
+    assert any(not ok(2, s, 8) and not ok(2, s, -1) and not ok(3, s, 22) and not ok(4, s, -2)
+               for s in range(nseg))
