@@ -117,12 +117,14 @@ int mpd_advance(mpd_solver *s, double dt);
  * (Diagnostics::ComputeDt after every step), the reference's relative-L2
  * convergence check every check_frequency steps, and an L-inf residual
  * criterion.  Runs until t >= T, convergence, or max_steps. */
-/* How mpd_run drives the steps.  GRAPH: one kernel per step (an interior and a
- * boundary kernel where mpd_set_ring_overlap says so), replayed from captured
- * CUDA graphs.  PERSISTENT: one cooperative
- * launch runs many steps with grid barriers between the interior and the
- * boundary phase (fast precision, no SolutionChange checks).  AUTO takes
- * GRAPH.  Both give the same results, bit for bit. */
+/* How mpd_run drives the steps.  GRAPH: one kernel per step, replayed from
+ * captured CUDA graphs; an interior and a boundary kernel in exact precision,
+ * for boundary configurations lf_step_kernel does not take, and where
+ * mpd_set_ring_overlap says so.  PERSISTENT: one cooperative launch runs many
+ * steps with grid barriers between the interior and the boundary phase (fast
+ * precision, no SolutionChange checks).  AUTO takes GRAPH.  Both give the same
+ * results, bit for bit, from any state that the other, mpd_advance or a batch
+ * left. */
 #define MPD_ENGINE_AUTO 0
 #define MPD_ENGINE_GRAPH 1
 #define MPD_ENGINE_PERSISTENT 2
@@ -239,8 +241,8 @@ int mpd_set_expression_ic(mpd_solver *s, const char *const exprs[8], int n_vars,
  * reference applies the faces after the central update, src/solver.cpp:
  * 22-37, and every form keeps that order of values).  on = 0 (the default):
  * in the interior's own kernel where the boundary configuration allows
- * (lf_step_kernel: no interpreted expressions, every face cell covered, AxisLF
- * segments disjoint), else in a kernel after it, reading the central cells it
+ * (lf_step_kernel: no interpreted expressions, every face cell covered, at most
+ * 16 segments, AxisLF segments disjoint and in order), else in a kernel after it, reading the central cells it
  * stored.  on = 1: in bc_overlap_kernel beside the interior kernel.  All give
  * the same bits.  Takes effect from the next step; exact precision, the first
  * step and (on = 1) grids with L_max < 4 always run it after the interior.

@@ -2,6 +2,7 @@
 // launch sequence, the graph-resident run loop, diagnostics and transfers.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <climits>
@@ -152,7 +153,9 @@ struct mpd_solver {
         cudaGraphExec_t exec;
         int check_at, parity;
     };
-    std::vector<RunGraph> graphs;
+    static constexpr int kRunGraphs = 16;
+    RunGraph graphs[kRunGraphs];      // the oldest first
+    int ngraphs = 0;
     cudaGraphExec_t graph = nullptr;  // the one of `graphs` in use
     long long graph_builds = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, snap_ev = nullptr, stage_ev = nullptr;
@@ -186,11 +189,17 @@ void RefreshMirror(mpd_solver *s) {
     s->hm->wait_fail = s->h_st->wait_fail;
 }
 
+void DropGraphs(mpd_solver *s) {
+    for (int i = 0; i < s->ngraphs; ++i) cudaGraphExecDestroy(s->graphs[i].exec);
+    s->ngraphs = 0;
+    s->graph = nullptr;
+}
+
 void FreeAll(mpd_solver *s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->side) cudaStreamSynchronize(s->side);
-    for (const mpd_solver::RunGraph &r : s->graphs) cudaGraphExecDestroy(r.exec);
+    DropGraphs(s);
     cudaFree(s->buf[0]);
     cudaFree(s->buf[1]);
     cudaFree(s->ic);
@@ -483,11 +492,10 @@ int CheckHandle(mpd_solver *s) {
 // where it may vary (a hint: a launch that finds another count is only slower).
 // A handle keeps the graphs of its last kind of run.  Continued runs start at
 // other step counts: there is a graph per parity and offset of the check, the
-// last kRunGraphs of them kept.  (100 steps of 100 x 40, B200: 0.6 ms to capture and instantiate; a check's two
-// nodes and the controller after every step instead of where due, which any
-// offset could share, cost 0.3 ms a hundred steps.)
-constexpr size_t kRunGraphs = 16;
-
+// last kRunGraphs of them kept.  (100 steps of 100 x 40, B200: 0.6 ms to capture
+// and instantiate; a check's two nodes and the controller after every step
+// instead of where due, which any offset could share, cost 0.3 ms a hundred
+// steps.)
 int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resid_every,
                int check_every, int check_at, int parity) {
     const mpd_solver::GraphKind kind{
@@ -495,18 +503,19 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
         with_check ? check_every : 0};
     s->graph = nullptr;
     if (!(kind == s->graph_kind)) {
-        for (const mpd_solver::RunGraph &r : s->graphs) cudaGraphExecDestroy(r.exec);
-        s->graphs.clear();
+        DropGraphs(s);
         s->graph_kind = kind;
     }
     if (!with_check) check_at = -1;
     if (!WholeStep(s)) parity = -1;
-    for (const mpd_solver::RunGraph &r : s->graphs)
-        if (r.check_at == check_at && r.parity == parity) s->graph = r.exec;
+    for (int i = 0; i < s->ngraphs; ++i)
+        if (s->graphs[i].check_at == check_at && s->graphs[i].parity == parity)
+            s->graph = s->graphs[i].exec;
     if (s->graph) return MPD_OK;
-    if (s->graphs.size() == kRunGraphs) {  // the stream is idle: no launch uses it
-        cudaGraphExecDestroy(s->graphs.front().exec);
-        s->graphs.erase(s->graphs.begin());
+    if (s->ngraphs == mpd_solver::kRunGraphs) {  // the stream is idle: no launch uses it
+        cudaGraphExecDestroy(s->graphs[0].exec);
+        std::move(s->graphs + 1, s->graphs + s->ngraphs, s->graphs);
+        s->ngraphs--;
     }
     cudaGraph_t graph = nullptr;
     MPD_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -538,7 +547,7 @@ int BuildGraph(mpd_solver *s, int steps, bool with_check, bool want_ws, int resi
     const cudaError_t e2 = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e2 != cudaSuccess) return Fail(MPD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2));
-    s->graphs.push_back({exec, check_at, parity});
+    s->graphs[s->ngraphs++] = {exec, check_at, parity};
     s->graph = exec;
     s->graph_builds++;
     return MPD_OK;
