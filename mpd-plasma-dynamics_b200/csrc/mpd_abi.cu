@@ -329,7 +329,8 @@ int RefreshWalls(mpd_solver *s, long long step) {
 // the guarded relative-L2 convergence check and, every residual_every steps,
 // the L-inf residual.  want_ws: fuse the maximum
 // wave speed (adaptive dt and the per-call ComputeDt need it).
-// Interior kernel of fast steps >= 1 on the graph and per-call paths:
+// Interior kernel of fast steps >= 1 on the graph and per-call paths where the
+// step is not one lf_step_kernel (WholeStep):
 // lf_tma_kernel (one point column per lane), or lf_pair_kernel (two) with
 // MPD_INTERIOR_PAIR 1; both give the same bits.  Measured on a B200 at
 // 1600 x 640 (30 back-to-back launches): 26.3 us one column, 28.4 us pair
